@@ -44,7 +44,7 @@ __device__ __forceinline__ void for_common(const int32_t *adj, int32_t a0, int32
     }
 }
 
-__device__ __forceinline__ void write_tri(TriBuf &tb, int64_t pos, int32_t a, int32_t b, int32_t c)
+__device__ __forceinline__ void write_tri(const TriBuf &tb, int64_t pos, int32_t a, int32_t b, int32_t c)
 {
     if (pos >= tb.budget) return;
     int32_t lo = min(a, min(b, c)), hi = max(a, max(b, c));
@@ -57,9 +57,10 @@ __device__ __forceinline__ void write_tri(TriBuf &tb, int64_t pos, int32_t a, in
 // remove degenerate triangles, sort lexicographically, unique (the first n
 // entries of the buffer); returns the new count
 template <class Team>
-__device__ int64_t tri_normalize(const Team &t, Scratch &sc, char *sm, int32_t *t1, int32_t *t2, int32_t *t3, int64_t n,
+__device__ __noinline__ int64_t tri_normalize(const Team &t, Scratch &sc, char *, int32_t *t1, int32_t *t2, int32_t *t3, int64_t n,
                                  int32_t nmax)
 {
+    char *sm = team_smem();
     if (n == 0) return 0;
     const int nb = bits_for((uint64_t)(nmax > 0 ? nmax : 1));
     uint64_t m = sc.arena.mark();
@@ -70,8 +71,8 @@ __device__ int64_t tri_normalize(const Team &t, Scratch &sc, char *sm, int32_t *
     const uint64_t mask = (nb == 0) ? 0 : ((uint64_t(1) << nb) - 1);
     // drop degenerate triangles; key the rest by lo and (md, hi)
     const int64_t w = team_compact(
-        t, sc, sm, n, [&](int64_t k) { return !(t1[k] == t2[k] || t1[k] == t3[k] || t2[k] == t3[k]); },
-        [&](int64_t k, int64_t p) {
+        t, sc, sm, n, [=](int64_t k) { return !(t1[k] == t2[k] || t1[k] == t3[k] || t2[k] == t3[k]); },
+        [=](int64_t k, int64_t p) {
             int32_t a = t1[k], b = t2[k], c = t3[k];
             int32_t lo = min(a, min(b, c)), hi = max(a, max(b, c));
             int32_t md = max(min(a, b), min(max(a, b), c));
@@ -88,13 +89,13 @@ __device__ int64_t tri_normalize(const Team &t, Scratch &sc, char *sm, int32_t *
         if (sc.arena.ok() && w < (int64_t(1) << 31)) {
             // the payload of each triangle is its lo, so every sorted position
             // rebuilds its keys from its own entries
-            auto lo = [&](int64_t i) { return tlo[i]; };
+            auto lo = [=](int64_t i) { return tlo[i]; };
             done = team_bucket_sort_ex(
-                t, sc, sm, w, nmax + 1, lo, lo, [&](int64_t i) { return u1[i]; }, lo, k2, bidx, bst);
+                t, sc, sm, w, nmax + 1, lo, lo, [=](int64_t i) { return u1[i]; }, lo, k2, bidx, bst);
             if (done) {
                 team_for_batched(
-                    t, w, [&](int64_t p) { return make_longlong2((long long)bidx[p], (long long)k2[p]); },
-                    [&](int64_t p, longlong2 v) {
+                    t, w, [=](int64_t p) { return make_longlong2((long long)bidx[p], (long long)k2[p]); },
+                    [=](int64_t p, longlong2 v) {
                         const uint64_t mh = (uint64_t)v.y;
                         k1[p] = pack_key((int32_t)v.x, (int32_t)(mh >> nb), nb);
                         u2[p] = mh & mask;
@@ -125,8 +126,8 @@ __device__ int64_t tri_normalize(const Team &t, Scratch &sc, char *sm, int32_t *
         team_sort_pairs(t, sc, sm, k1, u1, k2, u2, w, 2 * nb);
     }
     const int64_t u = team_compact(
-        t, sc, sm, w, [&](int64_t k) { return k == 0 || k1[k] != k1[k - 1] || u1[k] != u1[k - 1]; },
-        [&](int64_t k, int64_t p) {
+        t, sc, sm, w, [=](int64_t k) { return k == 0 || k1[k] != k1[k - 1] || u1[k] != u1[k - 1]; },
+        [=](int64_t k, int64_t p) {
             t1[p] = (int32_t)(k1[k] >> nb);
             t2[p] = (int32_t)(k1[k] & mask);
             t3[p] = (int32_t)u1[k];
@@ -187,16 +188,16 @@ __device__ void expansion_stage(const Team &t, Scratch &sc, char *sm, TriBuf &tb
         t.sync();
         const int64_t start = tb.count;
         const int64_t rem = tb.budget - start;
-        const int64_t tot = team_sum<Team, int64_t>(t, sc, sm, xn, [&](int64_t q) -> int64_t { return ccount[q]; });
+        const int64_t tot = team_sum<Team, int64_t>(t, sc, sm, xn, [=](int64_t q) -> int64_t { return ccount[q]; });
         // round-robin when the chunk does not fit: the largest K with
         // sum_q min(count_q, K) <= rem, and `extra` expansions keep one more
         int64_t K = KALL, extra = 0;
         if (tot > rem) {
-            const int32_t mx = team_max<Team, int32_t>(t, sc, sm, xn, 0, [&](int64_t q) { return ccount[q]; });
+            const int32_t mx = team_max<Team, int32_t>(t, sc, sm, xn, 0, [=](int64_t q) { return ccount[q]; });
             int64_t lo = 0, hi = mx, slo = 0;
             for (int guard = 0; lo < hi && guard < 40; ++guard) {
                 const int64_t k = (lo + hi + 1) >> 1;
-                const int64_t s = team_sum<Team, int64_t>(t, sc, sm, xn, [&](int64_t q) -> int64_t {
+                const int64_t s = team_sum<Team, int64_t>(t, sc, sm, xn, [=](int64_t q) -> int64_t {
                     const int64_t c = ccount[q];
                     return c < k ? c : k;
                 });
@@ -214,11 +215,11 @@ __device__ void expansion_stage(const Team &t, Scratch &sc, char *sm, TriBuf &tb
         // count_q is replaced by the number it keeps
         team_scan<Team, int64_t>(
             t, sc, sm, xn,
-            [&](int64_t q) -> int64_t {
+            [=](int64_t q) -> int64_t {
                 const int64_t c = ccount[q];
                 return ((c < K ? c : K) << 25) | (c > K ? 1 : 0);
             },
-            [&](int64_t q, int64_t pre, int64_t v) {
+            [=](int64_t q, int64_t pre, int64_t v) {
                 const int64_t pmin = pre >> 25, pbig = pre & ((int64_t(1) << 25) - 1);
                 cbase[q] = pmin + (pbig < extra ? pbig : extra);
                 ccount[q] = (int32_t)((v >> 25) + ((v & 1) && pbig < extra ? 1 : 0));
@@ -248,9 +249,11 @@ __device__ void expansion_stage(const Team &t, Scratch &sc, char *sm, TriBuf &tb
 // conflicted_cycles_cuda (:222-343).  Triangles land in tb (allocated here
 // in the temporaries); tb.count is the reference's counter.
 template <class Team>
-__device__ void conflicted_cycles(const Team &t, Scratch &sc, char *sm, const Graph &A, int max_len, float tri_factor,
+__device__ __noinline__ void conflicted_cycles(const Team &t, Scratch &sc, char *, const Graph &graph, int max_len, float tri_factor,
                                   float tol, TriBuf &tb)
 {
+    char *sm = team_smem();
+    const Graph A = graph;  // its pointers in registers
     tb.count = 0;
     tb.num = 0;
     tb.budget = 0;
@@ -260,7 +263,7 @@ __device__ void conflicted_cycles(const Team &t, Scratch &sc, char *sm, const Gr
     // the smallest cost: known from the pass that built the graph, or one pass
     const float mn = A.cmin == A.cmin
                          ? A.cmin
-                         : team_min<Team, float>(t, sc, sm, A.n, 3.4e38f, [&](int64_t e) { return A.cost[e]; });
+                         : team_min<Team, float>(t, sc, sm, A.n, 3.4e38f, [=](int64_t e) { return A.cost[e]; });
     const float thresh = mn * tol;          // determine_threshold (:170-174)
     const float pos_tol = -1.0f * thresh;   // create_matrices (:176-220)
     const int32_t N = A.max_dim();
@@ -311,7 +314,7 @@ __device__ void conflicted_cycles(const Team &t, Scratch &sc, char *sm, const Gr
     // one pass counts both: the low 32 bits count every repulsive edge (the
     // budget counts them all, :247), the high bits the kept ones; the kept
     // ones are compacted only when there are any
-    auto rep_code = [&](int64_t e) -> int64_t {
+    auto rep_code = [=](int64_t e) -> int64_t {
         if (!(A.cost[e] < thresh)) return 0;
         return (haspos[A.row[e]] && haspos[A.col[e]]) ? (int64_t(1) << 32) + 1 : 1;
     };
@@ -325,12 +328,12 @@ __device__ void conflicted_cycles(const Team &t, Scratch &sc, char *sm, const Gr
         return;
     }
     team_scan<Team, int64_t>(
-        t, sc, sm, A.n, [&](int64_t e) -> int64_t { return rep_code(e) >> 32; },
-        [&](int64_t e, int64_t pre, int64_t v) {
+        t, sc, sm, A.n, [=](int64_t e) -> int64_t { return rep_code(e) >> 32; },
+        [=](int64_t e, int64_t pre, int64_t v) {
             if (v) ridx[pre] = e;
         });
     prof_mark(t, sc, PH_CYCLES);
-    Csr C = build_symmetric_csr(t, sc, sm, A, N, [&](int64_t e) { return A.cost[e] > pos_tol; }, false);
+    Csr C = build_symmetric_csr(t, sc, sm, A, N, [=](int64_t e) { return A.cost[e] > pos_tol; }, false);
     prof_mark(t, sc, PH_CSR);
     const int64_t budget = (int64_t)(int32_t)(tri_factor * (float)Rall);  // (:247)
     tb.budget = budget < 0 ? 0 : budget;
@@ -341,18 +344,18 @@ __device__ void conflicted_cycles(const Team &t, Scratch &sc, char *sm, const Gr
     if (!sc.arena.ok()) return;
     const int32_t *off = C.off;
     const int32_t *adj = C.adj;
-    auto rv1 = [&](int64_t r) { return A.row[ridx[r]]; };
-    auto rv2 = [&](int64_t r) { return A.col[ridx[r]]; };
+    auto rv1 = [=](int64_t r) { return A.row[ridx[r]]; };
+    auto rv2 = [=](int64_t r) { return A.col[ridx[r]]; };
     // ---- 3-cycles: find_triangles_parallel (:31-61)
     {
-        TriBuf &T = tb;
+        const TriBuf T = tb;
         expansion_stage(
-            t, sc, sm, T, nullptr, R, R,
-            [&](int64_t r, int64_t) {
+            t, sc, sm, tb, nullptr, R, R,
+            [=](int64_t r, int64_t) {
                 int32_t v1 = rv1(r), v2 = rv2(r);
                 return count_common(adj, off[v1], off[v1 + 1], off[v2], off[v2 + 1]);
             },
-            [&](int64_t r, int64_t, int64_t pos, int64_t keep) {
+            [=](int64_t r, int64_t, int64_t pos, int64_t keep) {
                 int32_t v1 = rv1(r), v2 = rv2(r);
                 int64_t e = 0;
                 for_common(adj, off[v1], off[v1 + 1], off[v2], off[v2 + 1], [&](int32_t mid) {
@@ -365,19 +368,19 @@ __device__ void conflicted_cycles(const Team &t, Scratch &sc, char *sm, const Gr
     if (max_len >= 4 && tb.count < tb.budget) {
         tb.count = tri_normalize(t, sc, sm, tb.t1, tb.t2, tb.t3, tb.count, N);
         const int64_t X = team_scan<Team, int64_t>(
-            t, sc, sm, R, [&](int64_t r) -> int64_t { int32_t v1 = rv1(r); return off[v1 + 1] - off[v1]; },
-            [&](int64_t r, int64_t pre, int64_t) { xo[r] = pre; });
+            t, sc, sm, R, [=](int64_t r) -> int64_t { int32_t v1 = rv1(r); return off[v1 + 1] - off[v1]; },
+            [=](int64_t r, int64_t pre, int64_t) { xo[r] = pre; });
         if (t.rank() == 0) xo[R] = X;
         t.sync();
-        TriBuf &T = tb;
+        const TriBuf T = tb;
         expansion_stage(
-            t, sc, sm, T, xo, R, X,
-            [&](int64_t r, int64_t loc) {
+            t, sc, sm, tb, xo, R, X,
+            [=](int64_t r, int64_t loc) {
                 int32_t v1 = rv1(r), v2 = rv2(r);
                 int32_t n1 = adj[off[v1] + loc];
                 return 2 * count_common(adj, off[n1], off[n1 + 1], off[v2], off[v2 + 1]);
             },
-            [&](int64_t r, int64_t loc, int64_t pos, int64_t keep) {
+            [=](int64_t r, int64_t loc, int64_t pos, int64_t keep) {
                 int32_t v1 = rv1(r), v2 = rv2(r);
                 int32_t n1 = adj[off[v1] + loc];
                 int64_t e = 0;
@@ -394,17 +397,17 @@ __device__ void conflicted_cycles(const Team &t, Scratch &sc, char *sm, const Gr
         tb.count = tri_normalize(t, sc, sm, tb.t1, tb.t2, tb.t3, tb.count, N);
         const int64_t X = team_scan<Team, int64_t>(
             t, sc, sm, R,
-            [&](int64_t r) -> int64_t {
+            [=](int64_t r) -> int64_t {
                 int32_t v1 = rv1(r), v2 = rv2(r);
                 return (int64_t)(off[v1 + 1] - off[v1]) * (int64_t)(off[v2 + 1] - off[v2]);
             },
-            [&](int64_t r, int64_t pre, int64_t) { xo[r] = pre; });
+            [=](int64_t r, int64_t pre, int64_t) { xo[r] = pre; });
         if (t.rank() == 0) xo[R] = X;
         t.sync();
-        TriBuf &T = tb;
+        const TriBuf T = tb;
         expansion_stage(
-            t, sc, sm, T, xo, R, X,
-            [&](int64_t r, int64_t loc) {
+            t, sc, sm, tb, xo, R, X,
+            [=](int64_t r, int64_t loc) {
                 int32_t v1 = rv1(r), v2 = rv2(r);
                 int64_t d1 = off[v1 + 1] - off[v1];
                 int32_t n1 = adj[off[v1] + (int32_t)(loc % d1)];
@@ -412,7 +415,7 @@ __device__ void conflicted_cycles(const Team &t, Scratch &sc, char *sm, const Gr
                 if (n1 == n2) return 0;
                 return 3 * count_common(adj, off[n1], off[n1 + 1], off[n2], off[n2 + 1]);
             },
-            [&](int64_t r, int64_t loc, int64_t pos, int64_t keep) {
+            [=](int64_t r, int64_t loc, int64_t pos, int64_t keep) {
                 int32_t v1 = rv1(r), v2 = rv2(r);
                 int64_t d1 = off[v1 + 1] - off[v1];
                 int32_t n1 = adj[off[v1] + (int32_t)(loc % d1)];

@@ -75,8 +75,8 @@ __device__ void graph_set_dims(const Team &t, Scratch &sc, char *sm, Graph &g)
     int32_t mc = -1;
     float mn = 3.4e38f;
     team_maxi_minf(
-        t, sc, sm, g.n, -1, 3.4e38f, [&](int64_t e) { return g.col[e]; },
-        [&](int64_t e) { return g.row[e] != g.col[e] ? g.cost[e] : 3.4e38f; }, mc, mn);
+        t, sc, sm, g.n, -1, 3.4e38f, [=](int64_t e) { return g.col[e]; },
+        [=](int64_t e) { return g.row[e] != g.col[e] ? g.cost[e] : 3.4e38f; }, mc, mn);
     g.cols = mc + 1;
     g.rows = uread(&g.row[g.n - 1]) + 1;
     g.cmin = mn;
@@ -96,19 +96,20 @@ __device__ __forceinline__ uint64_t pack_key(int32_t a, int32_t b, int nbits)
 // their packed (min, max) keys inside the bucket sort; edge lists of 2^31 or
 // more take graph_from_edges_sorted (one radix sort of every edge's keys).
 template <class Team>
-__device__ Graph graph_from_edges_sorted(const Team &t, Scratch &sc, char *sm, const int32_t *i, const int32_t *j,
+__device__ __noinline__ Graph graph_from_edges_sorted(const Team &t, Scratch &sc, char *, const int32_t *i, const int32_t *j,
                                          const float *c, int64_t n);
 
 template <class Team>
-__device__ Graph graph_from_edges(const Team &t, Scratch &sc, char *sm, const int32_t *i, const int32_t *j,
+__device__ __noinline__ Graph graph_from_edges(const Team &t, Scratch &sc, char *, const int32_t *i, const int32_t *j,
                                   const float *c, int64_t n)
 {
+    char *sm = team_smem();
     if (n == 0 || n >= (int64_t(1) << 31)) return graph_from_edges_sorted(t, sc, sm, i, j, c, n);
     Graph out;
     out.n = n;
     out.rows = out.cols = 0;
     out.cmin = unknown_cost();
-    const int32_t mx = team_max<Team, int32_t>(t, sc, sm, n, 0, [&](int64_t e) { return i[e] > j[e] ? i[e] : j[e]; });
+    const int32_t mx = team_max<Team, int32_t>(t, sc, sm, n, 0, [=](int64_t e) { return i[e] > j[e] ? i[e] : j[e]; });
     const int nbh = bits_for((uint64_t)(mx > 0 ? mx : 1));
     uint64_t m = sc.arena.mark();
     int2 *lohi = sc.arena.take<int2>(n + 1);
@@ -119,16 +120,16 @@ __device__ Graph graph_from_edges(const Team &t, Scratch &sc, char *sm, const in
     if (!sc.arena.ok()) return out;
     const bool done = team_bucket_sort_ex(
         t, sc, sm, n, mx + 1,
-        [&](int64_t e) -> int64_t {
+        [=](int64_t e) -> int64_t {
             const int32_t a = i[e], b = j[e];
             const int32_t lo = a < b ? a : b, hi = a < b ? b : a;
             return ((int64_t)hi << 32) | (uint32_t)lo;
         },
-        [&](int64_t e) { return lohi[e].x; },
-        [&](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].y << 32) | (uint64_t)e; },
-        [&](int64_t e) { return __float_as_int(c[e]); }, sk, sbits, bst, sbk, -1,
-        [&](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].x << nbh) | (uint32_t)lohi[e].y; },
-        2 * nbh, [&](int64_t e, int64_t w) { lohi[e] = make_int2((int32_t)(uint32_t)w, (int32_t)(w >> 32)); });
+        [=](int64_t e) { return lohi[e].x; },
+        [=](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].y << 32) | (uint64_t)e; },
+        [=](int64_t e) { return __float_as_int(c[e]); }, sk, sbits, bst, sbk, -1,
+        [=](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].x << nbh) | (uint32_t)lohi[e].y; },
+        2 * nbh, [=](int64_t e, int64_t w) { lohi[e] = make_int2((int32_t)(uint32_t)w, (int32_t)(w >> 32)); });
     if (!done) return out;
     Arena &ar = sc.arena;
     const uint64_t bytes = (uint64_t)(n + 1) * 12 + 3 * 256;
@@ -144,8 +145,8 @@ __device__ Graph graph_from_edges(const Team &t, Scratch &sc, char *sm, const in
     g.cost = reinterpret_cast<float *>(ar.base + top + 2 * words);
     g.n = n;
     team_for_batched(
-        t, n, [&](int64_t p) { return make_int3(sbk[p], (int32_t)(sk[p] >> 32), sbits[p]); },
-        [&](int64_t p, int3 v) {
+        t, n, [=](int64_t p) { return make_int3(sbk[p], (int32_t)(sk[p] >> 32), sbits[p]); },
+        [=](int64_t p, int3 v) {
             g.row[p] = v.x;
             g.col[p] = v.y;
             g.cost[p] = __int_as_float(v.z);
@@ -159,13 +160,14 @@ __device__ Graph graph_from_edges(const Team &t, Scratch &sc, char *sm, const in
 }
 
 template <class Team>
-__device__ Graph graph_from_edges_sorted(const Team &t, Scratch &sc, char *sm, const int32_t *i, const int32_t *j,
+__device__ __noinline__ Graph graph_from_edges_sorted(const Team &t, Scratch &sc, char *, const int32_t *i, const int32_t *j,
                                          const float *c, int64_t n)
 {
+    char *sm = team_smem();
     Graph out;
     out.n = n;
     out.rows = out.cols = 0;
-    int32_t mx = team_max<Team, int32_t>(t, sc, sm, n, 0, [&](int64_t e) { return i[e] > j[e] ? i[e] : j[e]; });
+    int32_t mx = team_max<Team, int32_t>(t, sc, sm, n, 0, [=](int64_t e) { return i[e] > j[e] ? i[e] : j[e]; });
     const int nb = bits_for((uint64_t)mx);
     uint64_t m = sc.arena.mark();
     uint64_t *k1 = sc.arena.take<uint64_t>(n + 1), *k2 = sc.arena.take<uint64_t>(n + 1);
@@ -182,8 +184,8 @@ __device__ Graph graph_from_edges_sorted(const Team &t, Scratch &sc, char *sm, c
         int32_t *bidx = sc.arena.take<int32_t>(n + 1);
         if (sc.arena.ok() && n < (int64_t(1) << 31)) {
             done = team_bucket_sort(
-                t, sc, sm, n, mx + 1, [&](int64_t e) { return i[e] < j[e] ? i[e] : j[e]; },
-                [&](int64_t e) -> uint64_t {
+                t, sc, sm, n, mx + 1, [=](int64_t e) { return i[e] < j[e] ? i[e] : j[e]; },
+                [=](int64_t e) -> uint64_t {
                     return ((uint64_t)(uint32_t)(i[e] < j[e] ? j[e] : i[e]) << 32) | (uint64_t)e;
                 },
                 k2, bidx, bst);
@@ -234,9 +236,10 @@ __device__ Graph graph_from_edges_sorted(const Team &t, Scratch &sc, char *sm, c
 // BUCKET_MAX edges send the whole list through the LSD radix sort instead.
 // k1/v1 (and the spare k2/v2) hold n + 1 entries; the result ends in k1/v1.
 template <class Team>
-__device__ void contract_sorted_keys(const Team &t, Scratch &sc, char *sm, const Graph &A, const int32_t *map,
+__device__ __noinline__ void contract_sorted_keys(const Team &t, Scratch &sc, char *, const Graph &A, const int32_t *map,
                                      int32_t map_max, int nb, uint64_t *&k1, float *&v1, uint64_t *&k2, float *&v2)
 {
+    char *sm = team_smem();
     const int64_t n = A.n;
     bool done = false;
     uint64_t m = sc.arena.mark();
@@ -245,11 +248,11 @@ __device__ void contract_sorted_keys(const Team &t, Scratch &sc, char *sm, const
     if (sc.arena.ok() && n < (int64_t(1) << 31)) {
         done = team_bucket_sort(
             t, sc, sm, n, map_max + 1,
-            [&](int64_t e) {
+            [=](int64_t e) {
                 const int32_t a = map[A.row[e]], b = map[A.col[e]];
                 return a < b ? a : b;
             },
-            [&](int64_t e) -> uint64_t {
+            [=](int64_t e) -> uint64_t {
                 const int32_t a = map[A.row[e]], b = map[A.col[e]];
                 return ((uint64_t)(uint32_t)(a < b ? b : a) << 32) | (uint64_t)e;
             },
@@ -273,9 +276,10 @@ __device__ void contract_sorted_keys(const Team &t, Scratch &sc, char *sm, const
 }
 
 template <class Team>
-__device__ Graph graph_contract_sorted(const Team &t, Scratch &sc, char *sm, const Graph &A, const int32_t *map,
+__device__ __noinline__ Graph graph_contract_sorted(const Team &t, Scratch &sc, char *, const Graph &A, const int32_t *map,
                                        int32_t map_max, int *bad)
 {
+    char *sm = team_smem();
     const int64_t n = A.n;
     const int nb = bits_for((uint64_t)(map_max > 0 ? map_max : 0));
     uint64_t m = sc.arena.mark();
@@ -289,8 +293,8 @@ __device__ Graph graph_contract_sorted(const Team &t, Scratch &sc, char *sm, con
     contract_sorted_keys(t, sc, sm, A, map, map_max, nb, k1, v1, k2, v2);
     // run heads -> run index
     const int64_t nruns = team_compact(
-        t, sc, sm, n, [&](int64_t k) { return k == 0 || k1[k] != k1[k - 1]; },
-        [&](int64_t k, int64_t r) { runpos[r] = k; });
+        t, sc, sm, n, [=](int64_t k) { return k == 0 || k1[k] != k1[k - 1]; },
+        [=](int64_t k, int64_t r) { runpos[r] = k; });
     if (t.rank() == 0) runpos[nruns] = n;
     t.sync();
     Graph g = graph_alloc(t, sc, nruns);
@@ -306,7 +310,7 @@ __device__ Graph graph_contract_sorted(const Team &t, Scratch &sc, char *sm, con
         g.row[r] = (int32_t)(key >> nb);
         g.col[r] = (int32_t)(key & mask);
         if (e - s <= 32) {
-            g.cost[r] = rsum_serial((int)(e - s), [&](int k) { return v1[s + k]; });
+            g.cost[r] = rsum_serial((int)(e - s), [=](int k) { return v1[s + k]; });
         } else {
             int q = atomicAdd(nlong, 1);
             longq[q] = (int32_t)r;
@@ -317,7 +321,7 @@ __device__ Graph graph_contract_sorted(const Team &t, Scratch &sc, char *sm, con
     for (int64_t q = team_warp(t); q < nl; q += team_nwarps(t)) {
         int64_t r = longq[q];
         int64_t s = runpos[r], e = runpos[r + 1];
-        float v = rsum_warp(e - s, [&](int64_t k) { return v1[s + k]; });
+        float v = rsum_warp(e - s, [=](int64_t k) { return v1[s + k]; });
         if (lane_id() == 0) g.cost[r] = v;
     }
     t.sync();
@@ -329,8 +333,8 @@ __device__ Graph graph_contract_sorted(const Team &t, Scratch &sc, char *sm, con
     Graph h = graph_alloc(t, sc, nruns);
     if (!sc.arena.ok()) return out;
     const int64_t nk = team_compact(
-        t, sc, sm, nruns, [&](int64_t r) { return g.row[r] != g.col[r]; },
-        [&](int64_t r, int64_t p) {
+        t, sc, sm, nruns, [=](int64_t r) { return g.row[r] != g.col[r]; },
+        [=](int64_t r, int64_t p) {
             h.row[p] = g.row[r];
             h.col[p] = g.col[r];
             h.cost[p] = g.cost[r];
@@ -366,9 +370,10 @@ __device__ Graph graph_contract_sorted(const Team &t, Scratch &sc, char *sm, con
 // (one radix sort of every edge's packed keys) remains for edge lists of
 // 2^31 edges or more.  Both give the same graph bit for bit.
 template <class Team>
-__device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Graph &A, const int32_t *map,
+__device__ __noinline__ Graph graph_contract(const Team &t, Scratch &sc, char *, const Graph &A, const int32_t *map,
                                 int32_t map_max, int *bad)
 {
+    char *sm = team_smem();
     const int64_t n = A.n;
     Graph out = A;
     if (n == 0 || n >= (int64_t(1) << 31)) return graph_contract_sorted(t, sc, sm, A, map, map_max, bad);
@@ -391,16 +396,16 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
     }
     const bool done = team_bucket_sort_ex(
         t, sc, sm, n, nbk,
-        [&](int64_t e) -> int64_t {
+        [=](int64_t e) -> int64_t {
             const int32_t a = map[A.row[e]], b = map[A.col[e]];
             const int32_t lo = a < b ? a : b, hi = a < b ? b : a;
             return ((int64_t)hi << 32) | (uint32_t)lo;
         },
-        [&](int64_t e) { return lohi[e].x; },
-        [&](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].y << 32) | (uint64_t)e; },
-        [&](int64_t e) { return __float_as_int(A.cost[e]); }, sk, sbits, bst, sbk, PH_CSORT_SLOT,
-        [&](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].x << nbh) | (uint32_t)lohi[e].y; },
-        2 * nbh, [&](int64_t e, int64_t w) { lohi[e] = make_int2((int32_t)(uint32_t)w, (int32_t)(w >> 32)); });
+        [=](int64_t e) { return lohi[e].x; },
+        [=](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].y << 32) | (uint64_t)e; },
+        [=](int64_t e) { return __float_as_int(A.cost[e]); }, sk, sbits, bst, sbk, PH_CSORT_SLOT,
+        [=](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].x << nbh) | (uint32_t)lohi[e].y; },
+        2 * nbh, [=](int64_t e, int64_t w) { lohi[e] = make_int2((int32_t)(uint32_t)w, (int32_t)(w >> 32)); });
     if (!done) {
         sc.arena.release(m);
         return graph_contract_sorted(t, sc, sm, A, map, map_max, bad);
@@ -429,7 +434,7 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
     //    self-loop).  Then a pass over the runs sums each one, its end being
     //    the next run's start: runs of up to 32 edges by one thread, longer
     //    ones by a warp afterwards.
-    auto head = [&](int64_t p) {
+    auto head = [=](int64_t p) {
         return p == 0 || sbk[p] != sbk[p - 1] || (sk[p] >> 32) != (sk[p - 1] >> 32);
     };
     // lohi is dead after the sort: its two halves hold the runs' starts and slots
@@ -440,11 +445,11 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
     int32_t dloc = -1;
     const int64_t packed = team_scan<Team, int64_t>(
         t, sc, sm, n,
-        [&](int64_t p) -> int64_t {
+        [=](int64_t p) -> int64_t {
             if (!head(p)) return 0;
             return (int64_t(1) << 32) | ((int32_t)(sk[p] >> 32) != sbk[p] ? 1 : 0);
         },
-        [&](int64_t p, int64_t pre, int64_t v) {
+        [=, &dloc](int64_t p, int64_t pre, int64_t v) {
             if (!v) return;
             const int64_t k = pre & 0xffffffffll, r = pre >> 32;
             const int32_t b = sbk[p], hi = (int32_t)(sk[p] >> 32);
@@ -467,7 +472,7 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
     if (lane_id() == 0 && dloc >= 0) atomicMax(&fl[2], dloc);
     const float *cost_sorted = reinterpret_cast<const float *>(sbits);
     // a run's sum goes to its edge; a self-loop's negative sum is a bad contraction
-    auto finish = [&](int32_t k, float sum) {
+    auto finish = [=](int32_t k, float sum) {
         if (k >= 0)
             h.cost[k] = sum;
         else if (sum < 0.0f)
@@ -478,7 +483,7 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
         constexpr int U = 4;
         const int64_t S = t.size();
         int64_t r0 = t.rank();
-        auto one = [&](int64_t r, int32_t s, int32_t e, int32_t k) {
+        auto one = [=](int64_t r, int32_t s, int32_t e, int32_t k) {
             const int32_t len = e - s;
             if (len <= RSUM_THREAD_MAX)
                 finish(k, rsum_upto8(cost_sorted + s, len));
@@ -516,11 +521,11 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
         if (!sc.arena.ok()) return out;
         nchunks = team_scan<Team, int64_t>(
             t, sc, sm, nl,
-            [&](int64_t q) -> int64_t {
+            [=](int64_t q) -> int64_t {
                 const int64_t len = longq[q].y - longq[q].x;
                 return len > RSUM_CHUNK ? (len + RSUM_CHUNK - 1) / RSUM_CHUNK : 0;
             },
-            [&](int64_t q, int64_t pre, int64_t) { coff[q] = (int32_t)pre; });
+            [=](int64_t q, int64_t pre, int64_t) { coff[q] = (int32_t)pre; });
         chunk_sum = sc.arena.take<double>(nchunks + 1);
         if (!sc.arena.ok()) return out;
     }
@@ -528,7 +533,7 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
         if (w < nl) {
             const int4 L = longq[w];
             if (L.y - L.x <= RSUM_CHUNK) {
-                const float v = (float)rsum_chunk_warp(L.y - L.x, [&](int64_t x) { return cost_sorted[L.x + x]; });
+                const float v = (float)rsum_chunk_warp(L.y - L.x, [=](int64_t x) { return cost_sorted[L.x + x]; });
                 if (lane_id() == 0) finish(L.z, v);
             }
         } else {
@@ -545,7 +550,7 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
             const int4 L = longq[lo];
             const int64_t base = L.x + (g - coff[lo]) * RSUM_CHUNK;
             const int64_t len = L.y - base < RSUM_CHUNK ? L.y - base : RSUM_CHUNK;
-            const double d = rsum_chunk_warp(len, [&](int64_t x) { return cost_sorted[base + x]; });
+            const double d = rsum_chunk_warp(len, [=](int64_t x) { return cost_sorted[base + x]; });
             if (lane_id() == 0) chunk_sum[g] = d;
         }
     }
@@ -569,7 +574,7 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
     int32_t mc = -1;
     float mn = 3.4e38f;
     team_maxi_minf(
-        t, sc, sm, nk, -1, 3.4e38f, [&](int64_t e) { return h.col[e]; }, [&](int64_t e) { return h.cost[e]; }, mc,
+        t, sc, sm, nk, -1, 3.4e38f, [=](int64_t e) { return h.col[e]; }, [=](int64_t e) { return h.cost[e]; }, mc,
         mn);
     const int32_t dmax = uread(&fl[2]);
     h.n = nk;
@@ -587,11 +592,12 @@ __device__ Graph graph_contract(const Team &t, Scratch &sc, char *sm, const Grap
 // renumber the nodes that have edges to 0..k-1.  Outputs live in the
 // temporaries; idmap (size = max id + 1) maps original ids to new ones.
 template <class Team>
-__device__ int64_t sanitize_edges(const Team &t, Scratch &sc, char *sm, const int32_t *I, const int32_t *J,
+__device__ __noinline__ int64_t sanitize_edges(const Team &t, Scratch &sc, char *, const int32_t *I, const int32_t *J,
                                   const float *Cc, int64_t n, int32_t *&si, int32_t *&sj, float *&sw, int32_t *&idmap,
                                   int32_t &idsize)
 {
-    int32_t mx = team_max<Team, int32_t>(t, sc, sm, n, 0, [&](int64_t e) { return I[e] > J[e] ? I[e] : J[e]; });
+    char *sm = team_smem();
+    int32_t mx = team_max<Team, int32_t>(t, sc, sm, n, 0, [=](int64_t e) { return I[e] > J[e] ? I[e] : J[e]; });
     idsize = mx + 1;
     const int nb = bits_for((uint64_t)mx);
     si = sc.arena.take<int32_t>(n + 1);
@@ -612,8 +618,8 @@ __device__ int64_t sanitize_edges(const Team &t, Scratch &sc, char *sm, const in
     team_sort_pairs(t, sc, sm, k1, v1, k2, v2, n, 2 * nb);
     const uint64_t mask = (nb == 0) ? 0 : ((uint64_t(1) << nb) - 1);
     const int64_t u = team_compact(
-        t, sc, sm, n, [&](int64_t k) { return k == 0 || k1[k] != k1[k - 1]; },
-        [&](int64_t k, int64_t p) {
+        t, sc, sm, n, [=](int64_t k) { return k == 0 || k1[k] != k1[k - 1]; },
+        [=](int64_t k, int64_t p) {
             int32_t a = (int32_t)(k1[k] >> nb), b = (int32_t)(k1[k] & mask);
             si[p] = a;
             sj[p] = b;
@@ -622,8 +628,8 @@ __device__ int64_t sanitize_edges(const Team &t, Scratch &sc, char *sm, const in
             idmap[b] = 1;
         });
     team_scan<Team, int64_t>(
-        t, sc, sm, idsize, [&](int64_t v) -> int64_t { return idmap[v]; },
-        [&](int64_t v, int64_t pre, int64_t) { idmap[v] = (int32_t)pre; });
+        t, sc, sm, idsize, [=](int64_t v) -> int64_t { return idmap[v]; },
+        [=](int64_t v, int64_t pre, int64_t) { idmap[v] = (int32_t)pre; });
     for (int64_t e = t.rank(); e < u; e += t.size()) {
         si[e] = idmap[si[e]];
         sj[e] = idmap[sj[e]];
@@ -648,8 +654,8 @@ __device__ Graph graph_contract_raw(const Team &t, Scratch &sc, char *sm, const 
     if (!sc.arena.ok()) return out;
     contract_sorted_keys(t, sc, sm, A, map, map_max, nb, k1, v1, k2, v2);
     const int64_t nruns = team_compact(
-        t, sc, sm, n, [&](int64_t k) { return k == 0 || k1[k] != k1[k - 1]; },
-        [&](int64_t k, int64_t r) { runpos[r] = k; });
+        t, sc, sm, n, [=](int64_t k) { return k == 0 || k1[k] != k1[k - 1]; },
+        [=](int64_t k, int64_t r) { runpos[r] = k; });
     if (t.rank() == 0) runpos[nruns] = n;
     t.sync();
     Graph g = graph_alloc(t, sc, nruns);
@@ -660,13 +666,13 @@ __device__ Graph graph_contract_raw(const Team &t, Scratch &sc, char *sm, const 
         uint64_t key = k1[s];
         g.row[r] = (int32_t)(key >> nb);
         g.col[r] = (int32_t)(key & mask);
-        g.cost[r] = (e - s <= 32) ? rsum_serial((int)(e - s), [&](int k) { return v1[s + k]; }) : 0.0f;
+        g.cost[r] = (e - s <= 32) ? rsum_serial((int)(e - s), [=](int k) { return v1[s + k]; }) : 0.0f;
     }
     t.sync();
     for (int64_t r = team_warp(t); r < nruns; r += team_nwarps(t)) {
         int64_t s = runpos[r], e = runpos[r + 1];
         if (e - s <= 32) continue;
-        float v = rsum_warp(e - s, [&](int64_t k) { return v1[s + k]; });
+        float v = rsum_warp(e - s, [=](int64_t k) { return v1[s + k]; });
         if (lane_id() == 0) g.cost[r] = v;
     }
     t.sync();
@@ -692,9 +698,10 @@ struct Csr {
 };
 
 template <class Team, class Keep>
-__device__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char *sm, const Graph &A, int32_t nrows, Keep keep,
+__device__ __noinline__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char *, const Graph &A, int32_t nrows, Keep keep,
                                    bool with_eid, int64_t *kept_idx_out = nullptr)
 {
+    char *sm = team_smem();
     Csr C;
     C.nrows = nrows;
     C.m2 = 0;
@@ -704,7 +711,7 @@ __device__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char *sm, const G
     C.off = sc.arena.take<int32_t>((int64_t)nrows + 2);
     if (!sc.arena.ok()) return C;
     for (int64_t v = t.rank(); v <= nrows; v += t.size()) deg[v] = 0;
-    const int64_t m = team_compact(t, sc, sm, A.n, keep, [&](int64_t e, int64_t p) { kidx[p] = e; });
+    const int64_t m = team_compact(t, sc, sm, A.n, keep, [=](int64_t e, int64_t p) { kidx[p] = e; });
     C.m2 = 2 * m;
     C.adj = sc.arena.take<int32_t>(2 * m + 1);
     C.w = sc.arena.take<float>(2 * m + 1);
@@ -729,16 +736,16 @@ __device__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char *sm, const G
     }
     t.sync();
     team_scan<Team, int64_t>(
-        t, sc, sm, (int64_t)nrows, [&](int64_t v) -> int64_t { return deg[v]; },
-        [&](int64_t v, int64_t pre, int64_t) { C.off[v] = (int32_t)pre; });
+        t, sc, sm, (int64_t)nrows, [=](int64_t v) -> int64_t { return deg[v]; },
+        [=](int64_t v, int64_t pre, int64_t) { C.off[v] = (int32_t)pre; });
     // first position of each column among the column-sorted kept edges, and
     // of each row among the (row-sorted) kept edges
     team_scan<Team, int64_t>(
-        t, sc, sm, (int64_t)nrows, [&](int64_t v) -> int64_t { return infill[v]; },
-        [&](int64_t v, int64_t pre, int64_t) { colstart[v] = (int32_t)pre; });
+        t, sc, sm, (int64_t)nrows, [=](int64_t v) -> int64_t { return infill[v]; },
+        [=](int64_t v, int64_t pre, int64_t) { colstart[v] = (int32_t)pre; });
     team_scan<Team, int64_t>(
-        t, sc, sm, (int64_t)nrows, [&](int64_t v) -> int64_t { return deg[v] - infill[v]; },
-        [&](int64_t v, int64_t pre, int64_t) { rowstart[v] = (int32_t)pre; });
+        t, sc, sm, (int64_t)nrows, [=](int64_t v) -> int64_t { return deg[v] - infill[v]; },
+        [=](int64_t v, int64_t pre, int64_t) { rowstart[v] = (int32_t)pre; });
     if (t.rank() == 0) C.off[nrows] = (int32_t)(2 * m);
     t.sync();
     // 3. kept edges in column order, rows increasing within a column (a
@@ -748,7 +755,7 @@ __device__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char *sm, const G
     int32_t *bst = sc.arena.take<int32_t>((int64_t)nrows + 2);
     if (sc.arena.ok() && m < (int64_t(1) << 31) &&
         team_bucket_sort(
-            t, sc, sm, m, nrows, [&](int64_t p) { return A.col[kidx[p]]; }, [&](int64_t p) { return (uint64_t)p; },
+            t, sc, sm, m, nrows, [=](int64_t p) { return A.col[kidx[p]]; }, [=](int64_t p) { return (uint64_t)p; },
             k2, v2, bst)) {
         for (int64_t q = t.rank(); q < m; q += t.size()) {
             const int64_t p = (int64_t)k2[q];
@@ -788,9 +795,9 @@ __device__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char *sm, const G
 // lower bound of the directed graph: sum of min(0, c) (get_lb,
 // include/rama_utils.h:179-190), CSUM
 template <class Team>
-__device__ double graph_lb(const Team &t, Scratch &sc, const Graph &A)
+__device__ __noinline__ double graph_lb(const Team &t, Scratch &sc, const Graph &A)
 {
-    return team_csum(t, sc, A.n, [&](int64_t e) -> float {
+    return team_csum(t, sc, A.n, [=](int64_t e) -> float {
         const float c = A.cost[e];
         return c < 0.0f ? c : 0.0f;
     });
@@ -798,9 +805,10 @@ __device__ double graph_lb(const Team &t, Scratch &sc, const Graph &A)
 
 // compress_label_sequence (include/rama_utils.h:160-177)
 template <class Team>
-__device__ void compress_labels(const Team &t, Scratch &sc, char *sm, const int32_t *data, int64_t n,
+__device__ __noinline__ void compress_labels(const Team &t, Scratch &sc, char *, const int32_t *data, int64_t n,
                                 int32_t max_label, int32_t *out)
 {
+    char *sm = team_smem();
     uint64_t m = sc.arena.mark();
     int32_t *mask = sc.arena.take<int32_t>((int64_t)max_label + 2);
     if (!sc.arena.ok()) return;
@@ -809,8 +817,8 @@ __device__ void compress_labels(const Team &t, Scratch &sc, char *sm, const int3
     for (int64_t k = t.rank(); k < n; k += t.size()) mask[data[k]] = 1;
     t.sync();
     team_scan<Team, int64_t>(
-        t, sc, sm, (int64_t)max_label + 1, [&](int64_t l) -> int64_t { return mask[l]; },
-        [&](int64_t l, int64_t pre, int64_t) { mask[l] = (int32_t)pre; });
+        t, sc, sm, (int64_t)max_label + 1, [=](int64_t l) -> int64_t { return mask[l]; },
+        [=](int64_t l, int64_t pre, int64_t) { mask[l] = (int32_t)pre; });
     for (int64_t k = t.rank(); k < n; k += t.size()) out[k] = mask[data[k]];
     t.sync();
     sc.arena.release(m);

@@ -26,10 +26,12 @@ namespace rama {
 // atomicMax and the per-vertex match do not depend on the order: the map is
 // the same as with full passes.
 template <class Team>
-__device__ int32_t matching_contraction_map(const Team &t, Scratch &sc, char *sm, const Graph &A, float mm,
+__device__ __noinline__ int32_t matching_contraction_map(const Team &t, Scratch &sc, char *, const Graph &graph, float mm,
                                             int32_t *map_out, int32_t *M_out)
 {
-    int32_t mc = team_max<Team, int32_t>(t, sc, sm, A.n, -1, [&](int64_t e) { return A.col[e]; });
+    char *sm = team_smem();
+    const Graph A = graph;  // its pointers in registers
+    int32_t mc = team_max<Team, int32_t>(t, sc, sm, A.n, -1, [=](int64_t e) { return A.col[e]; });
     const int32_t M = mc + 1;
     *M_out = M;
     uint64_t mark = sc.arena.mark();
@@ -56,11 +58,7 @@ __device__ int32_t matching_contraction_map(const Team &t, Scratch &sc, char *sm
         return c >= 0.0f ? c : 0.0f;
     };
     auto counted = [cost](int64_t e) { return cost[e] >= 0.0f; };
-    double S;
-    if constexpr (std::is_same<Team, GridTeam>::value)
-        S = team_csum_count_outlined(t, sc, A.n, nonneg, counted, &K);
-    else
-        S = team_csum_count(t, sc, A.n, nonneg, counted, &K);
+    const double S = team_csum_count(t, sc, A.n, nonneg, counted, &K);
     int32_t prev = 0;
     if (K > 0) {
         const float sum_f = (float)(2.0 * S);
@@ -96,7 +94,7 @@ __device__ int32_t matching_contraction_map(const Team &t, Scratch &sc, char *sm
             // blockDim * MI edges with one atomic per list.
             constexpr int MI = 4;
             int32_t *wsum = reinterpret_cast<int32_t *>(sm);  // per warp: list count, touched count; then bases
-            auto offer_tile = [&](const int32_t (&u)[MI], const int32_t (&v)[MI], const uint32_t (&hb)[MI],
+            auto offer_tile = [=](const int32_t (&u)[MI], const int32_t (&v)[MI], const uint32_t (&hb)[MI],
                                   const bool (&live)[MI]) {
                 bool fu[MI], fv[MI];
 #pragma unroll
@@ -232,7 +230,7 @@ __device__ int32_t matching_contraction_map(const Team &t, Scratch &sc, char *sm
             // (the pairs are counted at their smaller end, one atomic per warp)
             int32_t mine = 0;
             auto offered = [](unsigned long long o) { return (int32_t)(~(uint32_t)(o & 0xffffffffull)); };
-            auto pair_up = [&](int32_t v, int32_t b, unsigned long long ob) {
+            auto pair_up = [=, &mine](int32_t v, int32_t b, unsigned long long ob) {
                 if (ob && offered(ob) == v && v < b) {
                     nm[b] = v;
                     matched[v] = 1;
@@ -287,10 +285,10 @@ __device__ int32_t matching_contraction_map(const Team &t, Scratch &sc, char *sm
     // among the roots
     int32_t *rank = reinterpret_cast<int32_t *>(offer[0]);  // the offers are dead by now
     team_scan<Team, int64_t>(
-        t, sc, sm, M, [&](int64_t v) -> int64_t { return nm[v] == (int32_t)v ? 1 : 0; },
-        [&](int64_t v, int64_t pre, int64_t) { rank[v] = (int32_t)pre; });
+        t, sc, sm, M, [=](int64_t v) -> int64_t { return nm[v] == (int32_t)v ? 1 : 0; },
+        [=](int64_t v, int64_t pre, int64_t) { rank[v] = (int32_t)pre; });
     team_for_batched(
-        t, M, [&](int64_t v) { return rank[nm[v]]; }, [&](int64_t v, int32_t r) { map_out[v] = r; });
+        t, M, [=](int64_t v) { return rank[nm[v]]; }, [=](int64_t v, int32_t r) { map_out[v] = r; });
     t.sync();
     prof_mark(t, sc, PH_MATCH_LABELS);
     sc.arena.release(mark);

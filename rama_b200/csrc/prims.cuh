@@ -3,8 +3,8 @@
 //
 // All results are independent of the team size: order-sensitive primitives
 // split the input into one contiguous chunk per CTA, and the floating-point
-// sums follow fixed reduction trees (CSUM, RSUM) that are defined by element
-// index only.
+// sums either follow a fixed reduction tree defined by element index only
+// (RSUM) or carry enough bits that the order does not show (CSUM).
 #pragma once
 #include <cstdint>
 #include <type_traits>
@@ -23,7 +23,7 @@ constexpr unsigned FULL = 0xffffffffu;
 // ---------------------------------------------------------------------------
 struct Scratch {
     Arena arena;
-    char *part[2];  // each >= 16 * (nblocks + 2) bytes
+    char *part[2];  // each >= 32 * (nblocks + 2) bytes
     int32_t *err;   // set when a bounded wait gave up (zeroed at the start of a solve)
     int parity;
     double alg_bytes;  // algorithmic bytes of the work done (team-uniform tally)
@@ -40,7 +40,7 @@ struct Scratch {
 
 // A workspace of `bytes` bytes at `base` (256-byte aligned) holds the two
 // partial buffers, the error word and then the arena.
-constexpr uint64_t SCRATCH_PART_BYTES = 16 * 4096;  // >= 16 * (max CTAs + 2)
+constexpr uint64_t SCRATCH_PART_BYTES = 16 * 4096;  // >= 32 * (max CTAs + 2)
 
 __device__ __forceinline__ Scratch scratch_over(char *base, uint64_t bytes)
 {
@@ -490,16 +490,29 @@ template <class Team, class Keep, class Emit>
 __device__ int64_t team_compact(const Team &t, Scratch &sc, char *sm, int64_t n, Keep keep, Emit emit)
 {
     return team_scan<Team, int64_t>(
-        t, sc, sm, n, [&](int64_t i) -> int64_t { return keep(i) ? 1 : 0; },
-        [&](int64_t i, int64_t pos, int64_t v) {
+        t, sc, sm, n, [=](int64_t i) -> int64_t { return keep(i) ? 1 : 0; },
+        [=](int64_t i, int64_t pos, int64_t v) {
             if (v) emit(i, pos);
         });
 }
 
 // ---------------------------------------------------------------------------
-// CSUM: compensated FP64 sum over a fixed tree (chunks of 4096 elements, 32
-// lane-strided TwoSum partials per chunk, pairwise tree over lanes; the same
-// scheme over the chunk partials).  Bit-identical to the CPU oracle.
+// CSUM: compensated FP64 sum of floats.  Every thread adds its elements with
+// TwoSum (the sum and its error, about 106 bits together), the pairs of a CTA
+// and then of the team are merged the same way, and the result is rounded
+// once.  The error of the pair is some 2^-35 of the result's last place at
+// 25 M elements (a few hundred roundings of the compensation, each 2^-53 of
+// it), so the result is the correctly rounded sum whatever the order and the
+// team, and equals the CPU oracle's, unless the exact sum comes that close to
+// the middle between two doubles without lying on it.
+//
+// What bounds it: the passes over memory for large n (7 FP64 additions per
+// element take less), the team sync and the L2 round trips for small n.  So
+// the elements are strided over all threads and there is one team sync.  One
+// warp per 4,096 elements with its 128-step chain, and two team syncs, took
+// 1.34 ms
+// for the six matching thresholds of the 24.8 M edge volume (with what is timed
+// beside them); this takes 0.74.
 // ---------------------------------------------------------------------------
 struct csum_t {
     double s, c;
@@ -516,114 +529,106 @@ __device__ __forceinline__ csum_t cs_merge(csum_t a, csum_t b)
     return r;
 }
 
-__device__ __forceinline__ csum_t cs_warp_tree(csum_t a)
+__device__ __forceinline__ csum_t cs_add(csum_t a, float x) { return cs_merge(a, csum_t{(double)x, 0.0}); }
+
+// The totals over the team of two pairs per thread, rounded, on every thread
+// (a count rides along as a second pair: its additions are exact).  One team
+// sync, which also makes the caller's earlier stores visible to the team.
+struct csum2_t {
+    double a, b;
+};
+
+template <class Team>
+__device__ __noinline__ csum2_t team_csum_fold(const Team &t, Scratch &sc, csum_t a, csum_t b)
 {
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        csum_t o;
-        o.s = __shfl_down_sync(FULL, a.s, off);
-        o.c = __shfl_down_sync(FULL, a.c, off);
-        if ((lane_id() & (2 * off - 1)) == 0) a = cs_merge(a, o);
+    __shared__ csum_t wa[32], wb[32];
+    __shared__ csum2_t res;
+    // merging is commutative, so a butterfly leaves the same pair on every lane
+    auto fold = [&](int lanes) {
+        for (int off = 1; off < lanes; off <<= 1) {
+            csum_t x, y;
+            x.s = __shfl_xor_sync(FULL, a.s, off);
+            x.c = __shfl_xor_sync(FULL, a.c, off);
+            y.s = __shfl_xor_sync(FULL, b.s, off);
+            y.c = __shfl_xor_sync(FULL, b.c, off);
+            a = cs_merge(a, x);
+            b = cs_merge(b, y);
+        }
+    };
+    const int nw = blockDim.x >> 5;
+    fold(32);
+    if (lane_id() == 0) {
+        wa[warp_in_block()] = a;
+        wb[warp_in_block()] = b;
     }
-    return a;
+    __syncthreads();
+    csum_t *part = reinterpret_cast<csum_t *>(sc.next_part());  // 32 B per CTA
+    if (warp_in_block() == 0) {
+        a = lane_id() < nw ? wa[lane_id()] : csum_t{0.0, 0.0};
+        b = lane_id() < nw ? wb[lane_id()] : csum_t{0.0, 0.0};
+        fold(nw);
+        if (lane_id() == 0) {
+            if (t.nblocks() == 1) {
+                res.a = __dadd_rn(a.s, a.c);
+                res.b = __dadd_rn(b.s, b.c);
+            } else {
+                part[2 * t.block()] = a;
+                part[2 * t.block() + 1] = b;
+            }
+        }
+    }
+    t.sync();
+    if (t.nblocks() > 1) {
+        if (warp_in_block() == 0) {
+            a = b = csum_t{0.0, 0.0};
+            const double2 *p = reinterpret_cast<const double2 *>(part);
+            for (int k = lane_id(); k < t.nblocks(); k += 32) {
+                const double2 x = __ldcg(p + 2 * k), y = __ldcg(p + 2 * k + 1);
+                a = cs_merge(a, csum_t{x.x, x.y});
+                b = cs_merge(b, csum_t{y.x, y.y});
+            }
+            fold(32);
+            if (lane_id() == 0) {
+                res.a = __dadd_rn(a.s, a.c);
+                res.b = __dadd_rn(b.s, b.c);
+            }
+        }
+        __syncthreads();
+    }
+    // the next fold writes `res` after a sync that follows this read
+    return res;
 }
 
-// returns the sum on every thread; two team syncs.  *count receives the
-// number of k with cnt(k) (an exact integer sum computed in the same pass).
+// The sum of get(k) over [0, n) on every thread; *count receives the number
+// of k with cnt(k).
 template <class Team, class Get, class Cnt>
 __device__ double team_csum_count(const Team &t, Scratch &sc, int64_t n, Get get, Cnt cnt, int64_t *count)
 {
-    const int64_t nch = (n + 4095) / 4096;
-    uint64_t m = sc.arena.mark();
-    csum_t *parts = sc.arena.take<csum_t>(nch + 1);
-    int64_t *pcnt = sc.arena.take<int64_t>(nch + 1);
-    double *res = reinterpret_cast<double *>(sc.next_part());
-    if (sc.arena.ok()) {
-        const int64_t w = team_warp(t), nw = team_nwarps(t);
-        for (int64_t ch = w; ch < nch; ch += nw) {
-            csum_t a = {0.0, 0.0};
-            int64_t c = 0;
-            const int64_t b0 = ch * 4096 + lane_id();
-            // 8 of the lane's 128 elements loaded at a time, merged in order;
-            // the values stay as get returns them (a float takes one register)
-            // until their merge, and full chunks need no bounds checks
-            using V = decltype(get(int64_t(0)));
-            if (ch * 4096 + 4096 <= n) {
-                for (int k = 0; k < 128; k += 8) {
-                    V x[8];
+    csum_t a = {0.0, 0.0};
+    int64_t c = 0;
+    {
+        // eight strides at a time, loads issued together
+        constexpr int U = 8;
+        const int64_t S = t.size();
+        int64_t i = t.rank();
+        for (; i + (U - 1) * S < n; i += U * S) {
+            float x[U];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const int64_t idx = b0 + 32 * (k + j);
-                        x[j] = get(idx);
-                        c += cnt(idx) ? 1 : 0;
-                    }
+            for (int k = 0; k < U; ++k) {
+                x[k] = get(i + k * S);
+                c += cnt(i + k * S) ? 1 : 0;
+            }
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) a = cs_merge(a, csum_t{(double)x[j], 0.0});
-                }
-            } else {
-                for (int k = 0; k < 128; ++k) {
-                    const int64_t idx = b0 + 32 * k;
-                    if (idx < n) {
-                        a = cs_merge(a, csum_t{(double)get(idx), 0.0});
-                        c += cnt(idx) ? 1 : 0;
-                    }
-                }
-            }
-            a = cs_warp_tree(a);
-            c = warp_sum(c);
-            if (lane_id() == 0) {
-                parts[ch] = a;
-                pcnt[ch] = c;
-            }
+            for (int k = 0; k < U; ++k) a = cs_add(a, x[k]);
+        }
+        for (; i < n; i += S) {
+            a = cs_add(a, get(i));
+            c += cnt(i) ? 1 : 0;
         }
     }
-    t.sync();
-    if (sc.arena.ok() && t.block() == 0 && warp_in_block() == 0) {
-        csum_t a = {0.0, 0.0};
-        int64_t c = 0;
-        // a lane merges partials k, k + 32, ... in order, eight loaded at a time
-        int64_t k = lane_id();
-        for (; k + 7 * 32 < nch; k += 8 * 32) {
-            csum_t x[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                x[j] = parts[k + 32 * j];
-                c += pcnt[k + 32 * j];
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) a = cs_merge(a, x[j]);
-        }
-        for (; k < nch; k += 32) {
-            a = cs_merge(a, parts[k]);
-            c += pcnt[k];
-        }
-        a = cs_warp_tree(a);
-        c = warp_sum(c);
-        if (lane_id() == 0) {
-            res[0] = __dadd_rn(a.s, a.c);
-            reinterpret_cast<int64_t *>(res)[1] = c;
-        }
-    }
-    t.sync();
-    double r = uread(&res[0]);
-    *count = uread(&reinterpret_cast<int64_t *>(res)[1]);
-    sc.arena.release(m);
-    // `res` lies in one of the two partial buffers: the next primitive uses the
-    // other one, and the one after it can write this one only after a team
-    // sync that every thread reaches after this read
-    return r;
-}
-
-// The same in a function of its own.  Inlined into the whole-GPU solve, the
-// matching threshold's sum took about 1.7x as long as called out of line
-// (the solver's live state crowds the FP64 loop).  Elsewhere (the bound of
-// message passing, the smaller teams) the call cost more than it saved, so
-// only that call site uses it.
-template <class Team, class Get, class Cnt>
-__device__ __noinline__ double team_csum_count_outlined(const Team &t, Scratch &sc, int64_t n, Get get, Cnt cnt,
-                                                        int64_t *count)
-{
-    return team_csum_count(t, sc, n, get, cnt, count);
+    const csum2_t r = team_csum_fold(t, sc, a, csum_t{(double)c, 0.0});
+    *count = (int64_t)r.b;
+    return r.a;
 }
 
 template <class Team, class Get>
@@ -742,7 +747,7 @@ __device__ __forceinline__ float rsum_warp(int64_t n, Get v)
     for (int64_t c = 0; c * RSUM_CHUNK < n; ++c) {
         const int64_t base = c * RSUM_CHUNK;
         const int64_t len = n - base < RSUM_CHUNK ? n - base : RSUM_CHUNK;
-        const double d = rsum_chunk_warp(len, [&](int64_t k) { return v(base + k); });
+        const double d = rsum_chunk_warp(len, [=](int64_t k) { return v(base + k); });
         if (lane_id() == (int)(c & 31)) acc = __dadd_rn(acc, d);
     }
     return (float)rsum_lane_tree(acc);
@@ -885,10 +890,13 @@ __device__ __forceinline__ unsigned warp_peers9(unsigned label)
 }
 
 template <class Team, class V>
-__device__ void team_sort_pairs(const Team &t, Scratch &sc, char *sm, uint64_t *&keys, V *&vals, uint64_t *&keys2,
-                                V *&vals2, int64_t n, int bits)
+__device__ __noinline__ void team_sort_pairs(const Team &t, Scratch &sc, char *, uint64_t *&keys_io, V *&vals_io,
+                                             uint64_t *&keys2_io, V *&vals2_io, int64_t n, int bits)
 {
     if (n <= 1 || bits <= 0) return;
+    char *sm = team_smem();
+    uint64_t *keys = keys_io, *keys2 = keys2_io;
+    V *vals = vals_io, *vals2 = vals2_io;
     using W = typename SortWord<V>::type;
     constexpr int ITEMS = sizeof(V) == 8 ? SORT_ITEMS / 2 : SORT_ITEMS;
     const int P = (bits + 7) / 8;
@@ -1034,6 +1042,10 @@ __device__ void team_sort_pairs(const Team &t, Scratch &sc, char *sm, uint64_t *
         vals = vals2;
         vals2 = tv;
     }
+    keys_io = keys;
+    keys2_io = keys2;
+    vals_io = vals;
+    vals2_io = vals2;
     sc.arena.release(am);
 }
 
@@ -1178,8 +1190,8 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
     // bucket starts; buckets of more than 64 items go to the warp and CTA
     // lists (any order); one of more than BUCKET_MAX ends the sort
     team_scan<Team, int64_t>(
-        t, sc, sm, nb, [&](int64_t b) -> int64_t { return bstart[b]; },
-        [&](int64_t b, int64_t pre, int64_t c) {
+        t, sc, sm, nb, [=](int64_t b) -> int64_t { return bstart[b]; },
+        [=](int64_t b, int64_t pre, int64_t c) {
             bstart[b] = (int32_t)pre;
             if (c > BUCKET_MAX)
                 nlist[2] = 1;
@@ -1235,7 +1247,7 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
     {
         // the rank of item p in its bucket; -1: sorted below (a bucket of
         // 65..BUCKET_MAX items is copied as it is) or by the big path
-        auto rank_in_bucket = [&](int64_t p, int32_t s, int32_t e, uint64_t key) -> int32_t {
+        auto rank_in_bucket = [=](int64_t p, int32_t s, int32_t e, uint64_t key) -> int32_t {
             if (e - s > 64) return e - s <= BUCKET_MAX ? (int32_t)p : -1;
             int32_t r = 0;
             for (int32_t q = s; q < e; ++q) {
@@ -1339,12 +1351,12 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
     if constexpr (!std::is_same<BigKey, NoBigKey>::value) if (has_big) {
         // the buckets beyond BUCKET_MAX: their items in input order, a stable
         // radix sort of big_key, then each into its bucket's range
-        auto bsize = [&](int64_t i) {
+        auto bsize = [=](int64_t i) {
             const int32_t b = (int32_t)bucket(i);
             return bstart[b + 1] - bstart[b];
         };
         uint64_t bm = sc.arena.mark();
-        const int64_t nbig = team_sum<Team, int64_t>(t, sc, sm, n, [&](int64_t i) -> int64_t {
+        const int64_t nbig = team_sum<Team, int64_t>(t, sc, sm, n, [=](int64_t i) -> int64_t {
             return bsize(i) > BUCKET_MAX ? 1 : 0;
         });
         uint64_t *bk1 = sc.arena.take<uint64_t>(nbig + 1), *bk2 = sc.arena.take<uint64_t>(nbig + 1);
@@ -1352,8 +1364,8 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
         int32_t *kfirst = sc.arena.take<int32_t>((int64_t)nb + 1);
         if (!sc.arena.ok()) return false;
         team_compact(
-            t, sc, sm, n, [&](int64_t i) { return bsize(i) > BUCKET_MAX; },
-            [&](int64_t i, int64_t k) {
+            t, sc, sm, n, [=](int64_t i) { return bsize(i) > BUCKET_MAX; },
+            [=](int64_t i, int64_t k) {
                 bk1[k] = big_key(i);
                 bv1[k] = (int32_t)i;
             });

@@ -79,7 +79,7 @@ __device__ void solve_instance(const Team &t, char *sm, Scratch sc, Instance *io
     int64_t num_labels = 0;
     int64_t eafter = 0;
     uint64_t *slot = reinterpret_cast<uint64_t *>(sc.arena.take<uint64_t>(4));
-    const int64_t bad_in = team_sum<Team, int64_t>(t, sc, sm, n, [&](int64_t e) -> int64_t {
+    const int64_t bad_in = team_sum<Team, int64_t>(t, sc, sm, n, [=](int64_t e) -> int64_t {
         int32_t a = I[e], b = J[e];
         return (a < 0 || b < 0 || a == b) ? 1 : 0;
     });
@@ -157,11 +157,11 @@ __device__ void solve_instance(const Team &t, char *sm, Scratch sc, Instance *io
                     // map_node_labels (src/rama_cuda.cu:32-52)
                     team_for_batched(
                         t, N0,
-                        [&](int64_t v) {
+                        [=](int64_t v) {
                             const int32_t m = nm[v];
                             return m < msize ? map[m] : m;
                         },
-                        [&](int64_t v, int32_t m) { nm[v] = m; });
+                        [=](int64_t v, int32_t m) { nm[v] = m; });
                     t.sync();
                     prof_mark(t, sc, PH_OTHER);
                     ++rounds;

@@ -121,9 +121,8 @@ __device__ void run_step(const Team &t, char *sm, Scratch sc, rama_step_args *a)
             t.sync();
             Mp mp;
             if (mp_build(t, sc, sm, A, tb, mp)) {
-                double lb0 = mp_lower_bound(t, sc, mp);
-                for (int it = 0; it < a->num_iter; ++it) mp_iteration(t, mp);
-                double lb1 = mp_lower_bound(t, sc, mp);
+                double lb0 = 0.0;
+                const double lb1 = mp_run(t, sc, mp, a->num_iter, -INFINITY, &lb0);
                 Graph g;
                 g.row = mp.row;
                 g.col = mp.col;

@@ -54,6 +54,15 @@ __device__ __forceinline__ T uread(const T *p)
     return *(const volatile T *)p;
 }
 
+// The CTA's dynamic shared memory.  The solver's phases are functions of their
+// own (__noinline__): each asks for it here instead of taking a pointer, so
+// that its accesses compile to shared-memory instructions.
+__device__ __forceinline__ char *team_smem()
+{
+    extern __shared__ __align__(16) char sm[];
+    return sm;
+}
+
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_in_block() { return threadIdx.x >> 5; }
 __device__ __forceinline__ unsigned lanemask_lt() { return (1u << lane_id()) - 1u; }

@@ -23,9 +23,10 @@ namespace rama {
 // chosen[e] = 1 for forest edges.
 // ---------------------------------------------------------------------------
 template <class Team, class EI, class EJ, class EW>
-__device__ bool team_msf(const Team &t, Scratch &sc, char *sm, int64_t m, int32_t nv0, EI ei, EJ ej, EW ew,
+__device__ __noinline__ bool team_msf(const Team &t, Scratch &sc, char *, int64_t m, int32_t nv0, EI ei, EJ ej, EW ew,
                          uint8_t *chosen)
 {
+    char *sm = team_smem();
     uint64_t mark = sc.arena.mark();
     const int64_t n2 = 2 * m;
     int32_t *u = sc.arena.take<int32_t>(n2 + 1), *v = sc.arena.take<int32_t>(n2 + 1);
@@ -97,14 +98,14 @@ __device__ bool team_msf(const Team &t, Scratch &sc, char *sm, int64_t m, int32_
         if (jumps == 62) ok = false;
         // renumber roots by rank (sort + mark_segments + scan, :285-298)
         const int64_t nroots = team_compact(
-            t, sc, sm, nv, [&](int64_t x) { return succ2[x] == (int32_t)x; },
-            [&](int64_t x, int64_t p) { newid[x] = (int32_t)p; });
+            t, sc, sm, nv, [=](int64_t x) { return succ2[x] == (int32_t)x; },
+            [=](int64_t x, int64_t p) { newid[x] = (int32_t)p; });
         for (int64_t x = t.rank(); x < nv; x += t.size()) succ[x] = newid[succ2[x]];
         t.sync();
         // keep edges between different super vertices, relabelled (:300-334)
         const int64_t ne2 = team_compact(
-            t, sc, sm, ne, [&](int64_t e) { return succ[u[e]] != succ[v[e]]; },
-            [&](int64_t e, int64_t p) {
+            t, sc, sm, ne, [=](int64_t e) { return succ[u[e]] != succ[v[e]]; },
+            [=](int64_t e, int64_t p) {
                 u2[p] = succ[u[e]];
                 v2[p] = succ[v[e]];
                 wk2[p] = wk[e];
@@ -145,7 +146,7 @@ struct Forest {
 template <class Team>
 __device__ void forest_offsets(const Team &t, Forest &F)
 {
-    team_offsets(t, F.m2, F.nn, [&](int64_t k) { return F.r[k]; }, F.off);
+    team_offsets(t, F.m2, F.nn, [=](int64_t k) { return F.r[k]; }, F.off);
 }
 
 __device__ __forceinline__ int32_t forest_find(const Forest &F, int32_t a, int32_t b)
@@ -164,8 +165,10 @@ __device__ __forceinline__ int32_t forest_find(const Forest &F, int32_t a, int32
 // drop the undirected edges whose entry is flagged in F.inv (both
 // directions); returns whether anything was removed.  F.inv is cleared.
 template <class Team>
-__device__ bool forest_remove_flagged(const Team &t, Scratch &sc, char *sm, Forest &F)
+__device__ __noinline__ bool forest_remove_flagged(const Team &t, Scratch &sc, char *, Forest &state)
 {
+    char *sm = team_smem();
+    Forest F = state;  // pointers in registers
     for (int64_t k = t.rank(); k < F.m2; k += t.size()) {
         if (F.inv[k] == 1) {
             int32_t q = forest_find(F, F.c[k], F.r[k]);
@@ -174,8 +177,8 @@ __device__ bool forest_remove_flagged(const Team &t, Scratch &sc, char *sm, Fore
     }
     t.sync();
     const int64_t kept = team_compact(
-        t, sc, sm, F.m2, [&](int64_t k) { return F.inv[k] == 0; },
-        [&](int64_t k, int64_t p) {
+        t, sc, sm, F.m2, [=](int64_t k) { return F.inv[k] == 0; },
+        [=](int64_t k, int64_t p) {
             F.r2[p] = F.r[k];
             F.c2[p] = F.c[k];
             F.w2[p] = F.w[k];
@@ -189,17 +192,20 @@ __device__ bool forest_remove_flagged(const Team &t, Scratch &sc, char *sm, Fore
     for (int64_t k = t.rank(); k < F.m2; k += t.size()) F.inv[k] = 0;
     forest_offsets(t, F);
     if (any) F.version++;
+    state = F;
     return any;
 }
 
 // filter_by_cc (src/edge_contractions_woc.cu:257-276)
 template <class Team>
-__device__ int64_t forest_filter_by_cc(const Team &t, Scratch &sc, char *sm, Forest &F)
+__device__ __noinline__ int64_t forest_filter_by_cc(const Team &t, Scratch &sc, char *, Forest &state)
 {
-    team_cc(t, sc, F.nn, F.m2, [&](int64_t k) { return F.r[k]; }, [&](int64_t k) { return F.c[k]; }, F.lab);
+    char *sm = team_smem();
+    Forest F = state;  // pointers in registers
+    team_cc(t, sc, F.nn, F.m2, [=](int64_t k) { return F.r[k]; }, [=](int64_t k) { return F.c[k]; }, F.lab);
     const int64_t R = team_compact(
-        t, sc, sm, F.R, [&](int64_t k) { return F.lab[F.rr[k]] == F.lab[F.rc[k]]; },
-        [&](int64_t k, int64_t p) {
+        t, sc, sm, F.R, [=](int64_t k) { return F.lab[F.rr[k]] == F.lab[F.rc[k]]; },
+        [=](int64_t k, int64_t p) {
             F.rr2[p] = F.rr[k];
             F.rc2[p] = F.rc[k];
         });
@@ -207,6 +213,7 @@ __device__ int64_t forest_filter_by_cc(const Team &t, Scratch &sc, char *sm, For
     tp = F.rr; F.rr = F.rr2; F.rr2 = tp;
     tp = F.rc; F.rc = F.rc2; F.rc2 = tp;
     F.R = R;
+    state = F;
     return R;
 }
 
@@ -228,8 +235,10 @@ __device__ __forceinline__ int32_t first_common_pos(const Forest &F, int32_t a, 
 
 // check_triangles_cuda (src/edge_contractions_woc.cu:10-37)
 template <class Team>
-__device__ bool forest_check_triangles(const Team &t, Scratch &sc, char *sm, Forest &F)
+__device__ __noinline__ bool forest_check_triangles(const Team &t, Scratch &sc, char *, Forest &state)
 {
+    char *sm = team_smem();
+    Forest F = state;  // pointers in registers
     if (F.R == 0) return false;
     for (int64_t k = t.rank(); k < F.R; k += t.size()) {
         int32_t p1, p2;
@@ -237,13 +246,15 @@ __device__ bool forest_check_triangles(const Team &t, Scratch &sc, char *sm, For
         F.inv[F.w[p1] < F.w[p2] ? p1 : p2] = 1;
     }
     t.sync();
-    return forest_remove_flagged(t, sc, sm, F);
+    return forest_remove_flagged(t, sc, sm, state);
 }
 
 // check_quadrangles_cuda (src/edge_contractions_woc.cu:39-79)
 template <class Team>
-__device__ bool forest_check_quadrangles(const Team &t, Scratch &sc, char *sm, Forest &F)
+__device__ __noinline__ bool forest_check_quadrangles(const Team &t, Scratch &sc, char *, Forest &state)
 {
+    char *sm = team_smem();
+    Forest F = state;  // pointers in registers
     if (F.R == 0) return false;
     for (int64_t k = t.rank(); k < F.R; k += t.size()) {
         int32_t v1 = F.rr[k], v2 = F.rc[k];
@@ -256,7 +267,7 @@ __device__ bool forest_check_quadrangles(const Team &t, Scratch &sc, char *sm, F
         }
     }
     t.sync();
-    return forest_remove_flagged(t, sc, sm, F);
+    return forest_remove_flagged(t, sc, sm, state);
 }
 
 // check_pentagons_cuda (src/edge_contractions_woc.cu:81-139): for every
@@ -266,8 +277,10 @@ __device__ bool forest_check_quadrangles(const Team &t, Scratch &sc, char *sm, F
 // reference's comparison order).  The reference ships this step disabled;
 // here it runs when the option asks for it.
 template <class Team>
-__device__ bool forest_check_pentagons(const Team &t, Scratch &sc, char *sm, Forest &F)
+__device__ __noinline__ bool forest_check_pentagons(const Team &t, Scratch &sc, char *, Forest &state)
 {
+    char *sm = team_smem();
+    Forest F = state;  // pointers in registers
     if (F.R == 0) return false;
     for (int64_t k = t.rank(); k < F.R; k += t.size()) {
         const int32_t v1 = F.rr[k], v2 = F.rc[k];
@@ -289,18 +302,18 @@ __device__ bool forest_check_pentagons(const Team &t, Scratch &sc, char *sm, For
         }
     }
     t.sync();
-    return forest_remove_flagged(t, sc, sm, F);
+    return forest_remove_flagged(t, sc, sm, state);
 }
 
 // filter_by_thresholding (src/edge_contractions_woc_thrust.cu:522-542)
 template <class Team>
 __device__ bool forest_threshold(const Team &t, Scratch &sc, char *sm, Forest &F)
 {
-    const double S = team_csum(t, sc, F.m2, [&](int64_t k) -> float {
+    const double S = team_csum(t, sc, F.m2, [=](int64_t k) -> float {
         const float x = F.w[k];
         return x >= 0.0f ? x : 0.0f;
     });
-    const int64_t cnt = team_sum<Team, int64_t>(t, sc, sm, F.m2, [&](int64_t k) -> int64_t { return F.w[k] >= 0.0f; });
+    const int64_t cnt = team_sum<Team, int64_t>(t, sc, sm, F.m2, [=](int64_t k) -> int64_t { return F.w[k] >= 0.0f; });
     const float thr = (0.9f * (float)S) / (float)cnt;
     for (int64_t k = t.rank(); k < F.m2; k += t.size()) F.inv[k] = F.w[k] < thr ? 3 : 0;
     t.sync();
@@ -311,8 +324,10 @@ __device__ bool forest_threshold(const Team &t, Scratch &sc, char *sm, Forest &F
 // the weight of the edge to the parent.  In a forest every vertex is found
 // by exactly one frontier vertex, so the BFS needs no atomics on par[].
 template <class Team>
-__device__ bool forest_root(const Team &t, Scratch &sc, char *sm, Forest &F)
+__device__ __noinline__ bool forest_root(const Team &t, Scratch &sc, char *, Forest &state)
 {
+    char *sm = team_smem();
+    Forest F = state;  // pointers in registers
     for (int64_t v = t.rank(); v < F.nn; v += t.size()) {
         F.par[v] = -2;
         F.dep[v] = 0;
@@ -320,8 +335,8 @@ __device__ bool forest_root(const Team &t, Scratch &sc, char *sm, Forest &F)
     }
     t.sync();
     int64_t nf = team_compact(
-        t, sc, sm, F.nn, [&](int64_t v) { return F.lab[v] == (int32_t)v && F.off[v + 1] > F.off[v]; },
-        [&](int64_t v, int64_t p) {
+        t, sc, sm, F.nn, [=](int64_t v) { return F.lab[v] == (int32_t)v && F.off[v + 1] > F.off[v]; },
+        [=](int64_t v, int64_t p) {
             F.front[p] = (int32_t)v;
             F.par[v] = -1;
         });
@@ -349,6 +364,8 @@ __device__ bool forest_root(const Team &t, Scratch &sc, char *sm, Forest &F)
         t.sync();
         if (t.rank() == 0) cntp[0] = 0;
     }
+    state.front = F.front;
+    state.front2 = F.front2;
     return true;
 }
 
@@ -383,7 +400,7 @@ __device__ int32_t forest_path_lengths(const Team &t, Scratch &sc, char *sm, For
         F.plen[k] = forest_meet(F, F.rr[k], F.rc[k], la, lb) ? la + lb : 0x3fffffff;
     }
     t.sync();
-    return team_min<Team, int32_t>(t, sc, sm, F.R, 0x7fffffff, [&](int64_t k) { return F.plen[k]; });
+    return team_min<Team, int32_t>(t, sc, sm, F.R, 0x7fffffff, [=](int64_t k) { return F.plen[k]; });
 }
 
 // Cut the bottleneck of every repulsive edge whose path has dr+dc edges: the
@@ -392,8 +409,10 @@ __device__ int32_t forest_path_lengths(const Team &t, Scratch &sc, char *sm, For
 // src/edge_contractions_woc_thrust.cu:201-216: the v1 side wins only when
 // strictly smaller).
 template <class Team>
-__device__ bool forest_resolve(const Team &t, Scratch &sc, char *sm, Forest &F, int32_t dr, int32_t dc)
+__device__ __noinline__ bool forest_resolve(const Team &t, Scratch &sc, char *, Forest &state, int32_t dr, int32_t dc)
 {
+    char *sm = team_smem();
+    Forest F = state;  // pointers in registers
     const int32_t s = dr + dc;
     for (int64_t k = t.rank(); k < F.R; k += t.size()) {
         if (F.plen[k] != s) continue;
@@ -463,16 +482,18 @@ __device__ bool forest_resolve(const Team &t, Scratch &sc, char *sm, Forest &F, 
         F.inv[forest_find(F, child, F.par[child])] = 1;
     }
     t.sync();
-    return forest_remove_flagged(t, sc, sm, F);
+    return forest_remove_flagged(t, sc, sm, state);
 }
 
 // edge_contractions_woc ctor + find_contraction_mapping.  map_out gets
 // max_dim(A) entries; returns the number of directed forest entries left
 // (0 = nothing to contract).
 template <class Team>
-__device__ int32_t woc_contraction_map(const Team &t, Scratch &sc, char *sm, const Graph &A, int32_t *map_out,
+__device__ __noinline__ int32_t woc_contraction_map(const Team &t, Scratch &sc, char *, const Graph &graph, int32_t *map_out,
                                        int32_t *map_size, int *err, bool pentagons = false)
 {
+    char *sm = team_smem();
+    const Graph A = graph;  // its pointers in registers
     Forest F;
     F.nn = A.max_dim();
     F.version = 0;
@@ -486,10 +507,10 @@ __device__ int32_t woc_contraction_map(const Team &t, Scratch &sc, char *sm, con
     if (!sc.arena.ok()) return 0;
     // 1. partition at cost > 0 (:345-375)
     const int64_t P = team_compact(
-        t, sc, sm, A.n, [&](int64_t e) { return A.cost[e] > 0.0f; }, [&](int64_t e, int64_t p) { pidx[p] = e; });
+        t, sc, sm, A.n, [=](int64_t e) { return A.cost[e] > 0.0f; }, [=](int64_t e, int64_t p) { pidx[p] = e; });
     F.R = team_compact(
-        t, sc, sm, A.n, [&](int64_t e) { return !(A.cost[e] > 0.0f); },
-        [&](int64_t e, int64_t p) {
+        t, sc, sm, A.n, [=](int64_t e) { return !(A.cost[e] > 0.0f); },
+        [=](int64_t e, int64_t p) {
             F.rr[p] = A.row[e];
             F.rc[p] = A.col[e];
         });
@@ -498,11 +519,11 @@ __device__ int32_t woc_contraction_map(const Team &t, Scratch &sc, char *sm, con
         return 0;
     }
     // 2. maximum spanning forest of the attractive edges
-    const int32_t nv0 = 1 + team_max<Team, int32_t>(t, sc, sm, P, 0, [&](int64_t p) { return A.col[pidx[p]]; });
+    const int32_t nv0 = 1 + team_max<Team, int32_t>(t, sc, sm, P, 0, [=](int64_t p) { return A.col[pidx[p]]; });
     uint8_t *chosen = sc.arena.take<uint8_t>(P + 1);
     if (!sc.arena.ok()) return 0;
-    if (!team_msf(t, sc, sm, P, nv0, [&](int64_t p) { return A.row[pidx[p]]; },
-                  [&](int64_t p) { return A.col[pidx[p]]; }, [&](int64_t p) { return A.cost[pidx[p]]; }, chosen)) {
+    if (!team_msf(t, sc, sm, P, nv0, [=](int64_t p) { return A.row[pidx[p]]; },
+                  [=](int64_t p) { return A.col[pidx[p]]; }, [=](int64_t p) { return A.cost[pidx[p]]; }, chosen)) {
         *err |= ERR_ITER_LIMIT;
     }
     prof_mark(t, sc, PH_WOC_MSF);
@@ -514,7 +535,7 @@ __device__ int32_t woc_contraction_map(const Team &t, Scratch &sc, char *sm, con
     for (int64_t p = t.rank(); p < P; p += t.size())
         if (chosen[p]) ekeep[pidx[p]] = 1;
     t.sync();
-    Csr C = build_symmetric_csr(t, sc, sm, A, F.nn, [&](int64_t e) { return ekeep[e] != 0; }, false);
+    Csr C = build_symmetric_csr(t, sc, sm, A, F.nn, [=](int64_t e) { return ekeep[e] != 0; }, false);
     F.m2 = C.m2;
     F.off = C.off;
     F.c = C.adj;

@@ -13,6 +13,8 @@ struct Graph {
     int64_t n;
     int32_t rows, cols;  // dCOO::rows_ / cols_
     float cmin;          // smallest cost of an edge with row != col (NaN: not known)
+    int32_t ecols;       // largest column of an edge + 1 (rows / cols keep dims from before the diagonal went)
+    int uniq;            // no two edges share both ends (0: not known)
     __device__ __forceinline__ int32_t max_dim() const { return rows > cols ? rows : cols; }
 };
 
@@ -29,6 +31,8 @@ __device__ Graph graph_alloc(const Team &t, Scratch &sc, int64_t n)
     g.n = n;
     g.rows = g.cols = 0;
     g.cmin = unknown_cost();
+    g.ecols = 0;
+    g.uniq = 0;
     return g;
 }
 
@@ -68,7 +72,7 @@ template <class Team>
 __device__ void graph_set_dims(const Team &t, Scratch &sc, char *sm, Graph &g)
 {
     if (g.n == 0) {
-        g.rows = g.cols = 0;
+        g.rows = g.cols = g.ecols = 0;
         g.cmin = unknown_cost();
         return;
     }
@@ -77,9 +81,19 @@ __device__ void graph_set_dims(const Team &t, Scratch &sc, char *sm, Graph &g)
     team_maxi_minf(
         t, sc, sm, g.n, -1, 3.4e38f, [=](int64_t e) { return g.col[e]; },
         [=](int64_t e) { return g.row[e] != g.col[e] ? g.cost[e] : 3.4e38f; }, mc, mn);
-    g.cols = mc + 1;
+    g.cols = g.ecols = mc + 1;
     g.rows = uread(&g.row[g.n - 1]) + 1;
     g.cmin = mn;
+}
+
+// whether no two neighbours of the sorted edge list share both ends
+template <class Team>
+__device__ bool graph_is_simple(const Team &t, Scratch &sc, char *sm, const Graph &g)
+{
+    const int32_t *row = g.row, *col = g.col;
+    return team_sum<Team, int64_t>(t, sc, sm, g.n, [=](int64_t e) -> int64_t {
+               return e > 0 && row[e] == row[e - 1] && col[e] == col[e - 1];
+           }) == 0;
 }
 
 __device__ __forceinline__ uint64_t pack_key(int32_t a, int32_t b, int nbits)
@@ -107,7 +121,8 @@ __device__ __noinline__ Graph graph_from_edges(const Team &t, Scratch &sc, char 
     if (n == 0 || n >= (int64_t(1) << 31)) return graph_from_edges_sorted(t, sc, sm, i, j, c, n);
     Graph out;
     out.n = n;
-    out.rows = out.cols = 0;
+    out.rows = out.cols = out.ecols = 0;
+    out.uniq = 0;
     out.cmin = unknown_cost();
     const int32_t mx = team_max<Team, int32_t>(t, sc, sm, n, 0, [=](int64_t e) { return i[e] > j[e] ? i[e] : j[e]; });
     const int nbh = bits_for((uint64_t)(mx > 0 ? mx : 1));
@@ -117,7 +132,9 @@ __device__ __noinline__ Graph graph_from_edges(const Team &t, Scratch &sc, char 
     int32_t *sbits = sc.arena.take<int32_t>(n + 1);
     int32_t *sbk = sc.arena.take<int32_t>(n + 1);
     int32_t *bst = sc.arena.take<int32_t>((int64_t)mx + 2);
+    int32_t *dup = sc.arena.take<int32_t>(1);
     if (!sc.arena.ok()) return out;
+    if (t.rank() == 0) dup[0] = 0;
     const bool done = team_bucket_sort_ex(
         t, sc, sm, n, mx + 1,
         [=](int64_t e) -> int64_t {
@@ -145,14 +162,22 @@ __device__ __noinline__ Graph graph_from_edges(const Team &t, Scratch &sc, char 
     g.cost = reinterpret_cast<float *>(ar.base + top + 2 * words);
     g.n = n;
     team_for_batched(
-        t, n, [=](int64_t p) { return make_int3(sbk[p], (int32_t)(sk[p] >> 32), sbits[p]); },
-        [=](int64_t p, int3 v) {
+        t, n,
+        [=](int64_t p) {
+            const int64_t q = p > 0 ? p - 1 : 0;
+            const int32_t hi = (int32_t)(sk[p] >> 32);
+            const int same = p > 0 && sbk[q] == sbk[p] && (int32_t)(sk[q] >> 32) == hi;
+            return make_int4(sbk[p], hi, sbits[p], same);
+        },
+        [=](int64_t p, int4 v) {
             g.row[p] = v.x;
             g.col[p] = v.y;
             g.cost[p] = __int_as_float(v.z);
+            if (v.w) dup[0] = 1;
         });
     t.sync();
     graph_set_dims(t, sc, sm, g);
+    g.uniq = uread(dup) == 0;
     ar.top = top;
     sc.arena.release(m);
     sc.alg_bytes += 24.0 * (double)n;
@@ -166,7 +191,8 @@ __device__ __noinline__ Graph graph_from_edges_sorted(const Team &t, Scratch &sc
     char *sm = team_smem();
     Graph out;
     out.n = n;
-    out.rows = out.cols = 0;
+    out.rows = out.cols = out.ecols = 0;
+    out.uniq = 0;
     int32_t mx = team_max<Team, int32_t>(t, sc, sm, n, 0, [=](int64_t e) { return i[e] > j[e] ? i[e] : j[e]; });
     const int nb = bits_for((uint64_t)mx);
     uint64_t m = sc.arena.mark();
@@ -344,6 +370,9 @@ __device__ __noinline__ Graph graph_contract_sorted(const Team &t, Scratch &sc, 
     h.rows = g.rows;
     h.cols = g.cols;
     h.cmin = g.cmin;
+    h.ecols = 0;
+    if (nk > 0) h.ecols = 1 + team_max<Team, int32_t>(t, sc, sm, nk, -1, [=](int64_t e) { return h.col[e]; });
+    h.uniq = 1;
     Graph res = graph_commit(t, sc, h);
     sc.arena.release(m);
     sc.alg_bytes += 20.0 * (double)n + 12.0 * (double)nruns;
@@ -581,6 +610,8 @@ __device__ __noinline__ Graph graph_contract(const Team &t, Scratch &sc, char *,
     h.rows = uread(&sbk[n - 1]) + 1;
     h.cols = (mc > dmax ? mc : dmax) + 1;
     h.cmin = nk > 0 ? mn : unknown_cost();
+    h.ecols = mc + 1;
+    h.uniq = 1;
     ar.top = top;
     sc.arena.release(m);
     sc.alg_bytes += 20.0 * (double)n + 12.0 * (double)nk;

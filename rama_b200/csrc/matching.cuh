@@ -31,8 +31,9 @@ __device__ __noinline__ int32_t matching_contraction_map(const Team &t, Scratch 
 {
     char *sm = team_smem();
     const Graph A = graph;  // its pointers in registers
-    int32_t mc = team_max<Team, int32_t>(t, sc, sm, A.n, -1, [=](int64_t e) { return A.col[e]; });
-    const int32_t M = mc + 1;
+    // largest column + 1: known from the pass that built the graph
+    const int32_t M = A.ecols > 0 ? A.ecols
+                                  : 1 + team_max<Team, int32_t>(t, sc, sm, A.n, -1, [=](int64_t e) { return A.col[e]; });
     *M_out = M;
     uint64_t mark = sc.arena.mark();
     int32_t *nm = sc.arena.take<int32_t>((int64_t)M + 1);

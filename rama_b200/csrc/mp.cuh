@@ -27,7 +27,7 @@ struct Mp {
     int32_t *inc_off;  // E + 1: first slot of each edge
     int32_t *longe;    // edges with more than RSUM_THREAD_MAX incident triangles
     int64_t nlong;
-    int32_t rows, cols;
+    int inplace;  // row, col and cost are the graph's own arrays (no chords)
 };
 
 // position of (a,b) in a (row,col)-sorted list with row offsets `off`
@@ -96,127 +96,31 @@ __device__ __forceinline__ int64_t lower_edge(const int32_t *off, const int32_t 
 }
 
 // multicut_message_passing ctor (:65-176)
+//
+// Bound by the number of dependent passes for small and mid-size graphs (a
+// team sync and one or two L2 round trips each), by the gathers of the edge
+// lookups for large ones.  So everything that can share a pass does: the
+// lookup of a triangle's sides counts the chords of each row, or, where every
+// side is known to be an edge (3-cycles), the triangles of each edge; the scan
+// of those counts gives the edges' shares and the list of long edges; and one
+// key per item is moved to order chords and incidences (team_bucket_starts).
+// On the 201,720-edge cube in PD+ mode the builds took 7.5 ms as passes of their own,
+// and 4.3 this way; the lists of attractive neighbours 5.3 and 1.8.
 template <class Team>
 __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const Graph &graph, TriBuf &tb, Mp &out)
 {
     char *sm = team_smem();
     const Graph A = graph;  // pointers in registers
     Mp mp;
-    int32_t nmax = A.max_dim();
+    const int32_t nmax = A.max_dim();
     // normalize_triangles (:79)
-    const int64_t T = tri_normalize(t, sc, sm, tb.t1, tb.t2, tb.t3, tb.num, nmax);
+    const int64_t T = tri_normalize(t, sc, sm, tb, tb.num, nmax);
     prof_mark(t, sc, PH_MP_NORM);
     if (!sc.arena.ok()) return false;
     mp.T = T;
     mp.t1 = tb.t1;
     mp.t2 = tb.t2;
     mp.t3 = tb.t3;
-    // row offsets of A over [0, nmax]
-    int32_t *aoff = sc.arena.take<int32_t>((int64_t)nmax + 2);
-    uint64_t *nk1 = sc.arena.take<uint64_t>(3 * T + 1), *nk2 = sc.arena.take<uint64_t>(3 * T + 1);
-    int32_t *nv1 = sc.arena.take<int32_t>(3 * T + 1), *nv2 = sc.arena.take<int32_t>(3 * T + 1);
-    if (!sc.arena.ok()) return false;
-    team_offsets(t, A.n, nmax, [=](int64_t e) { return A.row[e]; }, aoff);
-    const int nb = bits_for((uint64_t)(nmax > 0 ? nmax : 1));
-    // chords not in A: the three sides of each triangle are looked up
-    // together, and the compaction reads the flags (nv2 is free until the
-    // chord sort)
-    uint8_t *absent = reinterpret_cast<uint8_t *>(nv2);
-    for (int64_t k = t.rank(); k < T; k += t.size()) {
-        const int32_t a[3] = {mp.t1[k], mp.t1[k], mp.t2[k]};
-        const int32_t b[3] = {mp.t2[k], mp.t3[k], mp.t3[k]};
-        int32_t f[3];
-        find_edges3(aoff, A.col, a, b, f);
-#pragma unroll
-        for (int s = 0; s < 3; ++s) absent[3 * k + s] = f[s] < 0;
-    }
-    t.sync();
-    const int64_t nn = team_compact(
-        t, sc, sm, 3 * T, [=](int64_t q) { return absent[q] != 0; },
-        [=](int64_t q, int64_t p) {
-            int64_t k = q / 3;
-            int s = (int)(q % 3);
-            int32_t a = s == 2 ? mp.t2[k] : mp.t1[k];
-            int32_t b = s == 0 ? mp.t2[k] : mp.t3[k];
-            nk1[p] = pack_key(a, b, nb);
-            nv1[p] = 0;
-        });
-    {
-        // sort the chords (a, b): bucket by a, order by b (equal chords are
-        // merged below, so their order does not matter); rows of more than
-        // BUCKET_MAX chords: LSD radix sort
-        const uint64_t cmask = (nb == 0) ? 0 : ((uint64_t(1) << nb) - 1);
-        uint64_t bm = sc.arena.mark();
-        int32_t *bst = sc.arena.take<int32_t>((int64_t)nmax + 2);
-        bool done = false;
-        if (sc.arena.ok() && nn < (int64_t(1) << 31)) {
-            // the payload of each chord is its row, so every sorted position
-            // rebuilds its key from its own entries
-            auto row = [=](int64_t q) { return (int32_t)(nk1[q] >> nb); };
-            done = team_bucket_sort_ex(
-                t, sc, sm, nn, nmax + 1, row, row, [=](int64_t q) { return nk1[q] & cmask; }, row, nk2, nv2, bst);
-            if (done) {
-                team_for_batched(
-                    t, nn, [=](int64_t p) { return ((uint64_t)(uint32_t)nv2[p] << nb) | nk2[p]; },
-                    [=](int64_t p, uint64_t key) { nk1[p] = key; });
-                t.sync();
-            }
-        }
-        sc.arena.release(bm);
-        if (!done) team_sort_pairs(t, sc, sm, nk1, nv1, nk2, nv2, nn, 2 * nb);
-    }
-    uint64_t *nu = nk2;  // unique chords
-    const int64_t nu_n = team_compact(
-        t, sc, sm, nn, [=](int64_t k) { return k == 0 || nk1[k] != nk1[k - 1]; },
-        [=](int64_t k, int64_t p) { nu[p] = nk1[k]; });
-    // merged edge list (set_union_by_key, :130-158)
-    const int64_t E = A.n + nu_n;
-    mp.E = E;
-    mp.row = sc.arena.take<int32_t>(E + 1);
-    mp.col = sc.arena.take<int32_t>(E + 1);
-    mp.cost = sc.arena.take<float>(E + 1);
-    if (!sc.arena.ok()) return false;
-    const uint64_t mask = (nb == 0) ? 0 : ((uint64_t(1) << nb) - 1);
-    // row offsets of the chords: an edge counts the chords before it among
-    // those of its own row
-    // (counted per row and scanned: chords leave long runs of empty rows)
-    int32_t *coff = sc.arena.take<int32_t>((int64_t)nmax + 2);
-    if (!sc.arena.ok()) return false;
-    for (int64_t v = t.rank(); v <= nmax; v += t.size()) coff[v] = 0;
-    t.sync();
-    for (int64_t k = t.rank(); k < nu_n; k += t.size()) atomicAdd(&coff[(int32_t)(nu[k] >> nb)], 1);
-    t.sync();
-    team_scan<Team, int64_t>(
-        t, sc, sm, (int64_t)nmax + 1, [=](int64_t v) -> int64_t { return coff[v]; },
-        [=](int64_t v, int64_t pre, int64_t) { coff[v] = (int32_t)pre; });
-    for (int64_t e = t.rank(); e < A.n; e += t.size()) {
-        const int32_t r = A.row[e];
-        uint64_t key = pack_key(r, A.col[e], nb);
-        int64_t lo = coff[r], hi = coff[r + 1];  // chords < key: all of rows < r, then within row r
-        while (lo < hi) {
-            int64_t m = (lo + hi) >> 1;
-            if (nu[m] < key)
-                lo = m + 1;
-            else
-                hi = m;
-        }
-        int64_t p = e + lo;
-        mp.row[p] = A.row[e];
-        mp.col[p] = A.col[e];
-        mp.cost[p] = A.cost[e];
-    }
-    for (int64_t k = t.rank(); k < nu_n; k += t.size()) {
-        int32_t a = (int32_t)(nu[k] >> nb), b = (int32_t)(nu[k] & mask);
-        int64_t p = k + lower_edge(aoff, A.col, a, b);
-        mp.row[p] = a;
-        mp.col[p] = b;
-        mp.cost[p] = 0.0f;
-    }
-    t.sync();
-    prof_mark(t, sc, PH_MP_CHORDS);
-    // merged row offsets, correspondences (compute_triangle_edge_correspondence, :15-62)
-    int32_t *moff = aoff;  // reuse
-    team_offsets(t, E, nmax, [=](int64_t e) { return mp.row[e]; }, moff);
     mp.e12 = sc.arena.take<int32_t>(T + 1);
     mp.e13 = sc.arena.take<int32_t>(T + 1);
     mp.e23 = sc.arena.take<int32_t>(T + 1);
@@ -225,60 +129,269 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
     mp.c23 = sc.arena.take<float>(T + 1);
     mp.slot = sc.arena.take<float>(3 * T + 1);
     mp.pos = sc.arena.take<int32_t>(3 * T + 1);
-    mp.inc_off = sc.arena.take<int32_t>(E + 2);
-    uint64_t ik = sc.arena.mark();
-    uint64_t *q1 = sc.arena.take<uint64_t>(3 * T + 1), *q2 = sc.arena.take<uint64_t>(3 * T + 1);
-    int32_t *w1 = sc.arena.take<int32_t>(3 * T + 1), *w2 = sc.arena.take<int32_t>(3 * T + 1);
+    int32_t *aoff = sc.arena.take<int32_t>((int64_t)nmax + 2);  // row offsets of A over [0, nmax]
+    int32_t *slot = sc.arena.take<int32_t>(3 * T + 1);          // a side's slot among the chords of its row,
+                                                                // then among the triangles of its edge
+    int32_t *key = sc.arena.take<int32_t>(3 * T + 1);           // the keys moved to their buckets
     if (!sc.arena.ok()) return false;
-    for (int64_t k = t.rank(); k < T; k += t.size()) {
-        const int32_t a = mp.t1[k], b = mp.t2[k], c = mp.t3[k];
-        const int32_t from[3] = {a, a, b}, to[3] = {b, c, c};
-        int32_t f[3];
-        find_edges3(moff, mp.col, from, to, f);
-        const int32_t x = f[0], y = f[1], z = f[2];
-        mp.e12[k] = x;
-        mp.e13[k] = y;
-        mp.e23[k] = z;
-        q1[3 * k] = (uint64_t)x;
-        q1[3 * k + 1] = (uint64_t)y;
-        q1[3 * k + 2] = (uint64_t)z;
-        w1[3 * k] = (int32_t)(3 * k);
-        w1[3 * k + 1] = (int32_t)(3 * k + 1);
-        w1[3 * k + 2] = (int32_t)(3 * k + 2);
+    const bool closed = tb.closed != 0;
+    const int32_t nbk = nmax + 1;
+    // the counts of the first grouping: triangles per edge, or chords per row
+    const uint64_t cm = sc.arena.mark();
+    BucketLists L = bucket_lists(sc, 3 * T);
+    int32_t *cst = nullptr;
+    if (closed) {
+        mp.inc_off = sc.arena.take<int32_t>(A.n + 2);
+        if (!sc.arena.ok()) return false;
+        for (int64_t e = t.rank(); e <= A.n; e += t.size()) mp.inc_off[e] = 0;
+    } else {
+        cst = sc.arena.take<int32_t>((int64_t)nbk + 1);
+        if (!sc.arena.ok()) return false;
+        for (int64_t v = t.rank(); v <= nbk; v += t.size()) cst[v] = 0;
     }
-    t.sync();
-    // incidence order: (edge, 3t + corner) sorted by edge, then by 3t + corner;
-    // the rank of each (triangle, corner) in that order is its slot
-    if (3 * T < (int64_t(1) << 31) &&
-        team_bucket_sort(
-            t, sc, sm, 3 * T, (int32_t)E, [=](int64_t q) { return (int32_t)q1[q]; },
-            [=](int64_t q) { return (uint64_t)q; }, q2, w2, mp.inc_off)) {
-        for (int64_t q = t.rank(); q < 3 * T; q += t.size()) mp.pos[w2[q]] = (int32_t)q;
+    if (t.rank() < 4) L.n[t.rank()] = 0;
+    team_offsets(t, A.n, nmax, [=](int64_t e) { return A.row[e]; }, aoff);
+    // the triangles' sides in a (row, col)-sorted list; `each` gets the three
+    // positions (-1: not an edge) with all lanes of the warp present
+    auto lookup = [=](const int32_t *off, const int32_t *col, auto each) {
+        for (int64_t k0 = (int64_t)t.rank() - lane_id(); k0 < T; k0 += t.size()) {
+            const int64_t k = k0 + lane_id();
+            int32_t f[3] = {-1, -1, -1}, from[3] = {0, 0, 0};
+            if (k < T) {
+                const int32_t a = mp.t1[k], b = mp.t2[k], c = mp.t3[k];
+                const int32_t to[3] = {b, c, c};
+                from[0] = from[1] = a;
+                from[2] = b;
+                find_edges3(off, col, from, to, f);
+                mp.e12[k] = f[0];
+                mp.e13[k] = f[1];
+                mp.e23[k] = f[2];
+            }
+            each(k, k < T, from, f);
+        }
+    };
+    // counts a triangle's sides into their edges (neighbouring triangles share
+    // their first side often, the others seldom)
+    auto count_sides = [=](int64_t k, bool valid, const int32_t (&f)[3], int32_t *inc) {
+        const int32_t s0 = bucket_slot(inc, valid ? f[0] : -1);
+        if (valid) {
+            const int32_t s1 = atomicAdd(&inc[f[1]], 1), s2 = atomicAdd(&inc[f[2]], 1);
+            slot[3 * k] = s0;
+            slot[3 * k + 1] = s1;
+            slot[3 * k + 2] = s2;
+        }
+    };
+    int64_t nn = 0;
+    if (closed) {
+        int32_t *inc = mp.inc_off;
+        lookup(aoff, A.col, [=](int64_t k, bool valid, const int32_t (&)[3], const int32_t (&f)[3]) {
+            count_sides(k, valid, f, inc);
+        });
         t.sync();
     } else {
-        int32_t *incp = w1;
-        uint64_t *qk = q1;
-        team_sort_pairs(t, sc, sm, qk, incp, q2, w2, 3 * T, bits_for((uint64_t)(E > 0 ? E : 1)));
-        for (int64_t q = t.rank(); q < 3 * T; q += t.size()) mp.pos[incp[q]] = (int32_t)q;
-        team_offsets(t, 3 * T, (int32_t)E, [=](int64_t k) { return (int32_t)qk[k]; }, mp.inc_off);
+        // chords: sides that are no edges, by their row
+        lookup(aoff, A.col, [=](int64_t k, bool valid, const int32_t (&from)[3], const int32_t (&f)[3]) {
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const bool chord = valid && f[s] < 0;
+                const int32_t x = bucket_slot(cst, chord ? from[s] : -1);
+                if (valid) slot[3 * k + s] = chord ? x : -1;
+            }
+        });
+        t.sync();
+        nn = team_bucket_starts(t, sc, sm, nbk, cst, L, [](int64_t, int32_t, int32_t) {});
     }
-    sc.arena.release(ik);
-    prof_mark(t, sc, PH_MP_INCID);
-    // each covered edge's share of its cost, and the edges whose incoming
-    // messages a whole warp sums
-    mp.share = sc.arena.take<float>(E + 1);
-    mp.longe = sc.arena.take<int32_t>(E + 1);
+    mp.inplace = nn == 0;
+    if (mp.inplace) {
+        mp.E = A.n;
+        mp.row = A.row;
+        mp.col = A.col;
+        mp.cost = A.cost;
+        prof_mark(t, sc, PH_MP_CHORDS);
+        if (!closed) {
+            sc.arena.release(cm);
+            L = bucket_lists(sc, 3 * T);
+            mp.inc_off = sc.arena.take<int32_t>(A.n + 2);
+            if (!sc.arena.ok()) return false;
+            for (int64_t e = t.rank(); e <= A.n; e += t.size()) mp.inc_off[e] = 0;
+            if (t.rank() < 4) L.n[t.rank()] = 0;
+            t.sync();
+            int32_t *inc = mp.inc_off;
+            for (int64_t k0 = (int64_t)t.rank() - lane_id(); k0 < T; k0 += t.size()) {
+                const int64_t k = k0 + lane_id();
+                int32_t f[3] = {-1, -1, -1};
+                if (k < T) {
+                    f[0] = mp.e12[k];
+                    f[1] = mp.e13[k];
+                    f[2] = mp.e23[k];
+                }
+                count_sides(k, k < T, f, inc);
+            }
+            t.sync();
+        }
+    } else {
+        // the chords' columns, ascending within each row (equal ones adjacent),
+        // and their rows
+        int32_t *ccol = sc.arena.take<int32_t>(nn + 1), *crow = sc.arena.take<int32_t>(nn + 1);
+        int32_t *upre = sc.arena.take<int32_t>(nn + 1);  // distinct chords before each position
+        int32_t *ucol = sc.arena.take<int32_t>(nn + 1), *urow = sc.arena.take<int32_t>(nn + 1);
+        if (!sc.arena.ok()) return false;
+        auto side_from = [=](int64_t q) { return q % 3 == 2 ? mp.t2[q / 3] : mp.t1[q / 3]; };
+        auto side_to = [=](int64_t q) { return q % 3 == 0 ? mp.t2[q / 3] : mp.t3[q / 3]; };
+        if (!L.has_big()) {
+            for (int64_t q = t.rank(); q < 3 * T; q += t.size())
+                if (slot[q] >= 0) key[cst[side_from(q)] + slot[q]] = side_to(q);
+            t.sync();
+            for (int64_t q = t.rank(); q < 3 * T; q += t.size()) {
+                if (slot[q] < 0) continue;
+                const int32_t a = side_from(q), s = cst[a], e = cst[a + 1];
+                if (e - s > BUCKET_SMALL) continue;
+                const int32_t b = side_to(q);
+                const int32_t p = s + bucket_rank(key, s, e, b, s + slot[q]);
+                ccol[p] = b;
+                crow[p] = a;
+            }
+            if (L.has_long())
+                team_sort_long_buckets(t, sm, L, cst, reinterpret_cast<const uint32_t *>(key),
+                                       [=](int32_t b, int32_t p, uint32_t c) {
+                                           ccol[p] = (int32_t)c;
+                                           crow[p] = b;
+                                       });
+            t.sync();
+        } else {
+            // a row with more than BUCKET_MAX chords: LSD radix sort of (row, col)
+            const int nb = bits_for((uint64_t)(nmax > 0 ? nmax : 1));
+            const uint64_t rm = sc.arena.mark();
+            uint64_t *k1 = sc.arena.take<uint64_t>(nn + 1), *k2 = sc.arena.take<uint64_t>(nn + 1);
+            int32_t *v1 = sc.arena.take<int32_t>(nn + 1), *v2 = sc.arena.take<int32_t>(nn + 1);
+            if (!sc.arena.ok()) return false;
+            team_compact(
+                t, sc, sm, 3 * T, [=](int64_t q) { return slot[q] >= 0; },
+                [=](int64_t q, int64_t p) {
+                    k1[p] = pack_key(side_from(q), side_to(q), nb);
+                    v1[p] = 0;
+                });
+            team_sort_pairs(t, sc, sm, k1, v1, k2, v2, nn, 2 * nb);
+            for (int64_t p = t.rank(); p < nn; p += t.size()) {
+                ccol[p] = (int32_t)(k1[p] & ((uint64_t(1) << nb) - 1));
+                crow[p] = (int32_t)(k1[p] >> nb);
+            }
+            t.sync();
+            sc.arena.release(rm);
+        }
+        const int64_t nu = team_scan<Team, int64_t>(
+            t, sc, sm, nn,
+            [=](int64_t p) -> int64_t { return p == 0 || crow[p] != crow[p - 1] || ccol[p] != ccol[p - 1]; },
+            [=](int64_t p, int64_t pre, int64_t v) {
+                upre[p] = (int32_t)pre;
+                if (p == nn - 1) upre[nn] = (int32_t)(pre + v);
+                if (v) {
+                    ucol[pre] = ccol[p];
+                    urow[pre] = crow[p];
+                }
+            });
+        // merged edge list (set_union_by_key, :130-158) and its row offsets;
+        // an edge counts the chords before it among those of its own row
+        const int64_t E = A.n + nu;
+        mp.E = E;
+        mp.row = sc.arena.take<int32_t>(E + 1);
+        mp.col = sc.arena.take<int32_t>(E + 1);
+        mp.cost = sc.arena.take<float>(E + 1);
+        int32_t *moff = sc.arena.take<int32_t>((int64_t)nmax + 2);
+        mp.inc_off = sc.arena.take<int32_t>(E + 2);
+        if (!sc.arena.ok()) return false;
+        team_for_batched(
+            t, A.n,
+            [=](int64_t e) {
+                const int32_t r = A.row[e], c = A.col[e];
+                int32_t lo = upre[cst[r]], hi = upre[cst[r + 1]];
+                while (lo < hi) {
+                    const int32_t m = (lo + hi) >> 1;
+                    if (ucol[m] < c)
+                        lo = m + 1;
+                    else
+                        hi = m;
+                }
+                return make_int4(lo, r, c, __float_as_int(A.cost[e]));
+            },
+            [=](int64_t e, int4 v) {
+                const int64_t p = e + v.x;
+                mp.row[p] = v.y;
+                mp.col[p] = v.z;
+                mp.cost[p] = __int_as_float(v.w);
+            });
+        for (int64_t k = t.rank(); k < nu; k += t.size()) {
+            const int32_t a = urow[k], b = ucol[k];
+            const int64_t p = k + lower_edge(aoff, A.col, a, b);
+            mp.row[p] = a;
+            mp.col[p] = b;
+            mp.cost[p] = 0.0f;
+        }
+        for (int64_t v = t.rank(); v <= nmax; v += t.size()) moff[v] = aoff[v] + upre[cst[v]];
+        for (int64_t e = t.rank(); e <= E; e += t.size()) mp.inc_off[e] = 0;
+        if (t.rank() < 4) L.n[t.rank()] = 0;
+        t.sync();
+        prof_mark(t, sc, PH_MP_CHORDS);
+        // correspondences (compute_triangle_edge_correspondence, :15-62)
+        int32_t *inc = mp.inc_off;
+        lookup(moff, mp.col, [=](int64_t k, bool valid, const int32_t (&)[3], const int32_t (&f)[3]) {
+            count_sides(k, valid, f, inc);
+        });
+        t.sync();
+    }
+    // first slot of each edge, its share of its cost, and the edges whose
+    // incoming messages a whole warp sums
+    mp.share = sc.arena.take<float>(mp.E + 1);
+    mp.longe = sc.arena.take<int32_t>(3 * T / (RSUM_THREAD_MAX + 1) + 1);
     if (!sc.arena.ok()) return false;
-    mp.nlong = team_compact(
-        t, sc, sm, E, [=](int64_t e) { return mp.inc_off[e + 1] - mp.inc_off[e] > RSUM_THREAD_MAX; },
-        [=](int64_t e, int64_t p) { mp.longe[p] = (int32_t)e; });
-    for (int64_t e = t.rank(); e < E; e += t.size()) {
-        const int32_t n = mp.inc_off[e + 1] - mp.inc_off[e];
+    team_bucket_starts(t, sc, sm, (int32_t)mp.E, mp.inc_off, L, [=](int64_t e, int32_t, int32_t n) {
         mp.share[e] = n > 0 ? __fdiv_rn(mp.cost[e], (float)n) : 0.0f;
+        if (n > RSUM_THREAD_MAX) mp.longe[atomicAdd(&L.n[3], 1)] = (int32_t)e;
+    });
+    mp.nlong = uread(&L.n[3]);
+    // incidence order: 3t + corner ascending within each edge; the rank of
+    // each (triangle, corner) in that order is its slot
+    if (!L.has_big()) {
+        auto edge_of = [=](int64_t k, int c) { return c == 0 ? mp.e12[k] : (c == 1 ? mp.e13[k] : mp.e23[k]); };
+        for (int64_t k = t.rank(); k < T; k += t.size())
+#pragma unroll
+            for (int c = 0; c < 3; ++c) key[mp.inc_off[edge_of(k, c)] + slot[3 * k + c]] = (int32_t)(3 * k + c);
+        t.sync();
+        for (int64_t k = t.rank(); k < T; k += t.size()) {
+            int32_t s[3], e[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const int32_t x = edge_of(k, c);
+                s[c] = mp.inc_off[x];
+                e[c] = mp.inc_off[x + 1];
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                if (e[c] - s[c] <= BUCKET_SMALL)
+                    mp.pos[3 * k + c] = s[c] + bucket_rank(key, s[c], e[c], (int32_t)(3 * k + c), s[c] + slot[3 * k + c]);
+        }
+        if (L.has_long())
+            team_sort_long_buckets(t, sm, L, mp.inc_off, reinterpret_cast<const uint32_t *>(key),
+                                   [=](int32_t, int32_t p, uint32_t q) { mp.pos[q] = p; });
+        t.sync();
+    } else {
+        const uint64_t rm = sc.arena.mark();
+        uint64_t *k1 = sc.arena.take<uint64_t>(3 * T + 1), *k2 = sc.arena.take<uint64_t>(3 * T + 1);
+        int32_t *v1 = sc.arena.take<int32_t>(3 * T + 1), *v2 = key;
+        if (!sc.arena.ok()) return false;
+        for (int64_t k = t.rank(); k < T; k += t.size()) {
+            k1[3 * k] = (uint64_t)mp.e12[k];
+            k1[3 * k + 1] = (uint64_t)mp.e13[k];
+            k1[3 * k + 2] = (uint64_t)mp.e23[k];
+            for (int c = 0; c < 3; ++c) v1[3 * k + c] = (int32_t)(3 * k + c);
+        }
+        t.sync();
+        team_sort_pairs(t, sc, sm, k1, v1, k2, v2, 3 * T, bits_for((uint64_t)(mp.E > 0 ? mp.E : 1)));
+        for (int64_t q = t.rank(); q < 3 * T; q += t.size()) mp.pos[v1[q]] = (int32_t)q;
+        t.sync();
+        sc.arena.release(rm);
     }
-    t.sync();
-    mp.rows = A.rows;
-    mp.cols = A.cols;
+    prof_mark(t, sc, PH_MP_INCID);
     out = mp;
     return true;
 }
@@ -328,7 +441,7 @@ __device__ __forceinline__ float add_third(float a, double tm) { return (float)_
 // and four dependent loads per pass for small ones.
 // min_gain: the loop ends after an iteration that gains less (the reference's
 // 1e-3).  Returns the bound of the final state; *lb0, if given, receives the
-// bound before the first iteration.
+// bound before the first iteration, *cmin the smallest edge cost.
 __device__ __forceinline__ void mp_moves(const Mp &mp, int64_t k, float t12, float t13, float t23, csum_t &bt)
 {
     const double third = 1.0 / 3.0;
@@ -374,11 +487,15 @@ __device__ __forceinline__ void mp_moves(const Mp &mp, int64_t k, float t12, flo
 
 template <class Team>
 __device__ __noinline__ double mp_run(const Team &t, Scratch &sc, const Mp &state, int num_iter, double min_gain,
-                                      double *lb0 = nullptr)
+                                      float *cmin, double *lb0 = nullptr)
 {
     const Mp mp = state;  // pointers in registers
     csum_t be, bt;        // this thread's parts of the bound
-    auto edge_bound = [&](float c) { be = cs_add(be, c < 0.0f ? c : 0.0f); };
+    float mn = 3.4e38f;   // ... and its smallest edge cost
+    auto edge_bound = [&](float c) {
+        be = cs_add(be, c < 0.0f ? c : 0.0f);
+        mn = fminf(mn, c);
+    };
     // the bound before the first iteration: the triangles' costs are 0
     double lb = team_csum(t, sc, mp.E, [=](int64_t e) -> float {
         const float c = mp.cost[e];
@@ -392,6 +509,7 @@ __device__ __noinline__ double mp_run(const Team &t, Scratch &sc, const Mp &stat
         if (it > 0 && (lb - prev) < min_gain) break;
         prev = lb;
         be = bt = csum_t{0.0, 0.0};
+        mn = 3.4e38f;
         // two triangles a thread at a time: their loads and the gathers of
         // the edges' shares are in flight together
         int64_t k = t.rank();
@@ -441,7 +559,7 @@ __device__ __noinline__ double mp_run(const Team &t, Scratch &sc, const Mp &stat
                         mp.cost[e0 + q * S] = c[q];
                         mp.share[e0 + q * S] = __fdiv_rn(c[q], (float)n[q]);
                     }
-                    edge_bound(c[q]);  // long runs add nothing here
+                    if (n[q] <= RSUM_THREAD_MAX) edge_bound(c[q]);
                 }
             }
             for (; e0 < mp.E; e0 += S) {
@@ -468,15 +586,17 @@ __device__ __noinline__ double mp_run(const Team &t, Scratch &sc, const Mp &stat
                 edge_bound(c);
             }
         }
-        const csum2_t b = team_csum_fold(t, sc, be, bt);
+        const csum2_t b = team_csum_fold(t, sc, be, bt, mn);
         lb = b.a + b.b;
+        *cmin = b.m;
         sc.alg_bytes += 84.0 * (double)mp.T + 12.0 * (double)mp.E;
     }
     return lb;
 }
 
 // dual_update_cycle_length (src/dual_solver.cu:7-35).  On success the graph
-// in the top slot is replaced by the reparametrised one.
+// in the top slot is replaced by the reparametrised one (without chords, its
+// costs are updated where they lie).
 template <class Team>
 __device__ double dual_update_cycle_length(const Team &t, Scratch &sc, char *sm, Graph &A, int c, int num_iter,
                                            float tri_factor, float tol, int64_t *num_tri, bool *failed,
@@ -485,7 +605,7 @@ __device__ double dual_update_cycle_length(const Team &t, Scratch &sc, char *sm,
     uint64_t m = sc.arena.mark();
     TriBuf tb;
     prof_mark(t, sc, PH_OTHER);
-    conflicted_cycles(t, sc, sm, A, c, tri_factor, tol, tb);
+    conflicted_cycles(t, sc, sm, A, c, tri_factor, tol, false, tb);
     prof_mark(t, sc, PH_CYC_SEARCH);
     *failed = !sc.arena.ok();
     if (*failed) {
@@ -505,18 +625,26 @@ __device__ double dual_update_cycle_length(const Team &t, Scratch &sc, char *sm,
         return 0.0;
     }
     prof_mark(t, sc, PH_MP_BUILD);
-    const double fin = mp_run(t, sc, mp, num_iter, 1e-3);
+    float cmin = unknown_cost();
+    const double fin = mp_run(t, sc, mp, num_iter, 1e-3, &cmin);
     prof_mark(t, sc, PH_MP_ITER);
-    Graph g;
-    g.row = mp.row;
-    g.col = mp.col;
-    g.cost = mp.cost;
-    g.n = mp.E;
-    graph_set_dims(t, sc, sm, g);
-    Graph ng = graph_commit(t, sc, g);
+    // dims of the edge list: a chord joins two ends of edges, so the largest
+    // column stays what it was
+    Graph g = A;
+    g.rows = uread(&mp.row[mp.E - 1]) + 1;
+    g.cols = A.ecols;
+    g.cmin = cmin;
+    *failed = false;
+    if (!mp.inplace) {
+        g.row = mp.row;
+        g.col = mp.col;
+        g.cost = mp.cost;
+        g.n = mp.E;
+        g = graph_commit(t, sc, g);
+        *failed = !sc.arena.ok();
+    }
     prof_mark(t, sc, PH_DUAL_COMMIT);
-    *failed = !sc.arena.ok();
-    if (!*failed) A = ng;
+    if (!*failed) A = g;
     sc.arena.release(m);
     return fin;
 }

@@ -23,7 +23,7 @@ constexpr unsigned FULL = 0xffffffffu;
 // ---------------------------------------------------------------------------
 struct Scratch {
     Arena arena;
-    char *part[2];  // each >= 32 * (nblocks + 2) bytes
+    char *part[2];  // each >= 48 * (nblocks + 2) bytes
     int32_t *err;   // set when a bounded wait gave up (zeroed at the start of a solve)
     int parity;
     double alg_bytes;  // algorithmic bytes of the work done (team-uniform tally)
@@ -40,7 +40,7 @@ struct Scratch {
 
 // A workspace of `bytes` bytes at `base` (256-byte aligned) holds the two
 // partial buffers, the error word and then the arena.
-constexpr uint64_t SCRATCH_PART_BYTES = 16 * 4096;  // >= 32 * (max CTAs + 2)
+constexpr uint64_t SCRATCH_PART_BYTES = 16 * 4096;  // >= 48 * (max CTAs + 2)
 
 __device__ __forceinline__ Scratch scratch_over(char *base, uint64_t bytes)
 {
@@ -425,8 +425,10 @@ struct ScanItems {
     static constexpr int value = sizeof(T) == 8 ? 4 : 8;
 };
 
-template <class Team, class T, class In, class Out>
-__device__ T team_scan(const Team &t, Scratch &sc, char *sm, int64_t n, In in, Out out)
+// team_scan_while ends after the total (one team sync) when go_on(total) is
+// false.
+template <class Team, class T, class In, class Go, class Out>
+__device__ T team_scan_while(const Team &t, Scratch &sc, char *sm, int64_t n, In in, Go go_on, Out out)
 {
     constexpr int ITEMS = ScanItems<T>::value;
     T *tsm = reinterpret_cast<T *>(sm);
@@ -459,6 +461,7 @@ __device__ T team_scan(const Team &t, Scratch &sc, char *sm, int64_t n, In in, O
     }
     base = warp_sum(base);
     total = warp_sum(total);
+    if (!go_on(total)) return total;
     const int64_t TILE = (int64_t)blockDim.x * ITEMS;
     const int64_t wseg = (int64_t)warp_in_block() * 32 * ITEMS;
     for (int64_t tile = lo; tile < hi; tile += TILE) {
@@ -485,12 +488,18 @@ __device__ T team_scan(const Team &t, Scratch &sc, char *sm, int64_t n, In in, O
     return total;
 }
 
+template <class Team, class T, class In, class Out>
+__device__ T team_scan(const Team &t, Scratch &sc, char *sm, int64_t n, In in, Out out)
+{
+    return team_scan_while<Team, T>(t, sc, sm, n, in, [](T) { return true; }, out);
+}
+
 // stable compaction: emit(i, pos) for every kept i; returns the count
 template <class Team, class Keep, class Emit>
 __device__ int64_t team_compact(const Team &t, Scratch &sc, char *sm, int64_t n, Keep keep, Emit emit)
 {
-    return team_scan<Team, int64_t>(
-        t, sc, sm, n, [=](int64_t i) -> int64_t { return keep(i) ? 1 : 0; },
+    return team_scan_while<Team, int64_t>(
+        t, sc, sm, n, [=](int64_t i) -> int64_t { return keep(i) ? 1 : 0; }, [](int64_t total) { return total != 0; },
         [=](int64_t i, int64_t pos, int64_t v) {
             if (v) emit(i, pos);
         });
@@ -536,12 +545,14 @@ __device__ __forceinline__ csum_t cs_add(csum_t a, float x) { return cs_merge(a,
 // sync, which also makes the caller's earlier stores visible to the team.
 struct csum2_t {
     double a, b;
+    float m;  // the minimum of the threads' third values
 };
 
 template <class Team>
-__device__ __noinline__ csum2_t team_csum_fold(const Team &t, Scratch &sc, csum_t a, csum_t b)
+__device__ __noinline__ csum2_t team_csum_fold(const Team &t, Scratch &sc, csum_t a, csum_t b, float m = 3.4e38f)
 {
     __shared__ csum_t wa[32], wb[32];
+    __shared__ float wm[32];
     __shared__ csum2_t res;
     // merging is commutative, so a butterfly leaves the same pair on every lane
     auto fold = [&](int lanes) {
@@ -553,6 +564,7 @@ __device__ __noinline__ csum2_t team_csum_fold(const Team &t, Scratch &sc, csum_
             y.c = __shfl_xor_sync(FULL, b.c, off);
             a = cs_merge(a, x);
             b = cs_merge(b, y);
+            m = fminf(m, __shfl_xor_sync(FULL, m, off));
         }
     };
     const int nw = blockDim.x >> 5;
@@ -560,20 +572,24 @@ __device__ __noinline__ csum2_t team_csum_fold(const Team &t, Scratch &sc, csum_
     if (lane_id() == 0) {
         wa[warp_in_block()] = a;
         wb[warp_in_block()] = b;
+        wm[warp_in_block()] = m;
     }
     __syncthreads();
-    csum_t *part = reinterpret_cast<csum_t *>(sc.next_part());  // 32 B per CTA
+    csum_t *part = reinterpret_cast<csum_t *>(sc.next_part());  // 48 B per CTA
     if (warp_in_block() == 0) {
         a = lane_id() < nw ? wa[lane_id()] : csum_t{0.0, 0.0};
         b = lane_id() < nw ? wb[lane_id()] : csum_t{0.0, 0.0};
+        m = wm[lane_id() < nw ? lane_id() : 0];
         fold(nw);
         if (lane_id() == 0) {
             if (t.nblocks() == 1) {
                 res.a = __dadd_rn(a.s, a.c);
                 res.b = __dadd_rn(b.s, b.c);
+                res.m = m;
             } else {
-                part[2 * t.block()] = a;
-                part[2 * t.block() + 1] = b;
+                part[3 * t.block()] = a;
+                part[3 * t.block() + 1] = b;
+                part[3 * t.block() + 2].s = (double)m;
             }
         }
     }
@@ -583,14 +599,17 @@ __device__ __noinline__ csum2_t team_csum_fold(const Team &t, Scratch &sc, csum_
             a = b = csum_t{0.0, 0.0};
             const double2 *p = reinterpret_cast<const double2 *>(part);
             for (int k = lane_id(); k < t.nblocks(); k += 32) {
-                const double2 x = __ldcg(p + 2 * k), y = __ldcg(p + 2 * k + 1);
+                const double2 x = __ldcg(p + 3 * k), y = __ldcg(p + 3 * k + 1);
+                const double z = __ldcg(reinterpret_cast<const double *>(p + 3 * k + 2));
                 a = cs_merge(a, csum_t{x.x, x.y});
                 b = cs_merge(b, csum_t{y.x, y.y});
+                m = fminf(m, (float)z);
             }
             fold(32);
             if (lane_id() == 0) {
                 res.a = __dadd_rn(a.s, a.c);
                 res.b = __dadd_rn(b.s, b.c);
+                res.m = m;
             }
         }
         __syncthreads();
@@ -1389,6 +1408,144 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
     }
     sc.arena.release(am);
     return true;
+}
+
+// ---------------------------------------------------------------------------
+// Grouping by a bucket, for passes that know their items: the caller counts
+// each item into its bucket with an atomic whose result is the item's slot
+// (in the pass that computes the bucket anyway), team_bucket_starts turns the
+// counts into starts, the caller scatters one key per item to start + slot,
+// and every item then finds its place as the number of smaller keys in its
+// bucket (bucket_rank).  Buckets of more than BUCKET_SMALL keys are listed by
+// team_bucket_starts and sorted by team_sort_long_buckets (a warp each up to
+// 256 keys, a CTA up to BUCKET_MAX); what lies beyond is the caller's general
+// path.  Against team_bucket_sort_ex this moves one key per item instead of
+// an index, a bucket and a key in and out, and takes five team syncs
+// instead of eight.
+// ---------------------------------------------------------------------------
+constexpr int BUCKET_SMALL = 64;
+
+struct BucketLists {
+    int32_t *warp, *cta;  // buckets of 65..256 and of 257..BUCKET_MAX keys
+    int32_t *n;           // [0], [1]: their numbers, [2]: some bucket is larger (the caller zeroes all)
+    __device__ __forceinline__ bool has_long() const { return uread(&n[0]) + uread(&n[1]) > 0; }
+    __device__ __forceinline__ bool has_big() const { return uread(&n[2]) != 0; }
+};
+
+__device__ __forceinline__ BucketLists bucket_lists(Scratch &sc, int64_t nitems)
+{
+    BucketLists L;
+    L.warp = sc.arena.take<int32_t>(nitems / (BUCKET_SMALL + 1) + 1);
+    L.cta = sc.arena.take<int32_t>(nitems / 257 + 1);
+    L.n = sc.arena.take<int32_t>(4);
+    return L;
+}
+
+// counts[0, nb) -> starts, counts[nb] = the total (also returned); each(b,
+// start, count) is called once per bucket.  Two team syncs.
+template <class Team, class Each>
+__device__ __forceinline__ int64_t team_bucket_starts(const Team &t, Scratch &sc, char *sm, int32_t nb,
+                                                      int32_t *counts, BucketLists L, Each each)
+{
+    return team_scan<Team, int64_t>(
+        t, sc, sm, nb, [=](int64_t b) -> int64_t { return counts[b]; },
+        [=](int64_t b, int64_t pre, int64_t c) {
+            counts[b] = (int32_t)pre;
+            if (b == nb - 1) counts[nb] = (int32_t)(pre + c);
+            if (c > BUCKET_MAX)
+                L.n[2] = 1;
+            else if (c > 256)
+                L.cta[atomicAdd(&L.n[1], 1)] = (int32_t)b;
+            else if (c > BUCKET_SMALL)
+                L.warp[atomicAdd(&L.n[0], 1)] = (int32_t)b;
+            each(b, (int32_t)pre, (int32_t)c);
+        });
+}
+
+// keys in [s, e) ordered before the one at p (equal keys by position)
+template <class K>
+__device__ __forceinline__ int32_t bucket_rank(const K *keys, int32_t s, int32_t e, K key, int32_t p)
+{
+    int32_t r = 0, x = s;
+    for (; x + 3 < e; x += 4) {
+        const K a = keys[x], b = keys[x + 1], c = keys[x + 2], d = keys[x + 3];
+        r += (a < key || (a == key && x < p)) + (b < key || (b == key && x + 1 < p)) +
+             (c < key || (c == key && x + 2 < p)) + (d < key || (d == key && x + 3 < p));
+    }
+    for (; x < e; ++x) {
+        const K a = keys[x];
+        r += a < key || (a == key && x < p);
+    }
+    return r;
+}
+
+// the slot of this lane's item in bucket b (-1: no item): the lanes of a warp
+// that share a bucket take theirs with one atomic; every lane must call
+__device__ __forceinline__ int32_t bucket_slot(int32_t *counts, int32_t b)
+{
+    const unsigned peers = __match_any_sync(FULL, b);
+    const int leader = __ffs(peers) - 1;
+    int32_t s = 0;
+    if (b >= 0 && lane_id() == leader) s = atomicAdd(&counts[b], __popc(peers));
+    return __shfl_sync(FULL, s, leader) + __popc(peers & lanemask_lt());
+}
+
+template <class K, class Bar>
+__device__ __forceinline__ void smem_bitonic_keys(K *key, int m, int P, int lane, int nth, Bar bar)
+{
+    for (int i = m + lane; i < P; i += nth) key[i] = ~K(0);
+    bar();
+    for (int k = 2; k <= P; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            for (int i = lane; i < P; i += nth) {
+                const int x = i ^ j;
+                if (x > i) {
+                    const K a = key[i], b = key[x];
+                    if ((a > b) == ((i & k) == 0)) {
+                        key[i] = b;
+                        key[x] = a;
+                    }
+                }
+            }
+            bar();
+        }
+}
+
+// Sorts the listed buckets of keys[] (not written) and calls emit(b, p, key)
+// for every sorted position p.  Keys are below ~K(0).  The caller syncs.
+template <class Team, class K, class Emit>
+__device__ __forceinline__ void team_sort_long_buckets(const Team &t, char *sm, BucketLists L, const int32_t *start,
+                                                       const K *keys, Emit emit)
+{
+    {
+        K *wk = reinterpret_cast<K *>(sm) + warp_in_block() * 256;
+        const int32_t nw = uread(&L.n[0]);
+        for (int64_t q = team_warp(t); q < nw; q += team_nwarps(t)) {
+            const int32_t b = L.warp[q], s = start[b], m = start[b + 1] - s;
+            int P = 128;
+            while (P < m) P <<= 1;
+            for (int x = lane_id(); x < m; x += 32) wk[x] = keys[s + x];
+            __syncwarp();
+            smem_bitonic_keys(wk, m, P, lane_id(), 32, [] { __syncwarp(); });
+            for (int x = lane_id(); x < m; x += 32) emit(b, s + x, wk[x]);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    {
+        K *ck = reinterpret_cast<K *>(sm);
+        const int32_t nc = uread(&L.n[1]);
+        for (int64_t q = t.block(); q < nc; q += t.nblocks()) {
+            const int32_t b = L.cta[q], s = start[b], m = start[b + 1] - s;
+            int P = 512;
+            while (P < m) P <<= 1;
+            for (int x = threadIdx.x; x < m; x += blockDim.x) ck[x] = keys[s + x];
+            __syncthreads();
+            smem_bitonic_keys(ck, m, P, threadIdx.x, blockDim.x, [] { __syncthreads(); });
+            for (int x = threadIdx.x; x < m; x += blockDim.x) emit(b, s + x, ck[x]);
+            __syncthreads();
+        }
+    }
 }
 
 template <class Team, class Bk, class Sub>

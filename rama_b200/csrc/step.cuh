@@ -35,16 +35,32 @@ __device__ void run_step(const Team &t, char *sm, Scratch sc, rama_step_args *a)
     A.rows = a->rows;
     A.cols = a->cols;
     A.cmin = unknown_cost();
+    A.ecols = 0;
+    A.uniq = 0;
     const int op = a->op;
+    if (op == RAMA_STEP_CYCLES || op == RAMA_STEP_MP || op == RAMA_STEP_DUAL) {
+        // what the solver's graphs carry, and costs that the dual may update
+        // where they lie
+        const int32_t *col = A.col;
+        const float *cost = A.cost;
+        A.ecols = 1 + team_max<Team, int32_t>(t, sc, sm, A.n, -1, [=](int64_t e) { return col[e]; });
+        A.uniq = graph_is_simple(t, sc, sm, A);
+        float *copy = sc.arena.take<float>(A.n + 1);
+        if (sc.arena.ok()) {
+            for (int64_t e = t.rank(); e < A.n; e += t.size()) copy[e] = cost[e];
+            A.cost = copy;
+        }
+        t.sync();
+    }
     if (op == RAMA_STEP_INIT) {
         Graph g = graph_from_edges(t, sc, sm, a->i, a->j, a->c, a->m);
         if (sc.arena.ok()) copy_graph_out(t, g, a);
     } else if (op == RAMA_STEP_CONTRACT) {
-        int32_t mx = team_max<Team, int32_t>(t, sc, sm, a->map_size, 0, [&](int64_t k) { return a->map[k]; });
+        int32_t mx = team_max<Team, int32_t>(t, sc, sm, a->map_size, 0, [=](int64_t k) { return a->map[k]; });
         Graph g = graph_contract_raw(t, sc, sm, A, a->map, mx);
         if (sc.arena.ok()) copy_graph_out(t, g, a);
     } else if (op == RAMA_STEP_COARSEN) {
-        int32_t mx = team_max<Team, int32_t>(t, sc, sm, a->map_size, 0, [&](int64_t k) { return a->map[k]; });
+        int32_t mx = team_max<Team, int32_t>(t, sc, sm, a->map_size, 0, [=](int64_t k) { return a->map[k]; });
         int bad = 0;
         Graph g = graph_contract(t, sc, sm, A, a->map, mx, &bad);
         if (sc.arena.ok()) copy_graph_out(t, g, a);
@@ -66,16 +82,16 @@ __device__ void run_step(const Team &t, char *sm, Scratch sc, rama_step_args *a)
             a->status |= err;
         }
     } else if (op == RAMA_STEP_MSF) {
-        int32_t mx = team_max<Team, int32_t>(t, sc, sm, a->m, 0, [&](int64_t e) { return max(a->i[e], a->j[e]); });
-        bool ok = team_msf(t, sc, sm, a->m, mx + 1, [&](int64_t e) { return a->i[e]; },
-                           [&](int64_t e) { return a->j[e]; }, [&](int64_t e) { return a->c[e]; }, a->out_flags);
+        int32_t mx = team_max<Team, int32_t>(t, sc, sm, a->m, 0, [=](int64_t e) { return max(a->i[e], a->j[e]); });
+        bool ok = team_msf(t, sc, sm, a->m, mx + 1, [=](int64_t e) { return a->i[e]; },
+                           [=](int64_t e) { return a->j[e]; }, [=](int64_t e) { return a->c[e]; }, a->out_flags);
         if (t.leader() && !ok) a->status |= ERR_ITER_LIMIT;
     } else if (op == RAMA_STEP_CC) {
         const int32_t *off = a->offsets;
         const int32_t nn = a->num_nodes;
         bool ok = team_cc(
             t, sc, nn, a->adj_len,
-            [&](int64_t k) {
+            [=](int64_t k) {
                 int32_t lo = 0, hi = nn - 1;  // row of entry k: last v with off[v] <= k
                 while (lo < hi) {
                     int32_t mid = (lo + hi + 1) >> 1;
@@ -86,11 +102,11 @@ __device__ void run_step(const Team &t, char *sm, Scratch sc, rama_step_args *a)
                 }
                 return lo;
             },
-            [&](int64_t k) { return a->adj[k]; }, a->out_map);
+            [=](int64_t k) { return a->adj[k]; }, a->out_map);
         if (t.leader() && !ok) a->status |= ERR_ITER_LIMIT;
     } else if (op == RAMA_STEP_CYCLES) {
         TriBuf tb;
-        conflicted_cycles(t, sc, sm, A, a->max_cycle_length, a->tri_memory_factor, a->tol, tb);
+        conflicted_cycles(t, sc, sm, A, a->max_cycle_length, a->tri_memory_factor, a->tol, true, tb);
         if (sc.arena.ok()) {
             if (tb.num <= a->out_tri_cap)
                 for (int64_t k = t.rank(); k < tb.num; k += t.size()) {
@@ -106,6 +122,7 @@ __device__ void run_step(const Team &t, char *sm, Scratch sc, rama_step_args *a)
         }
     } else if (op == RAMA_STEP_MP) {
         TriBuf tb;
+        tb.none = tb.closed = tb.distinct = 0;
         tb.budget = a->T;
         tb.count = a->T;
         tb.num = a->T;
@@ -122,12 +139,14 @@ __device__ void run_step(const Team &t, char *sm, Scratch sc, rama_step_args *a)
             Mp mp;
             if (mp_build(t, sc, sm, A, tb, mp)) {
                 double lb0 = 0.0;
-                const double lb1 = mp_run(t, sc, mp, a->num_iter, -INFINITY, &lb0);
+                float cmin = unknown_cost();
+                const double lb1 = mp_run(t, sc, mp, a->num_iter, -INFINITY, &cmin, &lb0);
                 Graph g;
                 g.row = mp.row;
                 g.col = mp.col;
                 g.cost = mp.cost;
                 g.n = mp.E;
+                g.uniq = 0;
                 graph_set_dims(t, sc, sm, g);
                 copy_graph_out(t, g, a);
                 if (t.leader()) {
@@ -149,7 +168,7 @@ __device__ void run_step(const Team &t, char *sm, Scratch sc, rama_step_args *a)
             a->out_nr = oom;
         }
     } else if (op == RAMA_STEP_CSUM) {
-        double s = team_csum(t, sc, a->m, [&](int64_t k) -> float { return a->c[k]; });
+        double s = team_csum(t, sc, a->m, [=](int64_t k) -> float { return a->c[k]; });
         if (t.leader()) a->out_lb0 = s;
     } else if (op == RAMA_STEP_SORT) {
         uint64_t *k1 = sc.arena.take<uint64_t>(a->m + 1), *k2 = sc.arena.take<uint64_t>(a->m + 1);

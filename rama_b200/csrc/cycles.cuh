@@ -71,7 +71,9 @@ __device__ __forceinline__ void common_blocks(const int32_t *adj, int32_t a0, in
     int32_t a[CB], b[CB];
     auto load = [=](int32_t (&v)[CB], int32_t p, int32_t e, int32_t pad) {
 #pragma unroll
-        for (int k = 0; k < CB; ++k) v[k] = p + k < e ? adj[p + k] : pad;
+        for (int k = 0; k < CB; ++k) v[k] = adj[min(p + k, e - 1)];
+#pragma unroll
+        for (int k = 0; k < CB; ++k) v[k] = p + k < e ? v[k] : pad;
     };
     load(a, a0, a1, 0x7fffffff);
     load(b, b0, b1, 0x7ffffffe);
@@ -373,9 +375,11 @@ __device__ __forceinline__ int64_t expansion_owner(const int64_t *xo, int64_t R,
     return lo;
 }
 
-// The owners of 32 * EXP_RUN consecutive expansions, taken by a warp 32 at a
+// The owners of a run of consecutive expansions, taken by a warp 32 at a
 // time: one search (a probe per lane) for the first, then every lane steps
-// forward from the last owner of the 32 before it.
+// forward from the last owner of the 32 before it.  Runs of up to EXP_RUN
+// times 32, shorter where that would leave warps without work, and 1 where an
+// expansion is a rep edge and needs no search.
 constexpr int EXP_RUN = 8;
 
 struct OwnerWalk {
@@ -430,12 +434,14 @@ __device__ __forceinline__ void expansion_stage(const Team &t, Scratch &sc, char
     const int64_t budget = tb.budget;
     for (int64_t x0 = 0; x0 < X && count <= budget; x0 += CH) {
         const int64_t xn = (X - x0) < CH ? (X - x0) : CH;
+        const int64_t share = xn / (32 * (int64_t)team_nwarps(t));
+        const int run = !xo || share < 1 ? 1 : (share > EXP_RUN ? EXP_RUN : (int)share);
         // count
         int64_t mine = 0;
-        for (int64_t qb = (int64_t)team_warp(t) * (32 * EXP_RUN); qb < xn; qb += (int64_t)team_nwarps(t) * (32 * EXP_RUN)) {
+        for (int64_t qb = (int64_t)team_warp(t) * (32 * run); qb < xn; qb += (int64_t)team_nwarps(t) * (32 * run)) {
             OwnerWalk ow;
             ow.start(xo, R, x0 + qb);
-            for (int k = 0; k < EXP_RUN; ++k) {
+            for (int k = 0; k < run; ++k) {
                 const int64_t q = qb + 32 * k + lane_id();
                 const bool valid = q < xn;
                 const int64_t x = x0 + q, r = ow.next(xo, R, x, valid);
@@ -536,11 +542,11 @@ __device__ __forceinline__ void expansion_stage(const Team &t, Scratch &sc, char
                     cbase[q] = (int32_t)(pmin + (pbig < extra ? pbig : extra));
                     ccount[q] = (int32_t)((v >> 25) + ((v & 1) && pbig < extra ? 1 : 0));
                 });
-            for (int64_t qb = (int64_t)team_warp(t) * (32 * EXP_RUN); qb < xn;
-                 qb += (int64_t)team_nwarps(t) * (32 * EXP_RUN)) {
+            for (int64_t qb = (int64_t)team_warp(t) * (32 * run); qb < xn;
+                 qb += (int64_t)team_nwarps(t) * (32 * run)) {
                 OwnerWalk ow;
                 ow.start(xo, R, x0 + qb);
-                for (int k = 0; k < EXP_RUN; ++k) {
+                for (int k = 0; k < run; ++k) {
                     const int64_t q = qb + 32 * k + lane_id();
                     const bool valid = q < xn;
                     const int64_t x = x0 + q, r = ow.next(xo, R, x, valid);
@@ -596,15 +602,12 @@ __device__ __noinline__ void conflicted_cycles(const Team &t, Scratch &sc, char 
     for (int64_t v = t.rank(); v < N; v += t.size()) haspos[v] = 0;
     for (int64_t v = t.rank(); v <= N; v += t.size()) off[v] = 0;
     t.sync();
-    // four edges a thread at a time: costs, then the ends of the attractive
-    // ones, then the marks
+    // (all three arrays loaded at once: about half of the edges are attractive,
+    // so nearly every sector is needed, and no load waits for another)
     team_for_batched(
-        t, A.n,
-        [=](int64_t e) {
-            return A.cost[e] > pos_tol ? make_int2(A.row[e], A.col[e]) : make_int2(-1, -1);
-        },
-        [=](int64_t, int2 v) {
-            if (v.x >= 0) {
+        t, A.n, [=](int64_t e) { return make_int3(A.row[e], A.col[e], __float_as_int(A.cost[e])); },
+        [=](int64_t, int3 v) {
+            if (__int_as_float(v.z) > pos_tol) {
                 haspos[v.x] = 1;
                 haspos[v.y] = 1;
             }

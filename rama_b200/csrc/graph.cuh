@@ -101,14 +101,310 @@ __device__ __forceinline__ uint64_t pack_key(int32_t a, int32_t b, int nbits)
     return ((uint64_t)(uint32_t)a << nbits) | (uint32_t)b;
 }
 
+// ---------------------------------------------------------------------------
+// Edges ordered by (lo, hi, edge index), for the initial sort and for every
+// contraction.
+//
+// An edge travels as one 16-byte record (hi, edge index, cost bits, lo): the
+// slot pass maps the endpoints and takes a slot in bucket lo by an atomic, a
+// scan gives the bucket starts, and one 128-bit store per edge scatters the
+// record.  Buckets of up to BUCKET_SMALL records stay unordered: the tile pass
+// that reads them next orders them in shared memory.  Longer ones are sorted
+// where they lie (a warp each up to 256, a CTA up to BUCKET_MAX), those beyond
+// BUCKET_MAX by a stable radix sort of (lo, hi) over their edges in input
+// order.  Bound by the scatter (a 32-byte sector per 16-byte record) and by
+// the latency of the gathers and atomics of the slot pass.
+//
+// The form before this one scattered key, payload and bucket to three arrays,
+// ranked every edge against its bucket in global memory, wrote three sorted
+// arrays and read them twice more for the run heads and once for the sums:
+// 15.9 ms for the initial sort and the seven contractions of the 24.8 M
+// edge volume, against 10.6 this way.
+// ---------------------------------------------------------------------------
+struct Records {
+    int4 *rec;       // n: x = hi, y = edge, z = cost bits, w = lo
+    int32_t *start;  // nbk + 1
+    int2 *lohi;      // n: ends in edge order (free after the sort)
+    int32_t *slot;   // n: (free after the sort)
+};
+
+__device__ __forceinline__ uint64_t rec_key(const int4 &r) { return ((uint64_t)(uint32_t)r.x << 32) | (uint32_t)r.y; }
+
+// ends(e): (lo, hi) of edge e, loads only; nbh: bits of a node id
+template <class Team, class Ends>
+__device__ __forceinline__ bool team_sort_records(const Team &t, Scratch &sc, char *sm, int64_t n, int32_t nbk,
+                                                  int nbh, const float *cost, Ends ends, Records &R)
+{
+    R.rec = sc.arena.take<int4>(n + 1);
+    R.start = sc.arena.take<int32_t>((int64_t)nbk + 2);
+    R.lohi = sc.arena.take<int2>(n + 1);
+    R.slot = sc.arena.take<int32_t>(n + 1);
+    BucketLists L = bucket_lists(sc, n);
+    if (!sc.arena.ok()) return false;
+    int4 *rec = R.rec;
+    int32_t *start = R.start, *slot = R.slot;
+    int2 *lohi = R.lohi;
+    for (int64_t b = t.rank(); b <= nbk; b += t.size()) start[b] = 0;
+    if (t.rank() < 4) L.n[t.rank()] = 0;
+    t.sync();
+    {
+        // SORT_BATCH strides of a warp at a time: the ends, then the atomics,
+        // then the stores
+        constexpr int U = SORT_BATCH;
+        const int64_t S = t.size();
+        int64_t base = (int64_t)t.rank() - lane_id();
+        for (; base + (U - 1) * S + 31 < n; base += S * U) {
+            int2 w[U];
+            int32_t s[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) w[k] = ends(base + k * S + lane_id());
+#pragma unroll
+            for (int k = 0; k < U; ++k) s[k] = bucket_slot(start, w[k].x);
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                lohi[base + k * S + lane_id()] = w[k];
+                slot[base + k * S + lane_id()] = s[k];
+            }
+        }
+        for (; base < n; base += S) {
+            const int64_t e = base + lane_id();
+            const int2 w = e < n ? ends(e) : make_int2(-1, -1);
+            const int32_t s = bucket_slot(start, w.x);
+            if (e < n) {
+                lohi[e] = w;
+                slot[e] = s;
+            }
+        }
+    }
+    t.sync();
+    prof_mark(t, sc, PH_CSORT_SLOT);
+    team_bucket_starts(t, sc, sm, nbk, start, L, [](int64_t, int32_t, int32_t) {});
+    struct Item {
+        int4 r;
+        int32_t p;
+    };
+    team_for_batched(
+        t, n,
+        [=](int64_t e) {
+            const int2 w = lohi[e];
+            Item x;
+            x.r = make_int4(w.y, (int32_t)e, __float_as_int(cost[e]), w.x);
+            x.p = start[w.x] + slot[e];
+            return x;
+        },
+        [=](int64_t, Item x) { rec[x.p] = x.r; });
+    t.sync();
+    prof_mark(t, sc, PH_CSORT_SCATTER);
+    if (L.has_long()) {
+        // 65..256 records: a warp; up to BUCKET_MAX: a CTA
+        const int NW = blockDim.x >> 5;
+        {
+            uint64_t *wk = reinterpret_cast<uint64_t *>(sm) + warp_in_block() * 256;
+            int32_t *wi = reinterpret_cast<int32_t *>(sm + NW * 256 * 8) + warp_in_block() * 256;
+            const int32_t nw = uread(&L.n[0]);
+            for (int64_t q = team_warp(t); q < nw; q += team_nwarps(t)) {
+                const int32_t b = L.warp[q], s = start[b], m = start[b + 1] - s;
+                int P = 128;
+                while (P < m) P <<= 1;
+                for (int x = lane_id(); x < m; x += 32) {
+                    const int4 r = rec[s + x];
+                    wk[x] = rec_key(r);
+                    wi[x] = r.z;
+                }
+                __syncwarp();
+                smem_bitonic(wk, wi, m, P, lane_id(), 32, [] { __syncwarp(); });
+                for (int x = lane_id(); x < m; x += 32)
+                    rec[s + x] = make_int4((int32_t)(wk[x] >> 32), (int32_t)(uint32_t)wk[x], wi[x], b);
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        {
+            uint64_t *ck = reinterpret_cast<uint64_t *>(sm);
+            int32_t *ci = reinterpret_cast<int32_t *>(sm + BUCKET_MAX * 8);
+            const int32_t nc = uread(&L.n[1]);
+            for (int64_t q = t.block(); q < nc; q += t.nblocks()) {
+                const int32_t b = L.cta[q], s = start[b], m = start[b + 1] - s;
+                int P = 512;
+                while (P < m) P <<= 1;
+                for (int x = threadIdx.x; x < m; x += blockDim.x) {
+                    const int4 r = rec[s + x];
+                    ck[x] = rec_key(r);
+                    ci[x] = r.z;
+                }
+                __syncthreads();
+                smem_bitonic(ck, ci, m, P, threadIdx.x, blockDim.x, [] { __syncthreads(); });
+                for (int x = threadIdx.x; x < m; x += blockDim.x)
+                    rec[s + x] = make_int4((int32_t)(ck[x] >> 32), (int32_t)(uint32_t)ck[x], ci[x], b);
+                __syncthreads();
+            }
+        }
+        t.sync();
+    }
+    prof_mark(t, sc, PH_CSORT_RANK);
+    if (L.has_big()) {
+        // the buckets beyond BUCKET_MAX: their edges in input order, a stable
+        // radix sort of (lo, hi), then each into its bucket's range
+        auto is_big = [=](int64_t e) {
+            const int32_t b = lohi[e].x;
+            return start[b + 1] - start[b] > BUCKET_MAX;
+        };
+        uint64_t bm = sc.arena.mark();
+        const int64_t nbig = team_sum<Team, int64_t>(t, sc, sm, n, [=](int64_t e) -> int64_t { return is_big(e) ? 1 : 0; });
+        uint64_t *bk1 = sc.arena.take<uint64_t>(nbig + 1), *bk2 = sc.arena.take<uint64_t>(nbig + 1);
+        int32_t *bv1 = sc.arena.take<int32_t>(nbig + 1), *bv2 = sc.arena.take<int32_t>(nbig + 1);
+        int32_t *kfirst = sc.arena.take<int32_t>((int64_t)nbk + 1);
+        if (!sc.arena.ok()) return false;
+        team_compact(t, sc, sm, n, is_big, [=](int64_t e, int64_t k) {
+            const int2 w = lohi[e];
+            bk1[k] = ((uint64_t)(uint32_t)w.x << nbh) | (uint32_t)w.y;
+            bv1[k] = (int32_t)e;
+        });
+        team_sort_pairs(t, sc, sm, bk1, bv1, bk2, bv2, nbig, 2 * nbh);
+        for (int64_t k = t.rank(); k < nbig; k += t.size()) {
+            const int32_t b = (int32_t)(bk1[k] >> nbh);
+            if (k == 0 || (int32_t)(bk1[k - 1] >> nbh) != b) kfirst[b] = (int32_t)k;
+        }
+        t.sync();
+        const uint64_t mask = (uint64_t(1) << nbh) - 1;
+        for (int64_t k = t.rank(); k < nbig; k += t.size()) {
+            const int32_t b = (int32_t)(bk1[k] >> nbh), e = bv1[k];
+            rec[start[b] + (k - kfirst[b])] = make_int4((int32_t)(bk1[k] & mask), e, __float_as_int(cost[e]), b);
+        }
+        t.sync();
+        sc.arena.release(bm);
+        prof_mark(t, sc, PH_CSORT_BIG);
+    }
+    return true;
+}
+
+// Walks the ordered records of this CTA's share in tiles held in shared
+// memory.  A tile is a window of 4 * blockDim records less BUCKET_SMALL: the
+// CTA that holds a small bucket's first record has all of it in its window,
+// and orders it there (every record goes to the number of smaller keys in its
+// bucket; the records pass through registers).  Records of longer buckets are
+// in order already and belong to the tile that holds them.
+//
+// visit(T, base, prev, mine) is called by every thread of the CTA once per
+// tile, for its records win[base + 32 k] (k < 4; position order over (k, lane)
+// within a warp's 128): prev[k] is the record before, mine[k] whether the
+// position belongs to this CTA.  Two windows in turn, so that a tile's records
+// are read while slower warps still visit the last one's.
+struct RecTile {
+    const int4 *win;  // the window, win[0] at position p0
+    int64_t p0;
+    int64_t begin;    // this CTA's records of the tile: [begin, end)
+    int64_t end;
+};
+
+// first position at or after p that no earlier tile owns
+__device__ __forceinline__ int64_t rec_owned_from(const Records &R, int64_t p, int64_t n)
+{
+    if (p >= n) return n;
+    const int32_t lo = R.rec[p].w;
+    const int32_t s = R.start[lo], e = R.start[lo + 1];
+    return e - s > BUCKET_SMALL || s == p ? p : e;
+}
+
+template <class Team, class Visit>
+__device__ __forceinline__ void team_record_tiles(const Team &t, char *sm, const Records &R, int64_t n, Visit visit)
+{
+    constexpr int K = 4;
+    const int W = K * blockDim.x, TILE = W - BUCKET_SMALL;
+    const int64_t ntiles = (n + TILE - 1) / TILE;
+    const int64_t per = (ntiles + t.nblocks() - 1) / t.nblocks();
+    const int64_t t0 = (int64_t)t.block() * per;
+    const int64_t t1 = t0 + per < ntiles ? t0 + per : ntiles;
+    const int base = warp_in_block() * 32 * K + lane_id();
+    int64_t a = t0 < t1 ? rec_owned_from(R, t0 * TILE, n) : n;
+    int flip = 0;
+    for (int64_t tile = t0; tile < t1; ++tile, flip ^= 1) {
+        int4 *win = reinterpret_cast<int4 *>(sm) + flip * W;
+        const int64_t p0 = tile * TILE;
+        const int64_t b = rec_owned_from(R, p0 + TILE, n);
+        int4 r[K];
+        int32_t s[K], e[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int64_t p = p0 + base + 32 * k;
+            r[k] = R.rec[p < n ? p : n - 1];
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            s[k] = R.start[r[k].w];
+            e[k] = R.start[r[k].w + 1];
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) win[base + 32 * k] = r[k];
+        __syncthreads();
+        int dst[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int i = base + 32 * k;
+            const int64_t p = p0 + i;
+            dst[k] = i;
+            if (p >= a && p < b && e[k] - s[k] <= BUCKET_SMALL) {
+                const uint64_t key = rec_key(r[k]);
+                const int f = (int)(s[k] - p0), l = (int)(e[k] - p0);
+                int rank = 0;
+                for (int x = f; x < l; ++x) rank += rec_key(win[x]) < key;
+                dst[k] = f + rank;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int64_t p = p0 + base + 32 * k;
+            if (p >= a && p < b) win[dst[k]] = r[k];
+        }
+        __syncthreads();
+        RecTile T;
+        T.win = win;
+        T.p0 = p0;
+        T.begin = a;
+        T.end = b;
+        const int4 none = make_int4(-1, -1, 0, -1);
+        int4 prev[K];
+        bool mine[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int i = base + 32 * k;
+            const int64_t p = p0 + i;
+            mine[k] = p >= a && p < b;
+            prev[k] = !mine[k] ? none : (p > a ? win[i - 1] : (p > 0 ? R.rec[p - 1] : none));
+        }
+        visit(T, base, prev, mine);
+        a = b;
+    }
+    __syncthreads();  // the windows are free again
+}
+
+// shared memory of two windows of a CTA of `threads` threads
+__host__ __device__ constexpr int record_smem_bytes(int threads) { return 2 * 4 * threads * 16; }
+
+// the graph slot at the top of the arena, for n edges (team-uniform; fails
+// when it would overlap live temporaries)
+__device__ __forceinline__ bool graph_slot(Scratch &sc, int64_t n, Graph &g, uint64_t &top)
+{
+    Arena &ar = sc.arena;
+    const uint64_t bytes = (uint64_t)(n + 1) * 12 + 3 * 256;
+    top = (ar.cap - bytes) & ~uint64_t(255);
+    if (ar.failed || bytes > ar.cap || top < ar.lo) {
+        ar.failed = 1;
+        return false;
+    }
+    const uint64_t words = ((uint64_t)(n + 1) * 4 + 255) / 256 * 256;
+    g.row = reinterpret_cast<int32_t *>(ar.base + top);
+    g.col = reinterpret_cast<int32_t *>(ar.base + top + words);
+    g.cost = reinterpret_cast<float *>(ar.base + top + 2 * words);
+    return true;
+}
+
 // dCOO ctor with unsorted input (src/dCOO.cu:38-45): endpoints ordered,
-// sorted by (row,col), stable.  Inputs are (i, j, c) of length n.
-// By buckets of the smaller endpoint: the bucket sort orders each bucket by
-// (larger endpoint, edge index) and carries the cost bits and the bucket
-// along, and the sorted edges are written straight into the graph slot.
-// Buckets of more than BUCKET_MAX edges go through a stable radix sort of
-// their packed (min, max) keys inside the bucket sort; edge lists of 2^31 or
-// more take graph_from_edges_sorted (one radix sort of every edge's keys).
+// sorted by (row,col), stable.  Inputs are (i, j, c) of length n.  The sorted
+// edges go straight from the tile pass into the graph slot; edge lists of
+// 2^31 or more take graph_from_edges_sorted (one radix sort of every edge's
+// keys).
 template <class Team>
 __device__ __noinline__ Graph graph_from_edges_sorted(const Team &t, Scratch &sc, char *, const int32_t *i, const int32_t *j,
                                          const float *c, int64_t n);
@@ -119,66 +415,47 @@ __device__ __noinline__ Graph graph_from_edges(const Team &t, Scratch &sc, char 
 {
     char *sm = team_smem();
     if (n == 0 || n >= (int64_t(1) << 31)) return graph_from_edges_sorted(t, sc, sm, i, j, c, n);
-    Graph out;
-    out.n = n;
-    out.rows = out.cols = out.ecols = 0;
-    out.uniq = 0;
-    out.cmin = unknown_cost();
+    Graph g;
+    g.n = n;
+    g.rows = g.cols = g.ecols = 0;
+    g.uniq = 0;
+    g.cmin = unknown_cost();
     const int32_t mx = team_max<Team, int32_t>(t, sc, sm, n, 0, [=](int64_t e) { return i[e] > j[e] ? i[e] : j[e]; });
     const int nbh = bits_for((uint64_t)(mx > 0 ? mx : 1));
     uint64_t m = sc.arena.mark();
-    int2 *lohi = sc.arena.take<int2>(n + 1);
-    uint64_t *sk = sc.arena.take<uint64_t>(n + 1);
-    int32_t *sbits = sc.arena.take<int32_t>(n + 1);
-    int32_t *sbk = sc.arena.take<int32_t>(n + 1);
-    int32_t *bst = sc.arena.take<int32_t>((int64_t)mx + 2);
-    int32_t *dup = sc.arena.take<int32_t>(1);
-    if (!sc.arena.ok()) return out;
-    if (t.rank() == 0) dup[0] = 0;
-    const bool done = team_bucket_sort_ex(
-        t, sc, sm, n, mx + 1,
-        [=](int64_t e) -> int64_t {
-            const int32_t a = i[e], b = j[e];
-            const int32_t lo = a < b ? a : b, hi = a < b ? b : a;
-            return ((int64_t)hi << 32) | (uint32_t)lo;
-        },
-        [=](int64_t e) { return lohi[e].x; },
-        [=](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].y << 32) | (uint64_t)e; },
-        [=](int64_t e) { return __float_as_int(c[e]); }, sk, sbits, bst, sbk, -1,
-        [=](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].x << nbh) | (uint32_t)lohi[e].y; },
-        2 * nbh, [=](int64_t e, int64_t w) { lohi[e] = make_int2((int32_t)(uint32_t)w, (int32_t)(w >> 32)); });
-    if (!done) return out;
-    Arena &ar = sc.arena;
-    const uint64_t bytes = (uint64_t)(n + 1) * 12 + 3 * 256;
-    const uint64_t top = (ar.cap - bytes) & ~uint64_t(255);
-    if (ar.failed || bytes > ar.cap || top < ar.lo) {
-        ar.failed = 1;
-        return out;
-    }
-    const uint64_t words = ((uint64_t)(n + 1) * 4 + 255) / 256 * 256;
-    Graph g;
-    g.row = reinterpret_cast<int32_t *>(ar.base + top);
-    g.col = reinterpret_cast<int32_t *>(ar.base + top + words);
-    g.cost = reinterpret_cast<float *>(ar.base + top + 2 * words);
-    g.n = n;
-    team_for_batched(
-        t, n,
-        [=](int64_t p) {
-            const int64_t q = p > 0 ? p - 1 : 0;
-            const int32_t hi = (int32_t)(sk[p] >> 32);
-            const int same = p > 0 && sbk[q] == sbk[p] && (int32_t)(sk[q] >> 32) == hi;
-            return make_int4(sbk[p], hi, sbits[p], same);
-        },
-        [=](int64_t p, int4 v) {
-            g.row[p] = v.x;
-            g.col[p] = v.y;
-            g.cost[p] = __int_as_float(v.z);
-            if (v.w) dup[0] = 1;
-        });
-    t.sync();
-    graph_set_dims(t, sc, sm, g);
-    g.uniq = uread(dup) == 0;
-    ar.top = top;
+    Records R;
+    if (!team_sort_records(
+            t, sc, sm, n, mx + 1, nbh, c,
+            [=](int64_t e) {
+                const int32_t a = i[e], b = j[e];
+                return a < b ? make_int2(a, b) : make_int2(b, a);
+            },
+            R))
+        return g;
+    uint64_t top;
+    if (!graph_slot(sc, n, g, top)) return g;
+    int32_t dup = 0;
+    float mn = 3.4e38f;
+    team_record_tiles(t, sm, R, n, [&](const RecTile &T, int base, const int4 (&prev)[4], const bool (&mine)[4]) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (mine[k]) {
+                const int4 r = T.win[base + 32 * k];
+                const int64_t p = T.p0 + base + 32 * k;
+                g.row[p] = r.w;
+                g.col[p] = r.x;
+                g.cost[p] = __int_as_float(r.z);
+                if (r.w != r.x) mn = fminf(mn, __int_as_float(r.z));
+                dup |= prev[k].w == r.w && prev[k].x == r.x;
+            }
+    });
+    team_fold_maxi_minf(t, sc, sm, dup, mn);
+    // dims as in dCOO::init (src/dCOO.cu:47-51); the largest endpoint is a column
+    g.cols = g.ecols = mx + 1;
+    g.rows = uread(&R.rec[n - 1].w) + 1;
+    g.cmin = mn;
+    g.uniq = dup == 0;
+    sc.arena.top = top;
     sc.arena.release(m);
     sc.alg_bytes += 24.0 * (double)n;
     return g;
@@ -381,238 +658,260 @@ __device__ __noinline__ Graph graph_contract_sorted(const Team &t, Scratch &sc, 
 
 // The contraction (dCOO::contract_cuda + has_bad_contractions +
 // remove_diagonal) by buckets of the new row:
-//   1. each edge's contracted endpoints (lo, hi) are computed once, with its
-//      slot in bucket lo;
-//   2. the bucket sort orders every bucket by (hi, edge index), carrying the
-//      edge's cost bits and its bucket along (no gather afterwards);
-//   3. one scan over the sorted edges finds the heads of the runs of equal
-//      (lo, hi) and numbers the runs that are not self-loops; the head's
-//      thread sums its run (RSUM in edge order; runs of more than 32 by a
-//      warp afterwards) and writes the edge straight into the graph slot at
-//      the top of the arena (the old graph there is dead by then), or checks
-//      a self-loop's sum for a bad contraction;
-//   4. one pass over the new edges gives the largest column and the smallest
-//      cost; the rows are the last bucket + 1 (dims are taken before the
-//      diagonal goes, as the reference does).
-// Buckets of more than BUCKET_MAX edges are sorted by a stable radix sort of
-// their packed (lo, hi) keys inside the bucket sort; graph_contract_sorted
-// (one radix sort of every edge's packed keys) remains for edge lists of
-// 2^31 edges or more.  Both give the same graph bit for bit.
+//   1. the edges are ordered by their contracted ends (team_sort_records);
+//   2. a tile pass finds the heads of the runs of equal (lo, hi); a head's
+//      thread sums its run in edge order (RSUM) out of the tile and appends
+//      the edge to its CTA's part of the output, or checks a self-loop's sum
+//      for a bad contraction; runs of more than 32 records of long buckets go
+//      to warps afterwards, runs of more than RSUM_CHUNK by chunks to many;
+//   3. the CTAs' parts are joined in the graph slot at the top of the arena
+//      (the old graph there is dead by then), with the largest column and the
+//      smallest cost on the way; a single CTA writes there directly.  The
+//      rows are the last bucket + 1 (dims are taken before the diagonal goes,
+//      as the reference does).
+// graph_contract_sorted (one radix sort of every edge's packed keys) remains
+// for edge lists of 2^31 edges or more.  Both give the same graph bit for bit.
 template <class Team>
-__device__ __noinline__ Graph graph_contract(const Team &t, Scratch &sc, char *, const Graph &A, const int32_t *map,
-                                int32_t map_max, int *bad)
+__device__ __noinline__ Graph graph_contract(const Team &t, Scratch &sc, char *, const Graph &graph,
+                                             const int32_t *map, int32_t map_max, int *bad)
 {
     char *sm = team_smem();
+    const Graph A = graph;  // its pointers in registers
     const int64_t n = A.n;
     Graph out = A;
     if (n == 0 || n >= (int64_t(1) << 31)) return graph_contract_sorted(t, sc, sm, A, map, map_max, bad);
-    const int32_t nbk = map_max + 1;
     const int nbh = bits_for((uint64_t)(map_max > 0 ? map_max : 1));
     uint64_t m = sc.arena.mark();
-    int2 *lohi = sc.arena.take<int2>(n + 1);
-    uint64_t *sk = sc.arena.take<uint64_t>(n + 1);
-    int32_t *sbits = sc.arena.take<int32_t>(n + 1);
-    int32_t *sbk = sc.arena.take<int32_t>(n + 1);
-    int32_t *bst = sc.arena.take<int32_t>((int64_t)nbk + 2);
-    int4 *longq = sc.arena.take<int4>(n / 33 + 2);
     // [0] bad, [1] long runs, [2] largest self-loop column
     int32_t *fl = sc.arena.take<int32_t>(8);
+    int4 *longq = sc.arena.take<int4>(n / 33 + 2);  // long runs: first and last position, output (-1: self-loop)
     if (!sc.arena.ok()) return out;
     if (t.rank() == 0) {
         fl[0] = 0;
         fl[1] = 0;
         fl[2] = -1;
     }
-    const bool done = team_bucket_sort_ex(
-        t, sc, sm, n, nbk,
-        [=](int64_t e) -> int64_t {
-            const int32_t a = map[A.row[e]], b = map[A.col[e]];
-            const int32_t lo = a < b ? a : b, hi = a < b ? b : a;
-            return ((int64_t)hi << 32) | (uint32_t)lo;
-        },
-        [=](int64_t e) { return lohi[e].x; },
-        [=](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].y << 32) | (uint64_t)e; },
-        [=](int64_t e) { return __float_as_int(A.cost[e]); }, sk, sbits, bst, sbk, PH_CSORT_SLOT,
-        [=](int64_t e) -> uint64_t { return ((uint64_t)(uint32_t)lohi[e].x << nbh) | (uint32_t)lohi[e].y; },
-        2 * nbh, [=](int64_t e, int64_t w) { lohi[e] = make_int2((int32_t)(uint32_t)w, (int32_t)(w >> 32)); });
-    if (!done) {
-        sc.arena.release(m);
-        return graph_contract_sorted(t, sc, sm, A, map, map_max, bad);
-    }
+    Records R;
+    if (!team_sort_records(
+            t, sc, sm, n, map_max + 1, nbh, A.cost,
+            [=](int64_t e) {
+                const int32_t a = map[A.row[e]], b = map[A.col[e]];
+                return a < b ? make_int2(a, b) : make_int2(b, a);
+            },
+            R))
+        return out;
     // the new graph's slot, sized for at most n edges; it ends at the arena's
     // end, so it lies within the old graph's slot (n is the old edge count)
-    Arena &ar = sc.arena;
-    const uint64_t bytes = (uint64_t)(n + 1) * 12 + 3 * 256;
-    const uint64_t top = (ar.cap - bytes) & ~uint64_t(255);
-    if (ar.failed || bytes > ar.cap || top < ar.lo) {
-        ar.failed = 1;
-        return out;
-    }
+    Graph h;
+    uint64_t top;
+    if (!graph_slot(sc, n, h, top)) return out;
     // temporaries taken from here on stay below the new slot (when the old
     // graph does not live in the slot, as in a single step, the arena's top
     // is its end)
-    if (top < ar.top) ar.top = top;
-    const uint64_t words = ((uint64_t)(n + 1) * 4 + 255) / 256 * 256;
-    Graph h;
-    h.row = reinterpret_cast<int32_t *>(ar.base + top);
-    h.col = reinterpret_cast<int32_t *>(ar.base + top + words);
-    h.cost = reinterpret_cast<float *>(ar.base + top + 2 * words);
-    // 3. heads of the runs: one scan counts every run (high 32 bits) and the
-    //    runs that are not self-loops (low 32 bits), writes the row and column
-    //    of each new edge and notes each run's start and output slot (-1: a
-    //    self-loop).  Then a pass over the runs sums each one, its end being
-    //    the next run's start: runs of up to 32 edges by one thread, longer
-    //    ones by a warp afterwards.
-    auto head = [=](int64_t p) {
-        return p == 0 || sbk[p] != sbk[p - 1] || (sk[p] >> 32) != (sk[p - 1] >> 32);
-    };
-    // lohi is dead after the sort: its two halves hold the runs' starts and slots
-    int32_t *runstart = reinterpret_cast<int32_t *>(lohi);
-    int32_t *runk = runstart + (n + 1);
-    // the largest self-loop column, per thread first: one atomic per warp
-    // afterwards instead of one per self-loop run on a single word
-    int32_t dloc = -1;
-    const int64_t packed = team_scan<Team, int64_t>(
-        t, sc, sm, n,
-        [=](int64_t p) -> int64_t {
-            if (!head(p)) return 0;
-            return (int64_t(1) << 32) | ((int32_t)(sk[p] >> 32) != sbk[p] ? 1 : 0);
-        },
-        [=, &dloc](int64_t p, int64_t pre, int64_t v) {
-            if (!v) return;
-            const int64_t k = pre & 0xffffffffll, r = pre >> 32;
-            const int32_t b = sbk[p], hi = (int32_t)(sk[p] >> 32);
-            runstart[r] = (int32_t)p;
-            if (v & 1) {
-                runk[r] = (int32_t)k;
-                h.row[k] = b;
-                h.col[k] = hi;
-            } else {
-                runk[r] = -1;
-                dloc = hi > dloc ? hi : dloc;
-            }
-        });
-    const int64_t nk = packed & 0xffffffffll, nruns = packed >> 32;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const int32_t x = __shfl_xor_sync(FULL, dloc, o);
-        dloc = x > dloc ? x : dloc;
-    }
-    if (lane_id() == 0 && dloc >= 0) atomicMax(&fl[2], dloc);
-    const float *cost_sorted = reinterpret_cast<const float *>(sbits);
-    // a run's sum goes to its edge; a self-loop's negative sum is a bad contraction
-    auto finish = [=](int32_t k, float sum) {
-        if (k >= 0)
-            h.cost[k] = sum;
-        else if (sum < 0.0f)
-            fl[0] = 1;
-    };
-    {
-        // four runs a thread at a time: starts and slots, then the sums
-        constexpr int U = 4;
-        const int64_t S = t.size();
-        int64_t r0 = t.rank();
-        auto one = [=](int64_t r, int32_t s, int32_t e, int32_t k) {
-            const int32_t len = e - s;
-            if (len <= RSUM_THREAD_MAX)
-                finish(k, rsum_upto8(cost_sorted + s, len));
-            else if (len <= 32)
-                finish(k, rsum_upto32(cost_sorted + s, len));
+    if (top < sc.arena.top) sc.arena.top = top;
+    // where a CTA's edges go first: its own records' positions in two arrays
+    // that the sort no longer needs, or the slot itself
+    const bool direct = t.nblocks() == 1;
+    int2 *tends = R.lohi;
+    float *tcost = reinterpret_cast<float *>(R.slot);
+    __shared__ int32_t wtot[2][32];
+    int64_t first = -1;  // this CTA's first record
+    int64_t kept = 0;    // edges it has written
+    int parity = 0;
+    int32_t dloc = -1;  // largest self-loop column
+    auto finish = [=](int64_t k, float sum) {
+        if (k >= 0) {
+            if (direct)
+                h.cost[k] = sum;
             else
-                longq[atomicAdd(&fl[1], 1)] = make_int4(s, e, k, 0);
-        };
-        for (; r0 + (U - 1) * S < nruns; r0 += U * S) {
-            int32_t s[U], e[U], k[U];
-#pragma unroll
-            for (int j = 0; j < U; ++j) {
-                const int64_t r = r0 + j * S;
-                s[j] = runstart[r];
-                e[j] = r + 1 < nruns ? runstart[r + 1] : (int32_t)n;
-                k[j] = runk[r];
-            }
-#pragma unroll
-            for (int j = 0; j < U; ++j) one(r0 + j * S, s[j], e[j], k[j]);
+                tcost[k] = sum;
+        } else if (sum < 0.0f) {
+            fl[0] = 1;
         }
-        for (; r0 < nruns; r0 += S)
-            one(r0, runstart[r0], r0 + 1 < nruns ? runstart[r0 + 1] : (int32_t)n, runk[r0]);
+    };
+    team_record_tiles(t, sm, R, n, [&](const RecTile &T, int base, const int4 (&prev)[4], const bool (&mine)[4]) {
+        int4 r[4];
+        bool head[4];
+        unsigned keep[4];
+        int wsum = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            r[k] = T.win[base + 32 * k];
+            head[k] = mine[k] && (prev[k].w != r[k].w || prev[k].x != r[k].x);
+            keep[k] = __ballot_sync(FULL, head[k] && r[k].w != r[k].x);
+            wsum += __popc(keep[k]);
+        }
+        if (lane_id() == 0) wtot[parity][warp_in_block()] = wsum;
+        __syncthreads();
+        const int nw = blockDim.x >> 5;
+        const int wt = lane_id() < nw ? wtot[parity][lane_id()] : 0;
+        const int incl = warp_incl_scan(wt);
+        parity ^= 1;
+        if (first < 0) first = T.begin;  // (its edges are no more than its records)
+        int64_t k0 = (direct ? 0 : first) + kept +
+                     (warp_in_block() > 0 ? __shfl_sync(FULL, incl, warp_in_block() - 1) : 0);
+        kept += __shfl_sync(FULL, incl, 31);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int64_t mk = k0 + __popc(keep[k] & lanemask_lt());
+            k0 += __popc(keep[k]);
+            if (!head[k]) continue;
+            const bool loop = r[k].w == r[k].x;
+            const int64_t o = loop ? -1 : mk;
+            if (loop) {
+                dloc = max(dloc, r[k].x);
+            } else if (direct) {
+                h.row[o] = r[k].w;
+                h.col[o] = r[k].x;
+            } else {
+                tends[o] = make_int2(r[k].w, r[k].x);
+            }
+            // the run's end: within the tile, or anywhere in a long bucket
+            const int i = base + 32 * k;
+            const int lim = (int)(T.end - T.p0 < i + 33 ? T.end - T.p0 : i + 33);
+            int x = i + 1;
+            while (x < lim && T.win[x].x == r[k].x && T.win[x].w == r[k].w) ++x;
+            if (x == lim) {
+                const int32_t s = R.start[r[k].w], e = R.start[r[k].w + 1];
+                if (e - s > BUCKET_SMALL) {
+                    // first record of the bucket with a larger hi
+                    int64_t lo = T.p0 + x, hi = e;
+                    while (lo < hi) {
+                        const int64_t mid = (lo + hi) >> 1;
+                        if (R.rec[mid].x <= r[k].x)
+                            lo = mid + 1;
+                        else
+                            hi = mid;
+                    }
+                    const int64_t p = T.p0 + i;
+                    if (lo - p > 32)
+                        longq[atomicAdd(&fl[1], 1)] = make_int4((int32_t)p, (int32_t)lo, (int32_t)o, 0);
+                    else
+                        finish(o, rsum_upto64((int)(lo - p), [=](int q) { return __int_as_float(R.rec[p + q].z); }));
+                    continue;
+                }
+                const int l = (int)(e - T.p0);
+                while (x < l && T.win[x].x == r[k].x) ++x;
+            }
+            const int4 *v = T.win + i;
+            finish(o, rsum_upto64(x - i, [=](int q) { return __int_as_float(v[q].z); }));
+        }
+    });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dloc = max(dloc, __shfl_xor_sync(FULL, dloc, o));
+    if (lane_id() == 0 && dloc >= 0) atomicMax(&fl[2], dloc);
+    int64_t obase = 0, nk = kept;
+    if (!direct) {
+        int64_t *part = reinterpret_cast<int64_t *>(sc.next_part());
+        if (threadIdx.x == 0) part[t.block()] = kept;
+        t.sync();
+        cta_prefix_parts(t, sc, part, obase, nk);
+    } else {
+        t.sync();
     }
-    t.sync();
     // runs of 33..RSUM_CHUNK edges: a warp each.  Longer runs (a cluster's
     // self-loop run can hold a large part of the graph): their chunks of
     // RSUM_CHUNK edges are shared out over every warp of the team, then a warp
     // per run sums its chunk sums -- the same sum as rsum_warp.
     const int32_t nl = uread(&fl[1]);
-    int64_t nchunks = 0;
-    int32_t *coff = nullptr;
-    double *chunk_sum = nullptr;
     if (nl > 0) {
-        coff = sc.arena.take<int32_t>((int64_t)nl + 1);
+        const int4 *rec = R.rec;
+        int32_t *coff = sc.arena.take<int32_t>((int64_t)nl + 1);
         if (!sc.arena.ok()) return out;
-        nchunks = team_scan<Team, int64_t>(
+        const int64_t nchunks = team_scan<Team, int64_t>(
             t, sc, sm, nl,
             [=](int64_t q) -> int64_t {
                 const int64_t len = longq[q].y - longq[q].x;
                 return len > RSUM_CHUNK ? (len + RSUM_CHUNK - 1) / RSUM_CHUNK : 0;
             },
             [=](int64_t q, int64_t pre, int64_t) { coff[q] = (int32_t)pre; });
-        chunk_sum = sc.arena.take<double>(nchunks + 1);
+        double *chunk_sum = sc.arena.take<double>(nchunks + 1);
         if (!sc.arena.ok()) return out;
-    }
-    for (int64_t w = team_warp(t); w < nl + nchunks; w += team_nwarps(t)) {
-        if (w < nl) {
-            const int4 L = longq[w];
-            if (L.y - L.x <= RSUM_CHUNK) {
-                const float v = (float)rsum_chunk_warp(L.y - L.x, [=](int64_t x) { return cost_sorted[L.x + x]; });
-                if (lane_id() == 0) finish(L.z, v);
+        for (int64_t w = team_warp(t); w < nl + nchunks; w += team_nwarps(t)) {
+            if (w < nl) {
+                const int4 L = longq[w];
+                if (L.y - L.x <= RSUM_CHUNK) {
+                    const float v =
+                        (float)rsum_chunk_warp(L.y - L.x, [=](int64_t x) { return __int_as_float(rec[L.x + x].z); });
+                    if (lane_id() == 0) finish(L.z, v);
+                }
+            } else {
+                // chunk g belongs to the last run q with coff[q] <= g
+                const int64_t g = w - nl;
+                int32_t lo = 0, hi = nl - 1;
+                while (lo < hi) {
+                    const int32_t mid = (lo + hi + 1) >> 1;
+                    if (coff[mid] <= g)
+                        lo = mid;
+                    else
+                        hi = mid - 1;
+                }
+                const int4 L = longq[lo];
+                const int64_t cb = L.x + (g - coff[lo]) * RSUM_CHUNK;
+                const int64_t len = L.y - cb < RSUM_CHUNK ? L.y - cb : RSUM_CHUNK;
+                const double d = rsum_chunk_warp(len, [=](int64_t x) { return __int_as_float(rec[cb + x].z); });
+                if (lane_id() == 0) chunk_sum[g] = d;
             }
-        } else {
-            // chunk g belongs to the last run q with coff[q] <= g
-            const int64_t g = w - nl;
-            int32_t lo = 0, hi = nl - 1;
-            while (lo < hi) {
-                const int32_t mid = (lo + hi + 1) >> 1;
-                if (coff[mid] <= g)
-                    lo = mid;
-                else
-                    hi = mid - 1;
-            }
-            const int4 L = longq[lo];
-            const int64_t base = L.x + (g - coff[lo]) * RSUM_CHUNK;
-            const int64_t len = L.y - base < RSUM_CHUNK ? L.y - base : RSUM_CHUNK;
-            const double d = rsum_chunk_warp(len, [=](int64_t x) { return cost_sorted[base + x]; });
-            if (lane_id() == 0) chunk_sum[g] = d;
-        }
-    }
-    t.sync();
-    if (nchunks > 0) {
-        for (int64_t w = team_warp(t); w < nl; w += team_nwarps(t)) {
-            const int4 L = longq[w];
-            const int64_t len = L.y - L.x;
-            if (len <= RSUM_CHUNK) continue;
-            const int64_t c0 = coff[w], nc = (len + RSUM_CHUNK - 1) / RSUM_CHUNK;
-            double acc = 0.0;  // lane l: chunks l, l + 32, ... in order
-            for (int64_t c = lane_id(); c < nc; c += 32) acc = __dadd_rn(acc, chunk_sum[c0 + c]);
-            const float v = (float)rsum_lane_tree(acc);
-            if (lane_id() == 0) finish(L.z, v);
         }
         t.sync();
+        if (nchunks > 0) {
+            for (int64_t w = team_warp(t); w < nl; w += team_nwarps(t)) {
+                const int4 L = longq[w];
+                const int64_t len = L.y - L.x;
+                if (len <= RSUM_CHUNK) continue;
+                const int64_t c0 = coff[w], nc = (len + RSUM_CHUNK - 1) / RSUM_CHUNK;
+                double acc = 0.0;  // lane l: chunks l, l + 32, ... in order
+                for (int64_t c = lane_id(); c < nc; c += 32) acc = __dadd_rn(acc, chunk_sum[c0 + c]);
+                const float v = (float)rsum_lane_tree(acc);
+                if (lane_id() == 0) finish(L.z, v);
+            }
+            t.sync();
+        }
     }
-    prof_mark(t, sc, PH_CONTRACT_RUNS);
     *bad = uread(&fl[0]);
-    // 4. dims and the smallest cost (every new edge has row < col)
+    const int32_t dmax = uread(&fl[2]);
+    // 3. the edges to their places; dims and the smallest cost (every new
+    //    edge has row < col)
     int32_t mc = -1;
     float mn = 3.4e38f;
-    team_maxi_minf(
-        t, sc, sm, nk, -1, 3.4e38f, [=](int64_t e) { return h.col[e]; }, [=](int64_t e) { return h.cost[e]; }, mc,
-        mn);
-    const int32_t dmax = uread(&fl[2]);
+    if (direct) {
+        for (int64_t k = t.rank(); k < nk; k += t.size()) {
+            mc = max(mc, h.col[k]);
+            mn = fminf(mn, h.cost[k]);
+        }
+    } else {
+        constexpr int U = 4;
+        const int S = blockDim.x;
+        int64_t k = threadIdx.x;
+        auto put = [&](int64_t q, int2 w, float c) {
+            h.row[obase + q] = w.x;
+            h.col[obase + q] = w.y;
+            h.cost[obase + q] = c;
+            mc = max(mc, w.y);
+            mn = fminf(mn, c);
+        };
+        for (; k + (U - 1) * S < kept; k += U * S) {
+            int2 w[U];
+            float c[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                w[q] = tends[first + k + q * S];
+                c[q] = tcost[first + k + q * S];
+            }
+#pragma unroll
+            for (int q = 0; q < U; ++q) put(k + q * S, w[q], c[q]);
+        }
+        for (; k < kept; k += S) put(k, tends[first + k], tcost[first + k]);
+    }
+    team_fold_maxi_minf(t, sc, sm, mc, mn);
+    prof_mark(t, sc, PH_CONTRACT_RUNS);
     h.n = nk;
-    h.rows = uread(&sbk[n - 1]) + 1;
+    h.rows = uread(&R.rec[n - 1].w) + 1;
     h.cols = (mc > dmax ? mc : dmax) + 1;
     h.cmin = nk > 0 ? mn : unknown_cost();
     h.ecols = mc + 1;
     h.uniq = 1;
-    ar.top = top;
+    sc.arena.top = top;
     sc.arena.release(m);
     sc.alg_bytes += 20.0 * (double)n + 12.0 * (double)nk;
     return h;

@@ -11,8 +11,9 @@ namespace rama {
 
 constexpr int THREADS = 512;
 constexpr int SMEM = sort_smem_bytes(THREADS) + 1024;
-static_assert(THREADS / 32 * 1024 + BUCKET_MAX * 12 <= sort_smem_bytes(THREADS),
-              "the CTA bucket sort's staging area fits");
+static_assert(THREADS / 32 * 1024 + BUCKET_MAX * 12 <= sort_smem_bytes(THREADS) &&
+                  record_smem_bytes(THREADS) <= SMEM,
+              "the CTA bucket sort's staging area and the record windows fit");
 // the smaller CTA of k_solve_cta_small (the autotuner chooses between the two
 // for CTA-team solves); its shared memory also holds a CTA bucket sort of
 // BUCKET_MAX items

@@ -217,20 +217,48 @@ __device__ __forceinline__ void block_chunk(const Team &t, int64_t n, int64_t &l
 // team reductions (integer / min / max): one team sync
 // ---------------------------------------------------------------------------
 
+// The CTA's dynamic shared memory keeps no state between primitives, so the
+// results that one warp computes for the whole CTA go through static words,
+// two of them in turn: a thread that runs ahead into the next primitive writes
+// the other one, and passes a barrier before it comes back to the first.
+
 // Combines the per-CTA partials part[0, nb) written before the last team
-// sync.  Every warp reads them with independent L2 loads (ld.global.cg: the
-// values come from other SMs, so L1 must not serve them) spread over its
-// lanes, then combines the lanes; the result is valid on every lane.  Only
+// sync: a warp reads them with independent L2 loads (ld.global.cg: the values
+// come from other SMs, so L1 must not serve them) spread over its lanes, in
+// batches, then combines the lanes; the result is valid on every lane.  Only
 // for exact operations (integer sums, min, max), whose result does not depend
 // on the combination order.
 template <class T, class Op>
 __device__ __forceinline__ T warp_fold_parts(const T *part, int nb, T init, Op op)
 {
     T r = init;
-    for (int b = lane_id(); b < nb; b += 32) r = op(r, __ldcg(part + b));
+    constexpr int U = 5;
+    for (int b = lane_id(); b < nb; b += 32 * U) {
+        T v[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) v[k] = __ldcg(part + min(b + 32 * k, nb - 1));
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+            if (b + 32 * k < nb) r = op(r, v[k]);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) r = op(r, __shfl_xor_sync(FULL, r, o));
     return r;
+}
+
+// The same for the whole CTA.  With every warp reading all partials, a grid of
+// 296 CTAs moved 11 MB from L2 per reduction; here one warp reads them and the
+// others wait for it.
+template <class Team, class T, class Op>
+__device__ __forceinline__ T cta_fold_parts(const Team &t, Scratch &sc, const T *part, T init, Op op)
+{
+    __shared__ T res[2];
+    if (warp_in_block() == 0) {
+        const T r = warp_fold_parts<T>(part, t.nblocks(), init, op);
+        if (lane_id() == 0) res[sc.parity] = r;
+    }
+    __syncthreads();
+    return res[sc.parity];
 }
 
 // Grid-stride loop over [0, n) in batches of U strides: load(i) for every
@@ -258,10 +286,11 @@ template <class Team, class T>
 __device__ T team_total(const Team &t, Scratch &sc, char *sm, T v)
 {
     const T s = block_sum<T>(v, reinterpret_cast<T *>(sm));
+    if (t.nblocks() == 1) return s;  // the block's total, behind the block's barriers
     T *part = reinterpret_cast<T *>(sc.next_part());
     if (threadIdx.x == 0) part[t.block()] = s;
     t.sync();
-    return warp_fold_parts<T>(part, t.nblocks(), T(0), [](T a, T b) { return a + b; });
+    return cta_fold_parts<Team, T>(t, sc, part, T(0), [](T a, T b) { return a + b; });
 }
 
 template <class Team, class T, class Get>
@@ -283,10 +312,11 @@ __device__ T team_sum(const Team &t, Scratch &sc, char *sm, int64_t n, Get get)
         for (; i < n; i += S) s += get(i);
     }
     s = block_sum<T>(s, reinterpret_cast<T *>(sm));
+    if (t.nblocks() == 1) return s;  // the block's total, behind the block's barriers
     T *part = reinterpret_cast<T *>(sc.next_part());
     if (threadIdx.x == 0) part[t.block()] = s;
     t.sync();
-    return warp_fold_parts<T>(part, t.nblocks(), T(0), [](T a, T b) { return a + b; });
+    return cta_fold_parts<Team, T>(t, sc, part, T(0), [](T a, T b) { return a + b; });
 }
 
 template <class Team, class T, class Get>
@@ -310,10 +340,11 @@ __device__ T team_max(const Team &t, Scratch &sc, char *sm, int64_t n, T init, G
         }
     }
     s = block_max<T>(s, reinterpret_cast<T *>(sm));
+    if (t.nblocks() == 1) return s;  // the block's total, behind the block's barriers
     T *part = reinterpret_cast<T *>(sc.next_part());
     if (threadIdx.x == 0) part[t.block()] = s;
     t.sync();
-    return warp_fold_parts<T>(part, t.nblocks(), init, [](T a, T b) { return b > a ? b : a; });
+    return cta_fold_parts<Team, T>(t, sc, part, init, [](T a, T b) { return b > a ? b : a; });
 }
 
 template <class Team, class T, class Get>
@@ -325,10 +356,74 @@ __device__ T team_min(const Team &t, Scratch &sc, char *sm, int64_t n, T init, G
         s = x < s ? x : s;
     }
     s = block_min<T>(s, reinterpret_cast<T *>(sm));
+    if (t.nblocks() == 1) return s;  // the block's total, behind the block's barriers
     T *part = reinterpret_cast<T *>(sc.next_part());
     if (threadIdx.x == 0) part[t.block()] = s;
     t.sync();
-    return warp_fold_parts<T>(part, t.nblocks(), init, [](T a, T b) { return b < a ? b : a; });
+    return cta_fold_parts<Team, T>(t, sc, part, init, [](T a, T b) { return b < a ? b : a; });
+}
+
+// The maximum of a and the minimum of b over the team's threads, on every
+// thread; one team sync.
+template <class Team>
+__device__ void team_fold_maxi_minf(const Team &t, Scratch &sc, char *sm, int32_t &a, float &b)
+{
+    auto lanes = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const int32_t x = __shfl_xor_sync(FULL, a, o);
+            const float y = __shfl_xor_sync(FULL, b, o);
+            a = x > a ? x : a;
+            b = y < b ? y : b;
+        }
+    };
+    __shared__ int32_t ra[2];
+    __shared__ float rb[2];
+    lanes();
+    int32_t *sa = reinterpret_cast<int32_t *>(sm);
+    float *sb = reinterpret_cast<float *>(sm + 128);
+    if (lane_id() == 0) {
+        sa[warp_in_block()] = a;
+        sb[warp_in_block()] = b;
+    }
+    __syncthreads();
+    a = sa[0];
+    b = sb[0];
+    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
+        a = sa[k] > a ? sa[k] : a;
+        b = sb[k] < b ? sb[k] : b;
+    }
+    __syncthreads();
+    if (t.nblocks() == 1) return;
+    int32_t *part = reinterpret_cast<int32_t *>(sc.next_part());
+    if (threadIdx.x == 0) {
+        part[2 * t.block()] = a;
+        part[2 * t.block() + 1] = __float_as_int(b);
+    }
+    t.sync();
+    if (warp_in_block() == 0) {
+        constexpr int U = 5;
+        const int nb = t.nblocks();
+        const int2 *p = reinterpret_cast<const int2 *>(part);
+        for (int k = lane_id(); k < nb; k += 32 * U) {
+            int2 v[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) v[q] = __ldcg(p + min(k + 32 * q, nb - 1));
+#pragma unroll
+            for (int q = 0; q < U; ++q) {  // (a partial read twice changes nothing)
+                a = v[q].x > a ? v[q].x : a;
+                b = __int_as_float(v[q].y) < b ? __int_as_float(v[q].y) : b;
+            }
+        }
+        lanes();
+        if (lane_id() == 0) {
+            ra[sc.parity] = a;
+            rb[sc.parity] = b;
+        }
+    }
+    __syncthreads();
+    a = ra[sc.parity];
+    b = rb[sc.parity];
 }
 
 // The maximum of ia(i) and the minimum of fb(i) over [0, n) in one pass and
@@ -364,50 +459,40 @@ __device__ void team_maxi_minf(const Team &t, Scratch &sc, char *sm, int64_t n, 
             b = y < b ? y : b;
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const int32_t x = __shfl_xor_sync(FULL, a, o);
-        const float y = __shfl_xor_sync(FULL, b, o);
-        a = x > a ? x : a;
-        b = y < b ? y : b;
-    }
-    int32_t *sa = reinterpret_cast<int32_t *>(sm);
-    float *sb = reinterpret_cast<float *>(sm + 128);
-    if (lane_id() == 0) {
-        sa[warp_in_block()] = a;
-        sb[warp_in_block()] = b;
-    }
-    __syncthreads();
-    a = sa[0];
-    b = sb[0];
-    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) {
-        a = sa[k] > a ? sa[k] : a;
-        b = sb[k] < b ? sb[k] : b;
-    }
-    __syncthreads();
-    int32_t *part = reinterpret_cast<int32_t *>(sc.next_part());  // 16 B per block
-    if (threadIdx.x == 0) {
-        part[2 * t.block()] = a;
-        part[2 * t.block() + 1] = __float_as_int(b);
-    }
-    t.sync();
-    a = iinit;
-    b = finit;
-    for (int k = lane_id(); k < t.nblocks(); k += 32) {
-        const int32_t x = __ldcg(part + 2 * k);
-        const float y = __int_as_float(__ldcg(part + 2 * k + 1));
-        a = x > a ? x : a;
-        b = y < b ? y : b;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const int32_t x = __shfl_xor_sync(FULL, a, o);
-        const float y = __shfl_xor_sync(FULL, b, o);
-        a = x > a ? x : a;
-        b = y < b ? y : b;
-    }
+    team_fold_maxi_minf(t, sc, sm, a, b);
     imax = a;
     fmin = b;
+}
+
+// The sum of the partials of the CTAs before this one, and of all.
+template <class Team, class T>
+__device__ __forceinline__ void cta_prefix_parts(const Team &t, Scratch &sc, const T *part, T &base, T &total)
+{
+    __shared__ T res[2][2];
+    if (warp_in_block() == 0) {
+        T b = T(0), a = T(0);
+        constexpr int U = 5;
+        const int nb = t.nblocks();
+        for (int x = lane_id(); x < nb; x += 32 * U) {
+            T v[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) v[k] = __ldcg(part + min(x + 32 * k, nb - 1));
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                if (x + 32 * k < nb) a += v[k];
+                if (x + 32 * k < t.block()) b += v[k];
+            }
+        }
+        b = warp_sum(b);
+        a = warp_sum(a);
+        if (lane_id() == 0) {
+            res[sc.parity][0] = b;
+            res[sc.parity][1] = a;
+        }
+    }
+    __syncthreads();
+    base = res[sc.parity][0];
+    total = res[sc.parity][1];
 }
 
 // ---------------------------------------------------------------------------
@@ -450,17 +535,13 @@ __device__ T team_scan_while(const Team &t, Scratch &sc, char *sm, int64_t n, In
         for (; i < hi; i += S) s += in(i);
     }
     s = block_sum<T>(s, tsm);
-    T *part = reinterpret_cast<T *>(sc.next_part());
-    if (threadIdx.x == 0) part[t.block()] = s;
-    t.sync();
-    T base = T(0), total = T(0);
-    for (int b = lane_id(); b < t.nblocks(); b += 32) {
-        T x = __ldcg(part + b);
-        if (b < t.block()) base += x;
-        total += x;
+    T base = T(0), total = s;
+    if (t.nblocks() > 1) {
+        T *part = reinterpret_cast<T *>(sc.next_part());
+        if (threadIdx.x == 0) part[t.block()] = s;
+        t.sync();
+        cta_prefix_parts(t, sc, part, base, total);
     }
-    base = warp_sum(base);
-    total = warp_sum(total);
     if (!go_on(total)) return total;
     const int64_t TILE = (int64_t)blockDim.x * ITEMS;
     const int64_t wseg = (int64_t)warp_in_block() * 32 * ITEMS;
@@ -553,7 +634,7 @@ __device__ __noinline__ csum2_t team_csum_fold(const Team &t, Scratch &sc, csum_
 {
     __shared__ csum_t wa[32], wb[32];
     __shared__ float wm[32];
-    __shared__ csum2_t res;
+    __shared__ csum2_t res[2];
     // merging is commutative, so a butterfly leaves the same pair on every lane
     auto fold = [&](int lanes) {
         for (int off = 1; off < lanes; off <<= 1) {
@@ -583,9 +664,9 @@ __device__ __noinline__ csum2_t team_csum_fold(const Team &t, Scratch &sc, csum_
         fold(nw);
         if (lane_id() == 0) {
             if (t.nblocks() == 1) {
-                res.a = __dadd_rn(a.s, a.c);
-                res.b = __dadd_rn(b.s, b.c);
-                res.m = m;
+                res[sc.parity].a = __dadd_rn(a.s, a.c);
+                res[sc.parity].b = __dadd_rn(b.s, b.c);
+                res[sc.parity].m = m;
             } else {
                 part[3 * t.block()] = a;
                 part[3 * t.block() + 1] = b;
@@ -598,24 +679,36 @@ __device__ __noinline__ csum2_t team_csum_fold(const Team &t, Scratch &sc, csum_
         if (warp_in_block() == 0) {
             a = b = csum_t{0.0, 0.0};
             const double2 *p = reinterpret_cast<const double2 *>(part);
-            for (int k = lane_id(); k < t.nblocks(); k += 32) {
-                const double2 x = __ldcg(p + 3 * k), y = __ldcg(p + 3 * k + 1);
-                const double z = __ldcg(reinterpret_cast<const double *>(p + 3 * k + 2));
-                a = cs_merge(a, csum_t{x.x, x.y});
-                b = cs_merge(b, csum_t{y.x, y.y});
-                m = fminf(m, (float)z);
+            constexpr int U = 5;
+            const int nb = t.nblocks();
+            for (int k = lane_id(); k < nb; k += 32 * U) {
+                double2 x[U], y[U];
+                double z[U];
+#pragma unroll
+                for (int q = 0; q < U; ++q) {
+                    const int c = min(k + 32 * q, nb - 1);
+                    x[q] = __ldcg(p + 3 * c);
+                    y[q] = __ldcg(p + 3 * c + 1);
+                    z[q] = __ldcg(reinterpret_cast<const double *>(p + 3 * c + 2));
+                }
+#pragma unroll
+                for (int q = 0; q < U; ++q)
+                    if (k + 32 * q < nb) {
+                        a = cs_merge(a, csum_t{x[q].x, x[q].y});
+                        b = cs_merge(b, csum_t{y[q].x, y[q].y});
+                        m = fminf(m, (float)z[q]);
+                    }
             }
             fold(32);
             if (lane_id() == 0) {
-                res.a = __dadd_rn(a.s, a.c);
-                res.b = __dadd_rn(b.s, b.c);
-                res.m = m;
+                res[sc.parity].a = __dadd_rn(a.s, a.c);
+                res[sc.parity].b = __dadd_rn(b.s, b.c);
+                res[sc.parity].m = m;
             }
         }
         __syncthreads();
     }
-    // the next fold writes `res` after a sync that follows this read
-    return res;
+    return res[sc.parity];
 }
 
 // The sum of get(k) over [0, n) on every thread; *count receives the number
@@ -655,6 +748,29 @@ __device__ double team_csum(const Team &t, Scratch &sc, int64_t n, Get get)
 {
     int64_t unused = 0;
     return team_csum_count(t, sc, n, get, [](int64_t) { return false; }, &unused);
+}
+
+// RSUM of n <= 64 values v(k), k in [0, n), by one thread: the loads of a
+// group of 8 together, then the tree over the 32 lanes (a lane holds values l
+// and l + 32) as the pairwise sum of four trees over 8; +0.0 in the empty
+// lanes changes no sum.
+template <class Get>
+__device__ __forceinline__ float rsum_upto64(int n, Get v)
+{
+    auto group = [&](int q) {
+        double x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] = 8 * q + k < n ? __dadd_rn(0.0, (double)v(8 * q + k)) : 0.0;
+        if (n > 32) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (8 * q + k + 32 < n) x[k] = __dadd_rn(x[k], (double)v(8 * q + k + 32));
+        }
+        return __dadd_rn(__dadd_rn(__dadd_rn(x[0], x[1]), __dadd_rn(x[2], x[3])),
+                         __dadd_rn(__dadd_rn(x[4], x[5]), __dadd_rn(x[6], x[7])));
+    };
+    if (n <= 8) return (float)group(0);
+    return (float)__dadd_rn(__dadd_rn(group(0), group(1)), __dadd_rn(group(2), group(3)));
 }
 
 // RSUM over values v(k), k in [0,n) by ONE thread (n <= 32): the oracle's

@@ -61,22 +61,39 @@ __device__ __forceinline__ void for_common(const int32_t *adj, int32_t a0, int32
 // meet, and blocks meet in ascending order.  hit(mask, base) gets the matches
 // of one pair of blocks as bits over the first list's block at `base` and
 // returns whether to go on.
+//
+// A list's blocks start at the 16-byte boundary at or before its first entry
+// (adj is 256-byte aligned and padded to 256 bytes) and are read
+// by 128-bit loads; what lies outside the list is replaced by values that
+// match nothing.  The lanes of a warp read different lists, so a load
+// instruction costs a line per lane whatever its width.
 constexpr int CB = 8;
 
+__device__ __forceinline__ void list_block(const int32_t *adj, int32_t p, int32_t s, int32_t e, int32_t below,
+                                           int32_t above, int32_t (&v)[CB])
+{
+    const int4 x = *reinterpret_cast<const int4 *>(adj + p);
+    int4 y = make_int4(above, above, above, above);
+    if (p + 4 < e) y = *reinterpret_cast<const int4 *>(adj + p + 4);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+    v[4] = y.x, v[5] = y.y, v[6] = y.z, v[7] = y.w;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        if (p + k < s) v[k] = below;
+#pragma unroll
+    for (int k = 0; k < CB; ++k)
+        if (p + k >= e) v[k] = above;
+}
+
 template <class Hit>
-__device__ __forceinline__ void common_blocks(const int32_t *adj, int32_t a0, int32_t a1, int32_t b0, int32_t b1,
+__device__ __forceinline__ void common_blocks(const int32_t *adj, int32_t as, int32_t a1, int32_t bs, int32_t b1,
                                               Hit hit)
 {
-    if (a0 >= a1 || b0 >= b1) return;
+    if (as >= a1 || bs >= b1) return;
     int32_t a[CB], b[CB];
-    auto load = [=](int32_t (&v)[CB], int32_t p, int32_t e, int32_t pad) {
-#pragma unroll
-        for (int k = 0; k < CB; ++k) v[k] = adj[min(p + k, e - 1)];
-#pragma unroll
-        for (int k = 0; k < CB; ++k) v[k] = p + k < e ? v[k] : pad;
-    };
-    load(a, a0, a1, 0x7fffffff);
-    load(b, b0, b1, 0x7ffffffe);
+    int32_t a0 = as & ~3, b0 = bs & ~3;
+    list_block(adj, a0, as, a1, -1, 0x7fffffff, a);
+    list_block(adj, b0, bs, b1, -2, 0x7ffffffe, b);
     for (;;) {
         unsigned m = 0;
 #pragma unroll
@@ -93,12 +110,12 @@ __device__ __forceinline__ void common_blocks(const int32_t *adj, int32_t a0, in
         if (la <= lb) {
             a0 += CB;
             if (a0 >= a1) return;
-            load(a, a0, a1, 0x7fffffff);
+            list_block(adj, a0, as, a1, -1, 0x7fffffff, a);
         }
         if (lb <= la) {
             b0 += CB;
             if (b0 >= b1) return;
-            load(b, b0, b1, 0x7ffffffe);
+            list_block(adj, b0, bs, b1, -2, 0x7ffffffe, b);
         }
     }
 }
@@ -143,9 +160,13 @@ __device__ __forceinline__ void write_tri(const TriBuf &tb, int64_t pos, int32_t
 
 // Remove degenerate triangles, sort lexicographically, unique (the first n
 // entries of the buffer); returns the new count.  By buckets of the smallest
-// vertex, degenerate triangles in none; the rest of each triangle is its key
-// in the bucket.  With tb.distinct the sorted triangles go to new arrays that
-// take the buffer's place; otherwise a scan drops repetitions on the way back.
+// vertex, degenerate triangles in none: a triangle travels as a record (middle
+// vertex, largest vertex, -, smallest vertex) and the tile pass orders the
+// buckets in shared memory and writes the triangles in order.  (With every
+// triangle ranked against its bucket in global memory and written to its place
+// from there, the triangles of the 1M-point k-NN graph in D mode took 24.4 ms.)
+// With tb.distinct the sorted triangles go to new arrays that take the
+// buffer's place; otherwise a scan drops repetitions on the way back.
 template <class Team>
 __device__ __noinline__ int64_t tri_normalize(const Team &t, Scratch &sc, char *, TriBuf &tb, int64_t n, int32_t nmax)
 {
@@ -159,11 +180,15 @@ __device__ __noinline__ int64_t tri_normalize(const Team &t, Scratch &sc, char *
             *o3 = sc.arena.take<int32_t>(n + 1);
     const uint64_t m1 = sc.arena.mark();
     const int32_t nbk = nmax + 1;
-    int32_t *start = sc.arena.take<int32_t>((int64_t)nbk + 1);
-    int32_t *slot = sc.arena.take<int32_t>(n + 1);
-    uint64_t *tk = sc.arena.take<uint64_t>(n + 1);
+    Records R;
+    R.rec = sc.arena.take<int4>(n + 1);
+    R.start = sc.arena.take<int32_t>((int64_t)nbk + 1);
+    R.slot = sc.arena.take<int32_t>(n + 1);
+    R.lohi = nullptr;
     BucketLists L = bucket_lists(sc, n);
     if (!sc.arena.ok()) return 0;
+    int4 *rec = R.rec;
+    int32_t *start = R.start, *slot = R.slot;
     const uint64_t mask = (nb == 0) ? 0 : ((uint64_t(1) << nb) - 1);
     struct Tri {
         int32_t lo, md, hi;
@@ -180,15 +205,23 @@ __device__ __noinline__ int64_t tri_normalize(const Team &t, Scratch &sc, char *
     for (int64_t v = t.rank(); v <= nbk; v += t.size()) start[v] = 0;
     if (t.rank() < 4) L.n[t.rank()] = 0;
     t.sync();
-    for (int64_t k0 = (int64_t)t.rank() - lane_id(); k0 < n; k0 += t.size()) {
-        const int64_t k = k0 + lane_id();
-        int32_t b = -1;
-        if (k < n) {
-            const Tri r = tri(k);
-            if (r.ok()) b = r.lo;
+    {
+        constexpr int U = SORT_BATCH;
+        const int64_t S = t.size();
+        for (int64_t base = (int64_t)t.rank() - lane_id(); base < n; base += S * U) {
+            int32_t b[U], s[U];
+#pragma unroll
+            for (int k = 0; k < U; ++k) {
+                const int64_t q = base + k * S + lane_id();
+                const Tri r = tri(q < n ? q : n - 1);
+                b[k] = q < n && r.ok() ? r.lo : -1;
+            }
+#pragma unroll
+            for (int k = 0; k < U; ++k) s[k] = base + k * S < n ? bucket_slot(start, b[k]) : 0;
+#pragma unroll
+            for (int k = 0; k < U; ++k)
+                if (base + k * S + lane_id() < n) slot[base + k * S + lane_id()] = s[k];
         }
-        const int32_t s = bucket_slot(start, b);
-        if (k < n) slot[k] = s;
     }
     t.sync();
     const int64_t w = team_bucket_starts(t, sc, sm, nbk, start, L, [](int64_t, int32_t, int32_t) {});
@@ -197,34 +230,31 @@ __device__ __noinline__ int64_t tri_normalize(const Team &t, Scratch &sc, char *
             t, n,
             [=](int64_t k) {
                 const Tri r = tri(k);
-                return make_int4(r.ok() ? start[r.lo] + slot[k] : -1, r.md, r.hi, 0);
+                return make_int4(r.md, r.hi, r.ok() ? start[r.lo] + slot[k] : -1, r.lo);
             },
             [=](int64_t, int4 v) {
-                if (v.x >= 0) tk[v.x] = pack_key(v.y, v.z, nb);
+                if (v.z >= 0) rec[v.z] = v;
             });
         t.sync();
-        for (int64_t k = t.rank(); k < n; k += t.size()) {
-            const Tri r = tri(k);
-            if (!r.ok()) continue;
-            const int32_t s = start[r.lo], e = start[r.lo + 1];
-            if (e - s > BUCKET_SMALL) continue;
-            const int32_t p = s + bucket_rank(tk, s, e, pack_key(r.md, r.hi, nb), s + slot[k]);
-            o1[p] = r.lo;
-            o2[p] = r.md;
-            o3[p] = r.hi;
-        }
-        if (L.has_long())
-            team_sort_long_buckets(t, sm, L, start, tk, [=](int32_t b, int32_t p, uint64_t key) {
-                o1[p] = b;
-                o2[p] = (int32_t)(key >> nb);
-                o3[p] = (int32_t)(key & mask);
-            });
+        team_sort_long_records(t, sm, R, L);
+        team_record_tiles<true>(t, sm, R, w,
+                                [&](const RecTile &T, int base, const int4 (&)[4], const bool (&mine)[4]) {
+#pragma unroll
+                                    for (int k = 0; k < 4; ++k)
+                                        if (mine[k]) {
+                                            const int4 r = T.win[base + 32 * k];
+                                            const int64_t p = T.p0 + base + 32 * k;
+                                            o1[p] = r.w;
+                                            o2[p] = r.x;
+                                            o3[p] = r.y;
+                                        }
+                                });
         t.sync();
     } else {
         // a vertex with more than BUCKET_MAX triangles: LSD radix, stable sort
         // by hi carrying (lo, md), then by (lo, md) carrying hi
         uint64_t *k1 = sc.arena.take<uint64_t>(n + 1), *k2 = sc.arena.take<uint64_t>(n + 1);
-        uint64_t *u1 = sc.arena.take<uint64_t>(n + 1), *u2 = tk;
+        uint64_t *u1 = reinterpret_cast<uint64_t *>(rec), *u2 = u1 + (n + 1);  // (the records are not used here)
         if (!sc.arena.ok()) return 0;
         team_compact(
             t, sc, sm, n, [=](int64_t k) { return tri(k).ok(); },
@@ -616,9 +646,13 @@ __device__ __noinline__ void conflicted_cycles(const Team &t, Scratch &sc, char 
     // one pass counts both: the low 32 bits count every repulsive edge (the
     // budget counts them all, :247), the high bits the kept ones; the kept
     // ones are compacted only when there are any
+    // (the loads of several edges in flight together: none is skipped, an edge
+    // that is not repulsive looks at vertex 0)
     auto rep_code = [=](int64_t e) -> int64_t {
-        if (!(A.cost[e] < thresh)) return 0;
-        return (haspos[A.row[e]] && haspos[A.col[e]]) ? (int64_t(1) << 32) + 1 : 1;
+        const bool rep = A.cost[e] < thresh;
+        const int32_t r = A.row[e], c = A.col[e];
+        const int8_t a = haspos[rep ? r : 0], b = haspos[rep ? c : 0];
+        return rep ? ((a & b) != 0 ? (int64_t(1) << 32) + 1 : 1) : 0;
     };
     const int64_t packed = team_scan_while<Team, int64_t>(
         t, sc, sm, A.n, rep_code, [](int64_t total) { return (total >> 32) != 0; },

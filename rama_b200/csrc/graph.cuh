@@ -130,6 +130,57 @@ struct Records {
 
 __device__ __forceinline__ uint64_t rec_key(const int4 &r) { return ((uint64_t)(uint32_t)r.x << 32) | (uint32_t)r.y; }
 
+// Orders the listed buckets of records where they lie: 65..256 records by a
+// warp, up to BUCKET_MAX by a CTA.  Ends in a team sync if there are any.
+template <class Team>
+__device__ __forceinline__ void team_sort_long_records(const Team &t, char *sm, const Records &R, BucketLists L)
+{
+    if (!L.has_long()) return;
+    const int NW = blockDim.x >> 5;
+    {
+        uint64_t *wk = reinterpret_cast<uint64_t *>(sm) + warp_in_block() * 256;
+        int32_t *wi = reinterpret_cast<int32_t *>(sm + NW * 256 * 8) + warp_in_block() * 256;
+        const int32_t nw = uread(&L.n[0]);
+        for (int64_t q = team_warp(t); q < nw; q += team_nwarps(t)) {
+            const int32_t b = L.warp[q], s = R.start[b], m = R.start[b + 1] - s;
+            int P = 128;
+            while (P < m) P <<= 1;
+            for (int x = lane_id(); x < m; x += 32) {
+                const int4 r = R.rec[s + x];
+                wk[x] = rec_key(r);
+                wi[x] = r.z;
+            }
+            __syncwarp();
+            smem_bitonic(wk, wi, m, P, lane_id(), 32, [] { __syncwarp(); });
+            for (int x = lane_id(); x < m; x += 32)
+                R.rec[s + x] = make_int4((int32_t)(wk[x] >> 32), (int32_t)(uint32_t)wk[x], wi[x], b);
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    {
+        uint64_t *ck = reinterpret_cast<uint64_t *>(sm);
+        int32_t *ci = reinterpret_cast<int32_t *>(sm + BUCKET_MAX * 8);
+        const int32_t nc = uread(&L.n[1]);
+        for (int64_t q = t.block(); q < nc; q += t.nblocks()) {
+            const int32_t b = L.cta[q], s = R.start[b], m = R.start[b + 1] - s;
+            int P = 512;
+            while (P < m) P <<= 1;
+            for (int x = threadIdx.x; x < m; x += blockDim.x) {
+                const int4 r = R.rec[s + x];
+                ck[x] = rec_key(r);
+                ci[x] = r.z;
+            }
+            __syncthreads();
+            smem_bitonic(ck, ci, m, P, threadIdx.x, blockDim.x, [] { __syncthreads(); });
+            for (int x = threadIdx.x; x < m; x += blockDim.x)
+                R.rec[s + x] = make_int4((int32_t)(ck[x] >> 32), (int32_t)(uint32_t)ck[x], ci[x], b);
+            __syncthreads();
+        }
+    }
+    t.sync();
+}
+
 // ends(e): (lo, hi) of edge e, loads only; nbh: bits of a node id
 template <class Team, class Ends>
 __device__ __forceinline__ bool team_sort_records(const Team &t, Scratch &sc, char *sm, int64_t n, int32_t nbk,
@@ -195,52 +246,7 @@ __device__ __forceinline__ bool team_sort_records(const Team &t, Scratch &sc, ch
         [=](int64_t, Item x) { rec[x.p] = x.r; });
     t.sync();
     prof_mark(t, sc, PH_CSORT_SCATTER);
-    if (L.has_long()) {
-        // 65..256 records: a warp; up to BUCKET_MAX: a CTA
-        const int NW = blockDim.x >> 5;
-        {
-            uint64_t *wk = reinterpret_cast<uint64_t *>(sm) + warp_in_block() * 256;
-            int32_t *wi = reinterpret_cast<int32_t *>(sm + NW * 256 * 8) + warp_in_block() * 256;
-            const int32_t nw = uread(&L.n[0]);
-            for (int64_t q = team_warp(t); q < nw; q += team_nwarps(t)) {
-                const int32_t b = L.warp[q], s = start[b], m = start[b + 1] - s;
-                int P = 128;
-                while (P < m) P <<= 1;
-                for (int x = lane_id(); x < m; x += 32) {
-                    const int4 r = rec[s + x];
-                    wk[x] = rec_key(r);
-                    wi[x] = r.z;
-                }
-                __syncwarp();
-                smem_bitonic(wk, wi, m, P, lane_id(), 32, [] { __syncwarp(); });
-                for (int x = lane_id(); x < m; x += 32)
-                    rec[s + x] = make_int4((int32_t)(wk[x] >> 32), (int32_t)(uint32_t)wk[x], wi[x], b);
-                __syncwarp();
-            }
-        }
-        __syncthreads();
-        {
-            uint64_t *ck = reinterpret_cast<uint64_t *>(sm);
-            int32_t *ci = reinterpret_cast<int32_t *>(sm + BUCKET_MAX * 8);
-            const int32_t nc = uread(&L.n[1]);
-            for (int64_t q = t.block(); q < nc; q += t.nblocks()) {
-                const int32_t b = L.cta[q], s = start[b], m = start[b + 1] - s;
-                int P = 512;
-                while (P < m) P <<= 1;
-                for (int x = threadIdx.x; x < m; x += blockDim.x) {
-                    const int4 r = rec[s + x];
-                    ck[x] = rec_key(r);
-                    ci[x] = r.z;
-                }
-                __syncthreads();
-                smem_bitonic(ck, ci, m, P, threadIdx.x, blockDim.x, [] { __syncthreads(); });
-                for (int x = threadIdx.x; x < m; x += blockDim.x)
-                    rec[s + x] = make_int4((int32_t)(ck[x] >> 32), (int32_t)(uint32_t)ck[x], ci[x], b);
-                __syncthreads();
-            }
-        }
-        t.sync();
-    }
+    team_sort_long_records(t, sm, R, L);
     prof_mark(t, sc, PH_CSORT_RANK);
     if (L.has_big()) {
         // the buckets beyond BUCKET_MAX: their edges in input order, a stable
@@ -306,7 +312,9 @@ __device__ __forceinline__ int64_t rec_owned_from(const Records &R, int64_t p, i
     return e - s > BUCKET_SMALL || s == p ? p : e;
 }
 
-template <class Team, class Visit>
+//
+// TIES: records of a bucket may have equal keys (they keep their order).
+template <bool TIES = false, class Team, class Visit>
 __device__ __forceinline__ void team_record_tiles(const Team &t, char *sm, const Records &R, int64_t n, Visit visit)
 {
     constexpr int K = 4;
@@ -347,7 +355,10 @@ __device__ __forceinline__ void team_record_tiles(const Team &t, char *sm, const
                 const uint64_t key = rec_key(r[k]);
                 const int f = (int)(s[k] - p0), l = (int)(e[k] - p0);
                 int rank = 0;
-                for (int x = f; x < l; ++x) rank += rec_key(win[x]) < key;
+                for (int x = f; x < l; ++x) {
+                    const uint64_t o = rec_key(win[x]);
+                    rank += o < key || (TIES && o == key && x < i);
+                }
                 dst[k] = f + rank;
             }
         }

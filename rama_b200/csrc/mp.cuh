@@ -44,27 +44,28 @@ __device__ __forceinline__ int64_t find_edge(const int32_t *off, const int32_t *
     return (lo < off[a + 1] && col[lo] == b) ? lo : -1;
 }
 
-// find_edge of three (a, b) pairs at once: the three binary searches step in
-// lockstep, so each step's loads are in flight together
-__device__ __forceinline__ void find_edges3(const int32_t *off, const int32_t *col, const int32_t (&a)[3],
-                                           const int32_t (&b)[3], int32_t (&out)[3])
+// find_edge of N (a, b) pairs at once: the binary searches step in lockstep,
+// so each step's loads are in flight together
+template <int N>
+__device__ __forceinline__ void find_edges(const int32_t *off, const int32_t *col, const int32_t (&a)[N],
+                                           const int32_t (&b)[N], int32_t (&out)[N])
 {
-    int32_t lo[3], hi[3], end[3];
+    int32_t lo[N], hi[N], end[N];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
+    for (int k = 0; k < N; ++k) {
         lo[k] = off[a[k]];
         hi[k] = end[k] = off[a[k] + 1];
     }
     for (int step = 0; step < 32; ++step) {
-        int32_t m[3], c[3];
+        int32_t m[N], c[N];
         bool any = false;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
+        for (int k = 0; k < N; ++k) {
             m[k] = (lo[k] + hi[k]) >> 1;
             c[k] = lo[k] < hi[k] ? col[m[k]] : 0;
         }
 #pragma unroll
-        for (int k = 0; k < 3; ++k)
+        for (int k = 0; k < N; ++k)
             if (lo[k] < hi[k]) {
                 any = true;
                 if (c[k] < b[k])
@@ -74,11 +75,11 @@ __device__ __forceinline__ void find_edges3(const int32_t *off, const int32_t *c
             }
         if (!any) break;
     }
-    int32_t c[3];
+    int32_t c[N];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) c[k] = lo[k] < end[k] ? col[lo[k]] : 0;
+    for (int k = 0; k < N; ++k) c[k] = lo[k] < end[k] ? col[lo[k]] : 0;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) out[k] = (lo[k] < end[k] && c[k] == b[k]) ? lo[k] : -1;
+    for (int k = 0; k < N; ++k) out[k] = (lo[k] < end[k] && c[k] == b[k]) ? lo[k] : -1;
 }
 
 // number of entries of row a with col < b, plus all rows < a
@@ -151,10 +152,34 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
     }
     if (t.rank() < 4) L.n[t.rank()] = 0;
     team_offsets(t, A.n, nmax, [=](int64_t e) { return A.row[e]; }, aoff);
-    // the triangles' sides in a (row, col)-sorted list; `each` gets the three
-    // positions (-1: not an edge) with all lanes of the warp present
-    auto lookup = [=](const int32_t *off, const int32_t *col, auto each) {
-        for (int64_t k0 = (int64_t)t.rank() - lane_id(); k0 < T; k0 += t.size()) {
+    // the triangles' sides among the graph's edges; `each` gets the three
+    // positions (-1: not an edge) with all lanes of the warp present.  Two
+    // triangles a lane at a time where there are that many.
+    auto lookup = [=](auto each) {
+        const int64_t S = t.size();
+        int64_t k0 = (int64_t)t.rank() - lane_id();
+        for (; k0 + S + 31 < T; k0 += 2 * S) {
+            const int64_t k[2] = {k0 + lane_id(), k0 + S + lane_id()};
+            int32_t f[6], from[6], to[6];
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int32_t a = mp.t1[k[q]], b = mp.t2[k[q]], c = mp.t3[k[q]];
+                from[3 * q] = from[3 * q + 1] = a;
+                from[3 * q + 2] = to[3 * q] = b;
+                to[3 * q + 1] = to[3 * q + 2] = c;
+            }
+            find_edges<6>(aoff, A.col, from, to, f);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int32_t g[3] = {f[3 * q], f[3 * q + 1], f[3 * q + 2]};
+                mp.e12[k[q]] = g[0];
+                mp.e13[k[q]] = g[1];
+                mp.e23[k[q]] = g[2];
+                const int32_t h[3] = {from[3 * q], from[3 * q + 1], from[3 * q + 2]};
+                each(k[q], true, h, g);
+            }
+        }
+        for (; k0 < T; k0 += S) {
             const int64_t k = k0 + lane_id();
             int32_t f[3] = {-1, -1, -1}, from[3] = {0, 0, 0};
             if (k < T) {
@@ -162,7 +187,7 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
                 const int32_t to[3] = {b, c, c};
                 from[0] = from[1] = a;
                 from[2] = b;
-                find_edges3(off, col, from, to, f);
+                find_edges<3>(aoff, A.col, from, to, f);
                 mp.e12[k] = f[0];
                 mp.e13[k] = f[1];
                 mp.e23[k] = f[2];
@@ -184,13 +209,13 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
     int64_t nn = 0;
     if (closed) {
         int32_t *inc = mp.inc_off;
-        lookup(aoff, A.col, [=](int64_t k, bool valid, const int32_t (&)[3], const int32_t (&f)[3]) {
+        lookup([=](int64_t k, bool valid, const int32_t (&)[3], const int32_t (&f)[3]) {
             count_sides(k, valid, f, inc);
         });
         t.sync();
     } else {
         // chords: sides that are no edges, by their row
-        lookup(aoff, A.col, [=](int64_t k, bool valid, const int32_t (&from)[3], const int32_t (&f)[3]) {
+        lookup([=](int64_t k, bool valid, const int32_t (&from)[3], const int32_t (&f)[3]) {
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
                 const bool chord = valid && f[s] < 0;
@@ -238,18 +263,52 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
         if (!sc.arena.ok()) return false;
         auto side_from = [=](int64_t q) { return q % 3 == 2 ? mp.t2[q / 3] : mp.t1[q / 3]; };
         auto side_to = [=](int64_t q) { return q % 3 == 0 ? mp.t2[q / 3] : mp.t3[q / 3]; };
+        int32_t *corner_edge[3] = {mp.e12, mp.e13, mp.e23};
         if (!L.has_big()) {
-            for (int64_t q = t.rank(); q < 3 * T; q += t.size())
-                if (slot[q] >= 0) key[cst[side_from(q)] + slot[q]] = side_to(q);
+            struct Sides {
+                int32_t p[3], b, c;  // positions (-1: an edge) and the two larger vertices
+            };
+            team_for_batched<2>(
+                t, T,
+                [=](int64_t k) {
+                    const int32_t a = mp.t1[k], s0 = slot[3 * k], s1 = slot[3 * k + 1], s2 = slot[3 * k + 2];
+                    Sides x;
+                    x.b = mp.t2[k];
+                    x.c = mp.t3[k];
+                    const int32_t ca = cst[a], cb = cst[x.b];
+                    x.p[0] = s0 < 0 ? -1 : ca + s0;
+                    x.p[1] = s1 < 0 ? -1 : ca + s1;
+                    x.p[2] = s2 < 0 ? -1 : cb + s2;
+                    return x;
+                },
+                [=](int64_t, const Sides &x) {
+                    if (x.p[0] >= 0) key[x.p[0]] = x.b;
+                    if (x.p[1] >= 0) key[x.p[1]] = x.c;
+                    if (x.p[2] >= 0) key[x.p[2]] = x.c;
+                });
             t.sync();
-            for (int64_t q = t.rank(); q < 3 * T; q += t.size()) {
-                if (slot[q] < 0) continue;
-                const int32_t a = side_from(q), s = cst[a], e = cst[a + 1];
-                if (e - s > BUCKET_SMALL) continue;
-                const int32_t b = side_to(q);
-                const int32_t p = s + bucket_rank(key, s, e, b, s + slot[q]);
-                ccol[p] = b;
-                crow[p] = a;
+            // a chord's place goes to the triangle too, as -2 - place (a chord
+            // of a long row keeps -1 and is searched for below)
+            for (int64_t k = t.rank(); k < T; k += t.size()) {
+                const int32_t a = mp.t1[k], b = mp.t2[k], c = mp.t3[k];
+                const int32_t sl[3] = {slot[3 * k], slot[3 * k + 1], slot[3 * k + 2]};
+                const int32_t from[3] = {a, a, b}, to[3] = {b, c, c};
+                const int32_t sa = cst[a], ea = cst[a + 1], sb = cst[b], eb = cst[b + 1];
+                const int32_t s[3] = {sa, sa, sb}, e[3] = {ea, ea, eb};
+                int32_t p[3];
+#pragma unroll
+                for (int c3 = 0; c3 < 3; ++c3) {
+                    p[c3] = -1;
+                    if (sl[c3] >= 0 && e[c3] - s[c3] <= BUCKET_SMALL)
+                        p[c3] = s[c3] + bucket_rank(key, s[c3], e[c3], to[c3], s[c3] + sl[c3]);
+                }
+#pragma unroll
+                for (int c3 = 0; c3 < 3; ++c3)
+                    if (p[c3] >= 0) {
+                        ccol[p[c3]] = to[c3];
+                        crow[p[c3]] = from[c3];
+                        corner_edge[c3][k] = -2 - p[c3];
+                    }
             }
             if (L.has_long())
                 team_sort_long_buckets(t, sm, L, cst, reinterpret_cast<const uint32_t *>(key),
@@ -299,6 +358,9 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
         mp.cost = sc.arena.take<float>(E + 1);
         int32_t *moff = sc.arena.take<int32_t>((int64_t)nmax + 2);
         mp.inc_off = sc.arena.take<int32_t>(E + 2);
+        const uint64_t pm = sc.arena.mark();
+        int32_t *apos = sc.arena.take<int32_t>(A.n + 1);  // places of the graph's edges in the merged list
+        int32_t *upos = sc.arena.take<int32_t>(nu + 1);   // ... and of the distinct chords
         if (!sc.arena.ok()) return false;
         team_for_batched(
             t, A.n,
@@ -316,6 +378,7 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
             },
             [=](int64_t e, int4 v) {
                 const int64_t p = e + v.x;
+                apos[e] = (int32_t)p;
                 mp.row[p] = v.y;
                 mp.col[p] = v.z;
                 mp.cost[p] = __int_as_float(v.w);
@@ -323,6 +386,7 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
         for (int64_t k = t.rank(); k < nu; k += t.size()) {
             const int32_t a = urow[k], b = ucol[k];
             const int64_t p = k + lower_edge(aoff, A.col, a, b);
+            upos[k] = (int32_t)p;
             mp.row[p] = a;
             mp.col[p] = b;
             mp.cost[p] = 0.0f;
@@ -332,12 +396,34 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
         if (t.rank() < 4) L.n[t.rank()] = 0;
         t.sync();
         prof_mark(t, sc, PH_MP_CHORDS);
-        // correspondences (compute_triangle_edge_correspondence, :15-62)
+        // correspondences (compute_triangle_edge_correspondence, :15-62), from
+        // the positions that the lookup and the chords' order gave
         int32_t *inc = mp.inc_off;
-        lookup(moff, mp.col, [=](int64_t k, bool valid, const int32_t (&)[3], const int32_t (&f)[3]) {
-            count_sides(k, valid, f, inc);
-        });
+        for (int64_t k0 = (int64_t)t.rank() - lane_id(); k0 < T; k0 += t.size()) {
+            const int64_t k = k0 + lane_id();
+            int32_t f[3] = {-1, -1, -1};
+            if (k < T) {
+                int32_t u[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) f[c] = corner_edge[c][k];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) u[c] = f[c] <= -2 ? upre[-1 - f[c]] - 1 : 0;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    if (f[c] == -1) {
+                        const int32_t a = c == 2 ? mp.t2[k] : mp.t1[k], b = c == 0 ? mp.t2[k] : mp.t3[k];
+                        f[c] = (int32_t)find_edge(moff, mp.col, a, b);
+                    } else {
+                        f[c] = f[c] >= 0 ? apos[f[c]] : upos[u[c]];
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) corner_edge[c][k] = f[c];
+            }
+            count_sides(k, k < T, f, inc);
+        }
         t.sync();
+        sc.arena.release(pm);
     }
     // first slot of each edge, its share of its cost, and the edges whose
     // incoming messages a whole warp sums
@@ -352,24 +438,44 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
     // incidence order: 3t + corner ascending within each edge; the rank of
     // each (triangle, corner) in that order is its slot
     if (!L.has_big()) {
-        auto edge_of = [=](int64_t k, int c) { return c == 0 ? mp.e12[k] : (c == 1 ? mp.e13[k] : mp.e23[k]); };
-        for (int64_t k = t.rank(); k < T; k += t.size())
+        struct Runs {
+            int32_t s[3], e[3], p[3];
+        };
+        auto runs = [=](int64_t k) {
+            const int32_t x[3] = {mp.e12[k], mp.e13[k], mp.e23[k]};
+            Runs r;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) key[mp.inc_off[edge_of(k, c)] + slot[3 * k + c]] = (int32_t)(3 * k + c);
-        t.sync();
-        for (int64_t k = t.rank(); k < T; k += t.size()) {
-            int32_t s[3], e[3];
+            for (int c = 0; c < 3; ++c) r.p[c] = slot[3 * k + c];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const int32_t x = edge_of(k, c);
-                s[c] = mp.inc_off[x];
-                e[c] = mp.inc_off[x + 1];
+                r.s[c] = mp.inc_off[x[c]];
+                r.e[c] = mp.inc_off[x[c] + 1];
             }
 #pragma unroll
-            for (int c = 0; c < 3; ++c)
-                if (e[c] - s[c] <= BUCKET_SMALL)
-                    mp.pos[3 * k + c] = s[c] + bucket_rank(key, s[c], e[c], (int32_t)(3 * k + c), s[c] + slot[3 * k + c]);
-        }
+            for (int c = 0; c < 3; ++c) r.p[c] += r.s[c];
+            return r;
+        };
+        team_for_batched<2>(t, T, runs, [=](int64_t k, const Runs &r) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) key[r.p[c]] = (int32_t)(3 * k + c);
+        });
+        t.sync();
+        team_for_batched<2>(
+            t, T,
+            [=](int64_t k) {
+                Runs r = runs(k);
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    r.p[c] = r.e[c] - r.s[c] <= BUCKET_SMALL
+                                 ? r.s[c] + bucket_rank(key, r.s[c], r.e[c], (int32_t)(3 * k + c), r.p[c])
+                                 : -1;
+                return r;
+            },
+            [=](int64_t k, const Runs &r) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    if (r.p[c] >= 0) mp.pos[3 * k + c] = r.p[c];
+            });
         if (L.has_long())
             team_sort_long_buckets(t, sm, L, mp.inc_off, reinterpret_cast<const uint32_t *>(key),
                                    [=](int32_t, int32_t p, uint32_t q) { mp.pos[q] = p; });
@@ -442,9 +548,37 @@ __device__ __forceinline__ float add_third(float a, double tm) { return (float)_
 // min_gain: the loop ends after an iteration that gains less (the reference's
 // 1e-3).  Returns the bound of the final state; *lb0, if given, receives the
 // bound before the first iteration, *cmin the smallest edge cost.
-__device__ __forceinline__ void mp_moves(const Mp &mp, int64_t k, float t12, float t13, float t23, csum_t &bt)
+//
+// What holds a pass back is the number of loads that wait for one another, so
+// everything a triangle needs by index (its edges, its message slots, its
+// costs) is loaded before its first store: with the slots loaded between the
+// stores (which may alias them) a pair of triangles waited for eight round
+// trips instead of two.
+struct TriState {
+    int32_t e[3], p[3];  // edges and message slots of the corners 12, 13, 23
+    float c[3];          // costs, then with the edges' shares
+};
+
+__device__ __forceinline__ void mp_load(const Mp &mp, int64_t k, bool first, TriState &x)
+{
+    x.e[0] = mp.e12[k];
+    x.e[1] = mp.e13[k];
+    x.e[2] = mp.e23[k];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) x.p[q] = mp.pos[3 * k + q];
+    x.c[0] = x.c[1] = x.c[2] = 0.0f;
+    if (!first) {
+        x.c[0] = mp.c12[k];
+        x.c[1] = mp.c13[k];
+        x.c[2] = mp.c23[k];
+    }
+}
+
+// the triangle's moves; its bound is added to bt
+__device__ __forceinline__ void mp_moves(const Mp &mp, int64_t k, const TriState &x, const float (&s)[3], csum_t &bt)
 {
     const double third = 1.0 / 3.0;
+    float t12 = __fadd_rn(x.c[0], s[0]), t13 = __fadd_rn(x.c[1], s[1]), t23 = __fadd_rn(x.c[2], s[2]);
     float e12, e13, e23;
     {
         const double tm = __dmul_rn(third, (double)min_marginal(t12, t13, t23));
@@ -479,9 +613,9 @@ __device__ __forceinline__ void mp_moves(const Mp &mp, int64_t k, float t12, flo
     mp.c12[k] = t12;
     mp.c13[k] = t13;
     mp.c23[k] = t23;
-    mp.slot[mp.pos[3 * k]] = e12;
-    mp.slot[mp.pos[3 * k + 1]] = e13;
-    mp.slot[mp.pos[3 * k + 2]] = e23;
+    mp.slot[x.p[0]] = e12;
+    mp.slot[x.p[1]] = e13;
+    mp.slot[x.p[2]] = e23;
     bt = cs_add(bt, tri_lb(t12, t13, t23));
 }
 
@@ -514,66 +648,75 @@ __device__ __noinline__ double mp_run(const Team &t, Scratch &sc, const Mp &stat
         // the edges' shares are in flight together
         int64_t k = t.rank();
         for (; k + S < mp.T; k += 2 * S) {
-            const int64_t k2 = k + S;
-            const int32_t a12 = mp.e12[k], a13 = mp.e13[k], a23 = mp.e23[k];
-            const int32_t b12 = mp.e12[k2], b13 = mp.e13[k2], b23 = mp.e23[k2];
-            float ac12 = 0.0f, ac13 = 0.0f, ac23 = 0.0f, bc12 = 0.0f, bc13 = 0.0f, bc23 = 0.0f;
-            if (it > 0) {
-                ac12 = mp.c12[k], ac13 = mp.c13[k], ac23 = mp.c23[k];
-                bc12 = mp.c12[k2], bc13 = mp.c13[k2], bc23 = mp.c23[k2];
+            TriState x, y;
+            mp_load(mp, k, it == 0, x);
+            mp_load(mp, k + S, it == 0, y);
+            float sx[3], sy[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                sx[q] = mp.share[x.e[q]];
+                sy[q] = mp.share[y.e[q]];
             }
-            const float as12 = mp.share[a12], as13 = mp.share[a13], as23 = mp.share[a23];
-            const float bs12 = mp.share[b12], bs13 = mp.share[b13], bs23 = mp.share[b23];
-            mp_moves(mp, k, __fadd_rn(ac12, as12), __fadd_rn(ac13, as13), __fadd_rn(ac23, as23), bt);
-            mp_moves(mp, k2, __fadd_rn(bc12, bs12), __fadd_rn(bc13, bs13), __fadd_rn(bc23, bs23), bt);
+            mp_moves(mp, k, x, sx, bt);
+            mp_moves(mp, k + S, y, sy, bt);
         }
         for (; k < mp.T; k += S) {
-            const float s12 = mp.share[mp.e12[k]], s13 = mp.share[mp.e13[k]], s23 = mp.share[mp.e23[k]];
-            float c12 = 0.0f, c13 = 0.0f, c23 = 0.0f;
-            if (it > 0) c12 = mp.c12[k], c13 = mp.c13[k], c23 = mp.c23[k];
-            mp_moves(mp, k, __fadd_rn(c12, s12), __fadd_rn(c13, s13), __fadd_rn(c23, s23), bt);
+            TriState x;
+            mp_load(mp, k, it == 0, x);
+            const float sx[3] = {mp.share[x.e[0]], mp.share[x.e[1]], mp.share[x.e[2]]};
+            mp_moves(mp, k, x, sx, bt);
         }
         t.sync();
         // covered edges: c = 0 + RSUM(messages); long runs by a warp
         {
-            // four edges a thread at a time: offsets, then the messages, then
+            // four edges a thread at a time: offsets, then the first four
+            // messages of each (most edges have no more), then the rest and
             // the stores
             constexpr int U = 4;
+            auto first4 = [&](float (&x)[4], int32_t s, int32_t n, int64_t e) {
+                if (n > RSUM_THREAD_MAX) n = 0;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) x[j] = j < n ? mp.slot[s + j] : 0.0f;
+                if (n == 0) x[0] = mp.cost[e];
+            };
+            auto finish = [&](const float (&x)[4], int32_t s, int32_t n, int64_t e) {
+                if (n > RSUM_THREAD_MAX) return;
+                float c = x[0];
+                if (n > 0) {
+                    double y[8];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) y[j] = __dadd_rn(0.0, (double)x[j]);
+                    double sum = __dadd_rn(__dadd_rn(y[0], y[1]), __dadd_rn(y[2], y[3]));
+                    if (n > 4) {
+#pragma unroll
+                        for (int j = 4; j < 8; ++j) y[j] = j < n ? __dadd_rn(0.0, (double)mp.slot[s + j]) : 0.0;
+                        sum = __dadd_rn(sum, __dadd_rn(__dadd_rn(y[4], y[5]), __dadd_rn(y[6], y[7])));
+                    }
+                    c = __fadd_rn(0.0f, (float)sum);
+                    mp.cost[e] = c;
+                    mp.share[e] = __fdiv_rn(c, (float)n);
+                }
+                edge_bound(c);
+            };
             int64_t e0 = t.rank();
             for (; e0 + (U - 1) * S < mp.E; e0 += U * S) {
                 int32_t s[U], n[U];
-                float c[U];
+                float x[U][4];
 #pragma unroll
                 for (int q = 0; q < U; ++q) {
                     s[q] = mp.inc_off[e0 + q * S];
                     n[q] = mp.inc_off[e0 + q * S + 1] - s[q];
                 }
 #pragma unroll
-                for (int q = 0; q < U; ++q)
-                    c[q] = n[q] == 0 ? mp.cost[e0 + q * S]
-                                     : (n[q] > RSUM_THREAD_MAX ? 0.0f
-                                                               : __fadd_rn(0.0f, rsum_upto8(mp.slot + s[q], n[q])));
+                for (int q = 0; q < U; ++q) first4(x[q], s[q], n[q], e0 + q * S);
 #pragma unroll
-                for (int q = 0; q < U; ++q) {
-                    if (n[q] != 0 && n[q] <= RSUM_THREAD_MAX) {
-                        mp.cost[e0 + q * S] = c[q];
-                        mp.share[e0 + q * S] = __fdiv_rn(c[q], (float)n[q]);
-                    }
-                    if (n[q] <= RSUM_THREAD_MAX) edge_bound(c[q]);
-                }
+                for (int q = 0; q < U; ++q) finish(x[q], s[q], n[q], e0 + q * S);
             }
             for (; e0 < mp.E; e0 += S) {
                 const int32_t s = mp.inc_off[e0], n = mp.inc_off[e0 + 1] - s;
-                if (n > RSUM_THREAD_MAX) continue;
-                float c;
-                if (n == 0) {
-                    c = mp.cost[e0];
-                } else {
-                    c = __fadd_rn(0.0f, rsum_upto8(mp.slot + s, n));
-                    mp.cost[e0] = c;
-                    mp.share[e0] = __fdiv_rn(c, (float)n);
-                }
-                edge_bound(c);
+                float x[4];
+                first4(x, s, n, e0);
+                finish(x, s, n, e0);
             }
         }
         for (int64_t q = team_warp(t); q < mp.nlong; q += team_nwarps(t)) {

@@ -1578,19 +1578,18 @@ __device__ __forceinline__ int64_t team_bucket_starts(const Team &t, Scratch &sc
         });
 }
 
-// keys in [s, e) ordered before the one at p (equal keys by position)
+// keys in [s, e) ordered before the one at p (equal keys by position); four
+// loads at a time, past the end the last key again, which is not counted
 template <class K>
 __device__ __forceinline__ int32_t bucket_rank(const K *keys, int32_t s, int32_t e, K key, int32_t p)
 {
-    int32_t r = 0, x = s;
-    for (; x + 3 < e; x += 4) {
-        const K a = keys[x], b = keys[x + 1], c = keys[x + 2], d = keys[x + 3];
-        r += (a < key || (a == key && x < p)) + (b < key || (b == key && x + 1 < p)) +
-             (c < key || (c == key && x + 2 < p)) + (d < key || (d == key && x + 3 < p));
-    }
-    for (; x < e; ++x) {
-        const K a = keys[x];
-        r += a < key || (a == key && x < p);
+    int32_t r = 0;
+    for (int32_t x = s; x < e; x += 4) {
+        K a[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a[k] = keys[min(x + k, e - 1)];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r += x + k < e && (a[k] < key || (a[k] == key && x + k < p));
     }
     return r;
 }

@@ -216,8 +216,7 @@ __device__ __noinline__ int64_t tri_normalize(const Team &t, Scratch &sc, char *
                 const Tri r = tri(q < n ? q : n - 1);
                 b[k] = q < n && r.ok() ? r.lo : -1;
             }
-#pragma unroll
-            for (int k = 0; k < U; ++k) s[k] = base + k * S < n ? bucket_slot(start, b[k]) : 0;
+            bucket_slots<U>(start, b, s);
 #pragma unroll
             for (int k = 0; k < U; ++k)
                 if (base + k * S + lane_id() < n) slot[base + k * S + lane_id()] = s[k];
@@ -238,7 +237,7 @@ __device__ __noinline__ int64_t tri_normalize(const Team &t, Scratch &sc, char *
         t.sync();
         team_sort_long_records(t, sm, R, L);
         team_record_tiles<true>(t, sm, R, w,
-                                [&](const RecTile &T, int base, const int4 (&)[4], const bool (&mine)[4]) {
+                                [&](const RecTile<int4> &T, int base, const int4 (&)[4], const bool (&mine)[4]) {
 #pragma unroll
                                     for (int k = 0; k < 4; ++k)
                                         if (mine[k]) {
@@ -298,7 +297,12 @@ __device__ __noinline__ int64_t tri_normalize(const Team &t, Scratch &sc, char *
 }
 
 // The lists of attractive neighbours (cost > pos_tol), ascending: vertex v's
-// are adj[off[v], off[v + 1]).  By buckets of the vertex, each edge in two.
+// are adj[off[v], off[v + 1]).  By buckets of the vertex, each edge in two, as
+// records (neighbour, vertex) that the tile pass orders in shared memory.
+// Every edge's ends are loaded along with its cost: about half of the edges
+// are attractive, so nearly every sector is needed.  With loads behind the
+// cost's branch and each entry ranked in global memory by one thread, the
+// lists of the 1M-point k-NN graph in D mode took 16.1 ms.
 // `off` holds nrows + 1 zeros.  Returns false, with off used up, when a vertex
 // has more than BUCKET_MAX neighbours.
 template <class Team>
@@ -310,32 +314,35 @@ __device__ __noinline__ bool attractive_lists(const Team &t, Scratch &sc, char *
     int32_t *adj = sc.arena.take<int32_t>(2 * A.n + 1);
     adj_out = adj;
     const uint64_t m = sc.arena.mark();
-    int32_t *tadj = sc.arena.take<int32_t>(2 * A.n + 1);
+    RecordArray<int2> R;
+    R.rec = sc.arena.take<int2>(2 * A.n + 1);
+    R.start = off;
+    int2 *rec = R.rec;
     int2 *slot = sc.arena.take<int2>(A.n + 1);
     BucketLists L = bucket_lists(sc, 2 * A.n);
     m2 = 0;
     if (!sc.arena.ok()) return true;
     if (t.rank() < 4) L.n[t.rank()] = 0;
     {
-        // SORT_BATCH strides of a warp at a time: costs, ends, then the atomics
+        // SORT_BATCH strides of a warp at a time: the edges, then the atomics
         constexpr int U = SORT_BATCH;
         const int64_t S = t.size();
         for (int64_t base = (int64_t)t.rank() - lane_id(); base < A.n; base += S * U) {
             int32_t r[U], c[U], sr[U], sc2[U];
 #pragma unroll
             for (int k = 0; k < U; ++k) {
-                const int64_t e = base + k * S + lane_id();
-                r[k] = -1;
-                if (e < A.n && A.cost[e] > pos_tol) {
-                    r[k] = A.row[e];
-                    c[k] = A.col[e];
-                }
+                const int64_t e = base + k * S + lane_id(), x = e < A.n ? e : A.n - 1;
+                const float w = A.cost[x];
+                r[k] = A.row[x];
+                c[k] = A.col[x];
+                if (!(e < A.n && w > pos_tol)) r[k] = -1;
             }
 #pragma unroll
-            for (int k = 0; k < U; ++k)
+            for (int k = 0; k < U; ++k) {
+                sc2[k] = 0;
                 if (r[k] >= 0) sc2[k] = atomicAdd(&off[c[k]], 1);
-#pragma unroll
-            for (int k = 0; k < U; ++k) sr[k] = bucket_slot(off, r[k]);
+            }
+            bucket_slots<U>(off, r, sr);
 #pragma unroll
             for (int k = 0; k < U; ++k)
                 if (r[k] >= 0) slot[base + k * S + lane_id()] = make_int2(sr[k], sc2[k]);
@@ -348,41 +355,40 @@ __device__ __noinline__ bool attractive_lists(const Team &t, Scratch &sc, char *
         return false;
     }
     struct Ends {
-        int32_t r, c, pr, pc;
+        int32_t r, c, pr, pc;  // r: -1 if not attractive
     };
-    auto ends = [=](int64_t e) {
-        Ends x;
-        x.r = -1;
-        if (A.cost[e] > pos_tol) {
+    team_for_batched(
+        t, A.n,
+        [=](int64_t e) {
+            const float w = A.cost[e];
+            const int2 s = slot[e];  // (not set where it is not used)
+            Ends x;
             x.r = A.row[e];
             x.c = A.col[e];
-            const int2 s = slot[e];
-            x.pr = off[x.r] + s.x;
-            x.pc = off[x.c] + s.y;
-        }
-        return x;
-    };
-    team_for_batched(t, A.n, ends, [=](int64_t, Ends x) {
-        if (x.r < 0) return;
-        tadj[x.pr] = x.c;
-        tadj[x.pc] = x.r;
-    });
-    t.sync();
-    auto place = [=](int32_t v, int32_t nbr, int32_t p) {
-        const int32_t s = off[v], e = off[v + 1];
-        adj[e - s > BUCKET_SMALL ? p : s + bucket_rank(tadj, s, e, nbr, p)] = nbr;
-    };
-    team_for_batched<2>(t, A.n, ends, [=](int64_t, Ends x) {
-        if (x.r < 0) return;
-        place(x.r, x.c, x.pr);
-        place(x.c, x.r, x.pc);
-    });
+            const bool pos = w > pos_tol;
+            x.pr = off[pos ? x.r : 0] + s.x;
+            x.pc = off[pos ? x.c : 0] + s.y;
+            if (!pos) x.r = -1;
+            return x;
+        },
+        [=](int64_t, Ends x) {
+            if (x.r < 0) return;
+            rec[x.pr] = make_int2(x.c, x.r);
+            rec[x.pc] = make_int2(x.r, x.c);
+        });
     t.sync();
     if (L.has_long()) {
-        team_sort_long_buckets(t, sm, L, off, reinterpret_cast<const uint32_t *>(tadj),
-                               [=](int32_t, int32_t p, uint32_t key) { adj[p] = (int32_t)key; });
+        team_sort_long_buckets<uint32_t>(
+            t, sm, L, off, [=](int32_t p) { return (uint32_t)rec[p].x; },
+            [=](int32_t v, int32_t p, uint32_t key) { rec[p] = make_int2((int32_t)key, v); });
         t.sync();
     }
+    team_record_tiles<true>(t, sm, R, m2, [&](const RecTile<int2> &T, int base, const int2 (&)[4], const bool (&mine)[4]) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (mine[k]) adj[T.p0 + base + 32 * k] = T.win[base + 32 * k].x;
+    });
+    t.sync();
     sc.arena.release(m);
     return true;
 }
@@ -502,40 +508,51 @@ __device__ __forceinline__ void expansion_stage(const Team &t, Scratch &sc, char
             for (int b = threadIdx.x; b < EXP_BINS; b += blockDim.x)
                 if (lh[b]) atomicAdd(&hist[b], lh[b]);
             t.sync();
-            // every warp of every CTA: lane l holds bins 32 l .. 32 l + 31
-            constexpr int PER = EXP_BINS / 32;
-            int64_t n_l = 0, s_l = 0;  // expansions and emissions of the lane's bins
-            for (int k = 0; k < PER; ++k) {
-                const int b = lane_id() * PER + k;
-                const int64_t h = __ldcg(hist + b);
-                n_l += h;
-                s_l += h * b;
-            }
-            // expansions in higher bins, and emissions in lower ones
-            const int64_t n_all = warp_sum(n_l);
-            int64_t above = n_all - (warp_incl_scan(n_l) - n_l);  // counts >= the lane's first bin
-            int64_t below = warp_incl_scan(s_l) - s_l;
-            // S(k) = below(k) + k * (counts >= k), for k up to EXP_BINS - 1
-            int64_t bestk = -1, bests = 0;
-            for (int k = 0; k < PER; ++k) {
-                const int64_t b = lane_id() * PER + k;
-                const int64_t S = below + b * above;
-                if (S <= rem) {
-                    bestk = b;
-                    bests = S;
+            // The CTA takes the bins to shared memory and one warp finds K:
+            // lane l holds bins 32 l .. 32 l + 31.  (With every warp of the
+            // grid reading the bins from L2 a truncation took 0.35 ms.)
+            for (int b = threadIdx.x; b < EXP_BINS; b += blockDim.x) lh[b] = __ldcg(hist + b);
+            __shared__ int64_t best[2];
+            __syncthreads();
+            if (warp_in_block() == 0) {
+                constexpr int PER = EXP_BINS / 32;
+                int64_t n_l = 0, s_l = 0;  // expansions and emissions of the lane's bins
+                for (int k = 0; k < PER; ++k) {
+                    const int b = lane_id() * PER + k;
+                    n_l += lh[b];
+                    s_l += (int64_t)lh[b] * b;
                 }
-                const int64_t h = __ldcg(hist + b);
-                below += h * b;
-                above -= h;
-            }
+                // expansions in higher bins, and emissions in lower ones
+                const int64_t n_all = warp_sum(n_l);
+                int64_t above = n_all - (warp_incl_scan(n_l) - n_l);  // counts >= the lane's first bin
+                int64_t below = warp_incl_scan(s_l) - s_l;
+                // S(k) = below(k) + k * (counts >= k), for k up to EXP_BINS - 1
+                int64_t bestk = -1, bests = 0;
+                for (int k = 0; k < PER; ++k) {
+                    const int64_t b = lane_id() * PER + k;
+                    const int64_t S = below + b * above;
+                    if (S <= rem) {
+                        bestk = b;
+                        bests = S;
+                    }
+                    below += (int64_t)lh[b] * b;
+                    above -= lh[b];
+                }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const int64_t ok = __shfl_xor_sync(FULL, bestk, o), os = __shfl_xor_sync(FULL, bests, o);
-                if (ok > bestk) {
-                    bestk = ok;
-                    bests = os;
+                for (int o = 16; o > 0; o >>= 1) {
+                    const int64_t ok = __shfl_xor_sync(FULL, bestk, o), os = __shfl_xor_sync(FULL, bests, o);
+                    if (ok > bestk) {
+                        bestk = ok;
+                        bests = os;
+                    }
+                }
+                if (lane_id() == 0) {
+                    best[0] = bestk;
+                    best[1] = bests;
                 }
             }
+            __syncthreads();
+            const int64_t bestk = best[0], bests = best[1];
             int64_t lo = bestk, slo = bests;  // S(0) = 0 always fits
             if (lo == EXP_BINS - 1) {
                 const int32_t mx = team_max<Team, int32_t>(t, sc, sm, xn, 0, [=](int64_t q) { return ccount[q]; });

@@ -97,15 +97,27 @@ __device__ __noinline__ int32_t matching_contraction_map(const Team &t, Scratch 
             int32_t *wsum = reinterpret_cast<int32_t *>(sm);  // per warp: list count, touched count; then bases
             auto offer_tile = [=](const int32_t (&u)[MI], const int32_t (&v)[MI], const uint32_t (&hb)[MI],
                                   const bool (&live)[MI]) {
-                bool fu[MI], fv[MI];
+                // neighbouring edges of a row make one offer to it: the larger
+                unsigned long long best[MI];
+                bool offers[MI], fu[MI], fv[MI];
+#pragma unroll
+                for (int k = 0; k < MI; ++k) {
+                    best[k] = (unsigned long long)hb[k] << 32 | (unsigned long long)(~(uint32_t)v[k]);
+                    offers[k] = live[k];
+                }
+#pragma unroll
+                for (int k = 0; k + 1 < MI; ++k)
+                    if (live[k] && live[k + 1] && u[k] == u[k + 1]) {
+                        best[k + 1] = best[k] > best[k + 1] ? best[k] : best[k + 1];
+                        offers[k] = false;
+                    }
 #pragma unroll
                 for (int k = 0; k < MI; ++k) {
                     fu[k] = fv[k] = false;
-                    if (live[k]) {
-                        const unsigned long long hi = (unsigned long long)hb[k] << 32;
-                        fu[k] = atomicMax(&cur_offer[u[k]], hi | (unsigned long long)(~(uint32_t)v[k])) == 0ull;
-                        fv[k] = atomicMax(&cur_offer[v[k]], hi | (unsigned long long)(~(uint32_t)u[k])) == 0ull;
-                    }
+                    if (offers[k]) fu[k] = atomicMax(&cur_offer[u[k]], best[k]) == 0ull;
+                    if (live[k])
+                        fv[k] = atomicMax(&cur_offer[v[k]], (unsigned long long)hb[k] << 32 |
+                                                                (unsigned long long)(~(uint32_t)u[k])) == 0ull;
                 }
                 int nl = 0, nt = 0;
 #pragma unroll

@@ -26,7 +26,9 @@ struct Mp {
     float *share;      // E: cost / number of incident triangles (covered edges)
     int32_t *inc_off;  // E + 1: first slot of each edge
     int32_t *longe;    // edges with more than RSUM_THREAD_MAX incident triangles
-    int64_t nlong;
+    int64_t nlong;     // ... of them those with up to 64, from the front
+    int64_t nhuge;     // ... and the others, from the back (longe_cap)
+    int64_t longe_cap;
     int inplace;  // row, col and cost are the graph's own arrays (no chords)
 };
 
@@ -150,7 +152,7 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
         if (!sc.arena.ok()) return false;
         for (int64_t v = t.rank(); v <= nbk; v += t.size()) cst[v] = 0;
     }
-    if (t.rank() < 4) L.n[t.rank()] = 0;
+    if (t.rank() < 8) L.n[t.rank()] = 0;
     team_offsets(t, A.n, nmax, [=](int64_t e) { return A.row[e]; }, aoff);
     // the triangles' sides among the graph's edges; `each` gets the three
     // positions (-1: not an edge) with all lanes of the warp present.  Two
@@ -239,7 +241,7 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
             mp.inc_off = sc.arena.take<int32_t>(A.n + 2);
             if (!sc.arena.ok()) return false;
             for (int64_t e = t.rank(); e <= A.n; e += t.size()) mp.inc_off[e] = 0;
-            if (t.rank() < 4) L.n[t.rank()] = 0;
+            if (t.rank() < 8) L.n[t.rank()] = 0;
             t.sync();
             int32_t *inc = mp.inc_off;
             for (int64_t k0 = (int64_t)t.rank() - lane_id(); k0 < T; k0 += t.size()) {
@@ -311,11 +313,12 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
                     }
             }
             if (L.has_long())
-                team_sort_long_buckets(t, sm, L, cst, reinterpret_cast<const uint32_t *>(key),
-                                       [=](int32_t b, int32_t p, uint32_t c) {
-                                           ccol[p] = (int32_t)c;
-                                           crow[p] = b;
-                                       });
+                team_sort_long_buckets<uint32_t>(
+                    t, sm, L, cst, [=](int32_t p) { return (uint32_t)key[p]; },
+                    [=](int32_t b, int32_t p, uint32_t c) {
+                        ccol[p] = (int32_t)c;
+                        crow[p] = b;
+                    });
             t.sync();
         } else {
             // a row with more than BUCKET_MAX chords: LSD radix sort of (row, col)
@@ -393,7 +396,7 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
         }
         for (int64_t v = t.rank(); v <= nmax; v += t.size()) moff[v] = aoff[v] + upre[cst[v]];
         for (int64_t e = t.rank(); e <= E; e += t.size()) mp.inc_off[e] = 0;
-        if (t.rank() < 4) L.n[t.rank()] = 0;
+        if (t.rank() < 8) L.n[t.rank()] = 0;
         t.sync();
         prof_mark(t, sc, PH_MP_CHORDS);
         // correspondences (compute_triangle_edge_correspondence, :15-62), from
@@ -428,13 +431,18 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
     // first slot of each edge, its share of its cost, and the edges whose
     // incoming messages a whole warp sums
     mp.share = sc.arena.take<float>(mp.E + 1);
-    mp.longe = sc.arena.take<int32_t>(3 * T / (RSUM_THREAD_MAX + 1) + 1);
+    mp.longe_cap = 3 * T / (RSUM_THREAD_MAX + 1) + 1;
+    mp.longe = sc.arena.take<int32_t>(mp.longe_cap);
     if (!sc.arena.ok()) return false;
     team_bucket_starts(t, sc, sm, (int32_t)mp.E, mp.inc_off, L, [=](int64_t e, int32_t, int32_t n) {
         mp.share[e] = n > 0 ? __fdiv_rn(mp.cost[e], (float)n) : 0.0f;
-        if (n > RSUM_THREAD_MAX) mp.longe[atomicAdd(&L.n[3], 1)] = (int32_t)e;
+        if (n > 64)
+            mp.longe[mp.longe_cap - 1 - atomicAdd(&L.n[4], 1)] = (int32_t)e;
+        else if (n > RSUM_THREAD_MAX)
+            mp.longe[atomicAdd(&L.n[3], 1)] = (int32_t)e;
     });
     mp.nlong = uread(&L.n[3]);
+    mp.nhuge = uread(&L.n[4]);
     // incidence order: 3t + corner ascending within each edge; the rank of
     // each (triangle, corner) in that order is its slot
     if (!L.has_big()) {
@@ -477,8 +485,9 @@ __device__ __noinline__ bool mp_build(const Team &t, Scratch &sc, char *, const 
                     if (r.p[c] >= 0) mp.pos[3 * k + c] = r.p[c];
             });
         if (L.has_long())
-            team_sort_long_buckets(t, sm, L, mp.inc_off, reinterpret_cast<const uint32_t *>(key),
-                                   [=](int32_t, int32_t p, uint32_t q) { mp.pos[q] = p; });
+            team_sort_long_buckets<uint32_t>(
+                t, sm, L, mp.inc_off, [=](int32_t p) { return (uint32_t)key[p]; },
+                [=](int32_t, int32_t p, uint32_t q) { mp.pos[q] = p; });
         t.sync();
     } else {
         const uint64_t rm = sc.arena.mark();
@@ -719,8 +728,20 @@ __device__ __noinline__ double mp_run(const Team &t, Scratch &sc, const Mp &stat
                 finish(x, s, n, e0);
             }
         }
-        for (int64_t q = team_warp(t); q < mp.nlong; q += team_nwarps(t)) {
+        // longer runs: up to 64 messages by a thread, more by a warp.  (With a
+        // warp for every run of more than 8 its few round trips came in turn
+        // for some 80 edges a warp: 0.3 of the 0.5 ms this pass took on the
+        // 1M-point k-NN graph's dual with 398,000 such edges.)
+        for (int64_t q = t.rank(); q < mp.nlong; q += S) {
             const int32_t e = mp.longe[q];
+            const int32_t s = mp.inc_off[e], n = mp.inc_off[e + 1] - s;
+            const float c = __fadd_rn(0.0f, rsum_upto64(n, [=](int x) { return mp.slot[s + x]; }));
+            mp.cost[e] = c;
+            mp.share[e] = __fdiv_rn(c, (float)n);
+            edge_bound(c);
+        }
+        for (int64_t q = team_warp(t); q < mp.nhuge; q += team_nwarps(t)) {
+            const int32_t e = mp.longe[mp.longe_cap - 1 - q];
             const int32_t s = mp.inc_off[e], n = mp.inc_off[e + 1] - s;
             const float c = __fadd_rn(0.0f, rsum_warp(n, [=](int64_t x) { return mp.slot[s + x]; }));
             if (lane_id() == 0) {

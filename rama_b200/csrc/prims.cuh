@@ -1543,7 +1543,8 @@ constexpr int BUCKET_SMALL = 64;
 
 struct BucketLists {
     int32_t *warp, *cta;  // buckets of 65..256 and of 257..BUCKET_MAX keys
-    int32_t *n;           // [0], [1]: their numbers, [2]: some bucket is larger (the caller zeroes all)
+    int32_t *n;           // [0], [1]: their numbers, [2]: some bucket is larger, the rest is the caller's, who zeroes
+                          // what is used
     __device__ __forceinline__ bool has_long() const { return uread(&n[0]) + uread(&n[1]) > 0; }
     __device__ __forceinline__ bool has_big() const { return uread(&n[2]) != 0; }
 };
@@ -1553,7 +1554,7 @@ __device__ __forceinline__ BucketLists bucket_lists(Scratch &sc, int64_t nitems)
     BucketLists L;
     L.warp = sc.arena.take<int32_t>(nitems / (BUCKET_SMALL + 1) + 1);
     L.cta = sc.arena.take<int32_t>(nitems / 257 + 1);
-    L.n = sc.arena.take<int32_t>(4);
+    L.n = sc.arena.take<int32_t>(8);
     return L;
 }
 
@@ -1605,6 +1606,24 @@ __device__ __forceinline__ int32_t bucket_slot(int32_t *counts, int32_t b)
     return __shfl_sync(FULL, s, leader) + __popc(peers & lanemask_lt());
 }
 
+// The same for U items a lane at a time: the atomics of all of them are in
+// flight together (the contraction's slot passes of the 24.8 M edge volume
+// waited for four in turn before).
+template <int U>
+__device__ __forceinline__ void bucket_slots(int32_t *counts, const int32_t (&b)[U], int32_t (&s)[U])
+{
+    unsigned peers[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+        peers[k] = __match_any_sync(FULL, b[k]);
+        s[k] = 0;
+        if (b[k] >= 0 && lane_id() == __ffs(peers[k]) - 1) s[k] = atomicAdd(&counts[b[k]], __popc(peers[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+        s[k] = __shfl_sync(FULL, s[k], __ffs(peers[k]) - 1) + __popc(peers[k] & lanemask_lt());
+}
+
 template <class K, class Bar>
 __device__ __forceinline__ void smem_bitonic_keys(K *key, int m, int P, int lane, int nth, Bar bar)
 {
@@ -1626,11 +1645,12 @@ __device__ __forceinline__ void smem_bitonic_keys(K *key, int m, int P, int lane
         }
 }
 
-// Sorts the listed buckets of keys[] (not written) and calls emit(b, p, key)
-// for every sorted position p.  Keys are below ~K(0).  The caller syncs.
-template <class Team, class K, class Emit>
+// Sorts the listed buckets of the keys load(p) and calls emit(b, p, key) for
+// every sorted position p, after all loads of the bucket.  Keys are below
+// ~K(0).  The caller syncs.
+template <class K, class Team, class Load, class Emit>
 __device__ __forceinline__ void team_sort_long_buckets(const Team &t, char *sm, BucketLists L, const int32_t *start,
-                                                       const K *keys, Emit emit)
+                                                       Load load, Emit emit)
 {
     {
         K *wk = reinterpret_cast<K *>(sm) + warp_in_block() * 256;
@@ -1639,7 +1659,7 @@ __device__ __forceinline__ void team_sort_long_buckets(const Team &t, char *sm, 
             const int32_t b = L.warp[q], s = start[b], m = start[b + 1] - s;
             int P = 128;
             while (P < m) P <<= 1;
-            for (int x = lane_id(); x < m; x += 32) wk[x] = keys[s + x];
+            for (int x = lane_id(); x < m; x += 32) wk[x] = load(s + x);
             __syncwarp();
             smem_bitonic_keys(wk, m, P, lane_id(), 32, [] { __syncwarp(); });
             for (int x = lane_id(); x < m; x += 32) emit(b, s + x, wk[x]);
@@ -1654,7 +1674,7 @@ __device__ __forceinline__ void team_sort_long_buckets(const Team &t, char *sm, 
             const int32_t b = L.cta[q], s = start[b], m = start[b + 1] - s;
             int P = 512;
             while (P < m) P <<= 1;
-            for (int x = threadIdx.x; x < m; x += blockDim.x) ck[x] = keys[s + x];
+            for (int x = threadIdx.x; x < m; x += blockDim.x) ck[x] = load(s + x);
             __syncthreads();
             smem_bitonic_keys(ck, m, P, threadIdx.x, blockDim.x, [] { __syncthreads(); });
             for (int x = threadIdx.x; x < m; x += blockDim.x) emit(b, s + x, ck[x]);

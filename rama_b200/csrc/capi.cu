@@ -28,12 +28,28 @@ namespace {
 // Launch parameters a handle starts with (rama_tuning; the autotuner of
 // rama_b200/autotune.py replaces them with measured choices).  None of them
 // changes a result: every team computes the same solve.
-constexpr int DEFAULT_CLUSTER_CTAS = 8;            // CTAs of a cluster team (the portable maximum)
+constexpr int DEFAULT_CLUSTER_CTAS = 8;  // rama_tuning's starting value: the size follows the use, as below
+constexpr int SINGLE_CLUSTER_CTAS = 16;  // CTAs of a cluster that has the GPU to itself
+constexpr int BATCH_CLUSTER_CTAS = 4;    // ... of many clusters in a batch
 constexpr int64_t DEFAULT_SINGLE_CLUSTER_MIN = 4000;  // a single solve from this size on runs on a cluster
 constexpr int64_t DEFAULT_SINGLE_GRID_MIN = 100000;   // ... and from this size on on the whole GPU
-constexpr int64_t DEFAULT_BATCH_CLUSTER_MIN = 20000;  // smaller batch instances always run on one CTA
-constexpr float DEFAULT_BATCH_CLUSTER_SHARE = 1.5f;   // ... larger ones on a cluster above this many
-                                                      // times the batch's edges per CTA
+// Solves without a dual have a fraction of the passes' work per edge, so they
+// change teams at twice these sizes.  Measured (ms, one CTA / cluster of 16 /
+// whole GPU): region graphs without a dual, 5,822 edges 0.88 / 1.03 / 1.49,
+// 8,785 edges 0.98 / 0.98 / 1.43, 208,942 edges - / 1.65 / 1.73; with, 2,874
+// edges 2.26 / 2.26 / 3.46, 5,822 edges 3.43 / 2.63 / 4.14, 89,308 edges
+// - / 4.62 / 5.02, 208,942 edges - / 7.10 / 5.31.
+constexpr int64_t WIDE_CLUSTER_MIN = 7000;  // single clusters below this size take 8 CTAs: 2.57 and 2.63 ms at 5,822
+                                            // edges with a dual, 2.15 and 2.05 at 8,064
+// One CTA per SM solves graphs of up to 1.5 M edges sooner (fewer partial
+// results to fold; 2.83 ms against 3.24 at 753,664 edges, 10.9 against 11.4 at
+// 1.14 M), two larger ones (4.49 against 4.70 at 3.06 M, 17.9 against 24.8 at
+// 24.8 M).
+constexpr int64_t DEFAULT_GRID_SMALL_MAX = 1500000;
+constexpr int64_t DEFAULT_BATCH_CLUSTER_MIN = 10000;  // smaller batch instances always run on one CTA
+constexpr float DEFAULT_BATCH_CLUSTER_SHARE = 1.0f;   // ... larger ones on a cluster above this many
+                                                      // times the batch's edges per CTA (256 region graphs
+                                                      // PD: 15.0 ms, against 15.8 at 20,000 and 1.5)
 
 thread_local std::string g_err;
 
@@ -77,6 +93,12 @@ Options to_opts(const rama_options *o)
     r.sanitize_graph = o->sanitize_graph;
     r.woc_pentagons = o->woc_pentagons;
     return r;
+}
+
+bool has_dual(const Options &o)
+{
+    return (o.max_cycle_length_lb >= 3 && o.num_dual_itr_lb != 0 && o.num_outer_itr_dual != 0) ||
+           (!o.only_compute_lb && o.max_cycle_length_primal >= 3 && o.num_dual_itr_primal != 0);
 }
 
 }  // namespace
@@ -226,17 +248,32 @@ int cluster_capacity(rama_context *h, int size)
     return h->cluster_cap[size] > 0 ? h->cluster_cap[size] : 0;
 }
 
+// The cluster size of a launch of `ncluster` instances for clusters, the
+// largest of `edges` edges.  One solve finishes soonest on the largest
+// cluster; where they do not all run at once the clusters' CTA time counts.
+// Measured (ms): region graph of 59,436 edges PD on 4, 8, 16 CTAs 7.88, 5.29,
+// 4.05; 12 graphs of 500 to 20,000 nodes on 4 and 16 7.00, 4.22; 40 of them
+// 6.12, 7.62; 256 of them on 4, 8, 16 15.8, 21.8, 34.2.
+int cluster_size(rama_context *h, int32_t ncluster, bool batch, int64_t edges)
+{
+    if (h->tune.cluster_ctas != DEFAULT_CLUSTER_CTAS) return h->tune.cluster_ctas;
+    if (ncluster * SINGLE_CLUSTER_CTAS <= h->sms && (batch || edges >= WIDE_CLUSTER_MIN) &&
+        cluster_capacity(h, SINGLE_CLUSTER_CTAS) > 0)
+        return SINGLE_CLUSTER_CTAS;
+    return ncluster * DEFAULT_CLUSTER_CTAS <= h->sms ? DEFAULT_CLUSTER_CTAS : BATCH_CLUSTER_CTAS;
+}
+
 int launch_solve(rama_context *h, int32_t count, int team, cudaStream_t st, int32_t ncluster = 0,
-                 int64_t grid_edges = 0)
+                 int64_t edges = 0, bool batch = false)
 {
     if (team == 2) {
         GridLaunch L{h->d_inst, h->ws, h->ws_bytes};
         void *args[] = {&L};
-        const int per_sm = grid_edges < h->tune.grid_small_max ? h->tune.grid_small_ctas_per_sm
+        const int per_sm = edges < h->tune.grid_small_max ? h->tune.grid_small_ctas_per_sm
                                                                 : h->tune.grid_ctas_per_sm;
         CU(cudaLaunchCooperativeKernel((void *)k_solve_grid, dim3(per_sm * h->sms), dim3(THREADS), args, SMEM, st));
     } else if (ncluster > 0) {
-        const int csz = h->tune.cluster_ctas;
+        const int csz = cluster_size(h, ncluster, batch, edges);
         const int64_t want = (int64_t)ncluster * csz + (count - ncluster);
         const int64_t cap = (int64_t)std::max(1, cluster_capacity(h, csz)) * csz;
         const int64_t ctas = (std::min(want, cap) + csz - 1) / csz * csz;
@@ -279,7 +316,10 @@ int solve_one(rama_context *h, const int32_t *d_i, const int32_t *d_j, const flo
     Options o = to_opts(opts);
     int team = opts->team;
     if (team < 1 || team > 3)
-        team = n < h->tune.single_cluster_min ? 1 : (n < h->tune.single_grid_min ? 3 : 2);
+    {
+        const int64_t size = has_dual(o) ? n : n / 2;
+        team = size < h->tune.single_cluster_min ? 1 : (size < h->tune.single_grid_min ? 3 : 2);
+    }
     int rc = ensure_inst(h, 1);
     if (rc) return rc;
     // timeline buffer
@@ -455,8 +495,8 @@ int rama_create(int device, uint64_t workspace_bytes, rama_handle *out)
     h->grid_per_sm_max = per_sm;
     h->grid_ctas = per_sm * h->sms;
     h->tune.grid_ctas_per_sm = per_sm;
-    h->tune.grid_small_ctas_per_sm = per_sm;
-    h->tune.grid_small_max = 0;
+    h->tune.grid_small_ctas_per_sm = 1;
+    h->tune.grid_small_max = DEFAULT_GRID_SMALL_MAX;
     h->tune.cluster_ctas = DEFAULT_CLUSTER_CTAS;
     h->tune.single_cluster_min = DEFAULT_SINGLE_CLUSTER_MIN;
     h->tune.single_grid_min = DEFAULT_SINGLE_GRID_MIN;
@@ -645,8 +685,8 @@ int rama_batch_launch(rama_handle h, const int32_t *d_i, const int32_t *d_j, con
         h->b_order[k] = k;
     }
     // Automatic teams: an instance goes to a cluster when one CTA alone would
-    // take much longer than the batch as a whole, i.e. when it holds more than
-    // 1.5 times the edges per CTA of the batch (a cluster finishes it sooner
+    // take longer than the batch as a whole, i.e. when it holds more edges than
+    // the batch has per CTA (a cluster finishes it sooner
     // but spends more CTA time on it).
     {
         int64_t total_edges = 0;
@@ -693,7 +733,7 @@ int rama_batch_launch(rama_handle h, const int32_t *d_i, const int32_t *d_j, con
     if (count == 1 && opts[0].team == 2)
         rc = launch_solve(h, 1, 2, st, 0, h->b_in[0].n);
     else
-        rc = launch_solve(h, count, 1, st, ncluster);
+        rc = launch_solve(h, count, 1, st, ncluster, 0, true);
     if (rc) return rc;
     CU(cudaEventRecord(h->ev1, st));
     CU(cudaMemcpyAsync(h->b_host, h->d_inst, sizeof(Instance) * count, cudaMemcpyDeviceToHost, st));
@@ -759,7 +799,7 @@ int rama_batch_wait(rama_handle h, int64_t *num_labels, double *lbs, int32_t *st
         CU(cudaMemcpyAsync(h->d_inst, sub.data(), sizeof(Instance) * sub.size(), cudaMemcpyHostToDevice, h->b_stream));
         CU(cudaMemcpyAsync(h->d_order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice,
                            h->b_stream));
-        rc = launch_solve(h, (int32_t)sub.size(), 1, h->b_stream, ncl);
+        rc = launch_solve(h, (int32_t)sub.size(), 1, h->b_stream, ncl, 0, true);
         if (rc) return rc;
         CU(cudaMemcpyAsync(sub.data(), h->d_inst, sizeof(Instance) * sub.size(), cudaMemcpyDeviceToHost, h->b_stream));
         CU(cudaStreamSynchronize(h->b_stream));

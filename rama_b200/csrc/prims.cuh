@@ -160,12 +160,16 @@ __device__ __forceinline__ T block_excl_scan(T v, T *sm, T &total)
     return r;
 }
 
+// the sum over the CTA, on every thread; `sm` needs 32 * sizeof(T) bytes
 template <class T>
 __device__ __forceinline__ T block_sum(T v, T *sm)
 {
-    T t;
-    block_excl_scan(v, sm, t);
-    return t;
+    v = warp_sum(v);
+    if (lane_id() == 0) sm[warp_in_block()] = v;
+    __syncthreads();
+    const T r = warp_sum(lane_id() < (int)(blockDim.x >> 5) ? sm[lane_id()] : T(0));
+    __syncthreads();
+    return r;
 }
 
 template <class T>
@@ -504,6 +508,10 @@ __device__ __forceinline__ void cta_prefix_parts(const Team &t, Scratch &sc, con
 // in order with shuffles, and one block scan of the warp totals per tile
 // keeps the CTA's barriers few.  Integer sums only, so the result does not
 // depend on the tiling.
+//
+// Where every CTA's chunk is at most one tile (up to 303,000 elements on 148
+// CTAs) the values are read and scanned once, before the team sync, and stay
+// in registers: such scans wait for round trips, not for bandwidth.
 // ---------------------------------------------------------------------------
 template <class T>
 struct ScanItems {
@@ -519,8 +527,20 @@ __device__ T team_scan_while(const Team &t, Scratch &sc, char *sm, int64_t n, In
     T *tsm = reinterpret_cast<T *>(sm);
     int64_t lo, hi;
     block_chunk(t, n, lo, hi);
-    T s = T(0);
-    {
+    const int64_t TILE = (int64_t)blockDim.x * ITEMS;
+    const int64_t wseg = (int64_t)warp_in_block() * 32 * ITEMS;
+    const bool one = (n + TILE - 1) / TILE <= t.nblocks();
+    T base = T(0), total = T(0);
+    auto prefix = [&](T mine) {  // base and total from the CTAs' sums; one team sync
+        total = mine;
+        if (t.nblocks() == 1) return;
+        T *part = reinterpret_cast<T *>(sc.next_part());
+        if (threadIdx.x == 0) part[t.block()] = mine;
+        t.sync();
+        cta_prefix_parts(t, sc, part, base, total);
+    };
+    if (!one) {
+        T s = T(0);
         // four strides at a time, loads issued together
         constexpr int U = 4;
         const int64_t S = blockDim.x;
@@ -533,19 +553,10 @@ __device__ T team_scan_while(const Team &t, Scratch &sc, char *sm, int64_t n, In
             for (int k = 0; k < U; ++k) s += v[k];
         }
         for (; i < hi; i += S) s += in(i);
+        prefix(block_sum<T>(s, tsm));
+        if (!go_on(total)) return total;
     }
-    s = block_sum<T>(s, tsm);
-    T base = T(0), total = s;
-    if (t.nblocks() > 1) {
-        T *part = reinterpret_cast<T *>(sc.next_part());
-        if (threadIdx.x == 0) part[t.block()] = s;
-        t.sync();
-        cta_prefix_parts(t, sc, part, base, total);
-    }
-    if (!go_on(total)) return total;
-    const int64_t TILE = (int64_t)blockDim.x * ITEMS;
-    const int64_t wseg = (int64_t)warp_in_block() * 32 * ITEMS;
-    for (int64_t tile = lo; tile < hi; tile += TILE) {
+    for (int64_t tile = lo; one || tile < hi; tile += TILE) {
         const int64_t i0 = tile + wseg + lane_id();
         T v[ITEMS], ex[ITEMS];
 #pragma unroll
@@ -558,11 +569,16 @@ __device__ T team_scan_while(const Team &t, Scratch &sc, char *sm, int64_t n, In
             wrun += __shfl_sync(FULL, x, 31);
         }
         T ts;
-        const T wofs = base + block_excl_scan<T>(lane_id() == 0 ? wrun : T(0), tsm, ts);
-        const T wbase = __shfl_sync(FULL, wofs, 0);
+        const T wofs = block_excl_scan<T>(lane_id() == 0 ? wrun : T(0), tsm, ts);
+        if (one) {
+            prefix(ts);
+            if (!go_on(total)) return total;
+        }
+        const T wbase = base + __shfl_sync(FULL, wofs, 0);
 #pragma unroll
         for (int k = 0; k < ITEMS; ++k)
             if (i0 + 32 * k < hi) out(i0 + 32 * k, wbase + ex[k], v[k]);
+        if (one) break;
         base += ts;
     }
     t.sync();
@@ -1545,8 +1561,10 @@ struct BucketLists {
     int32_t *warp, *cta;  // buckets of 65..256 and of 257..BUCKET_MAX keys
     int32_t *n;           // [0], [1]: their numbers, [2]: some bucket is larger, the rest is the caller's, who zeroes
                           // what is used
-    __device__ __forceinline__ bool has_long() const { return uread(&n[0]) + uread(&n[1]) > 0; }
-    __device__ __forceinline__ bool has_big() const { return uread(&n[2]) != 0; }
+    bool some;            // some bucket holds more than BUCKET_SMALL keys (comes with the scan of the counts, so
+                          // that the numbers are read only then)
+    __device__ __forceinline__ bool has_long() const { return some && uread(&n[0]) + uread(&n[1]) > 0; }
+    __device__ __forceinline__ bool has_big() const { return some && uread(&n[2]) != 0; }
 };
 
 __device__ __forceinline__ BucketLists bucket_lists(Scratch &sc, int64_t nitems)
@@ -1555,6 +1573,7 @@ __device__ __forceinline__ BucketLists bucket_lists(Scratch &sc, int64_t nitems)
     L.warp = sc.arena.take<int32_t>(nitems / (BUCKET_SMALL + 1) + 1);
     L.cta = sc.arena.take<int32_t>(nitems / 257 + 1);
     L.n = sc.arena.take<int32_t>(8);
+    L.some = false;
     return L;
 }
 
@@ -1562,11 +1581,19 @@ __device__ __forceinline__ BucketLists bucket_lists(Scratch &sc, int64_t nitems)
 // start, count) is called once per bucket.  Two team syncs.
 template <class Team, class Each>
 __device__ __forceinline__ int64_t team_bucket_starts(const Team &t, Scratch &sc, char *sm, int32_t nb,
-                                                      int32_t *counts, BucketLists L, Each each)
+                                                      int32_t *counts, BucketLists &lists, Each each)
 {
-    return team_scan<Team, int64_t>(
-        t, sc, sm, nb, [=](int64_t b) -> int64_t { return counts[b]; },
-        [=](int64_t b, int64_t pre, int64_t c) {
+    // sums of counts below 2^36, the number of long buckets above
+    constexpr int64_t LONG = int64_t(1) << 36;
+    const BucketLists L = lists;
+    const int64_t total = team_scan<Team, int64_t>(
+        t, sc, sm, nb,
+        [=](int64_t b) -> int64_t {
+            const int32_t c = counts[b];
+            return c > BUCKET_SMALL ? c + LONG : c;
+        },
+        [=](int64_t b, int64_t sums, int64_t v) {
+            const int64_t pre = sums & (LONG - 1), c = v & (LONG - 1);
             counts[b] = (int32_t)pre;
             if (b == nb - 1) counts[nb] = (int32_t)(pre + c);
             if (c > BUCKET_MAX)
@@ -1577,6 +1604,8 @@ __device__ __forceinline__ int64_t team_bucket_starts(const Team &t, Scratch &sc
                 L.warp[atomicAdd(&L.n[0], 1)] = (int32_t)b;
             each(b, (int32_t)pre, (int32_t)c);
         });
+    lists.some = total >= LONG;
+    return total & (LONG - 1);
 }
 
 // keys in [s, e) ordered before the one at p (equal keys by position); four

@@ -340,25 +340,45 @@ template <class Team>
 __device__ int64_t parse_multicut(const Team &t, Scratch &sc, char *sm, const char *text, int64_t len, int32_t *oi,
                                   int32_t *oj, float *oc, int64_t cap)
 {
-    const int64_t nl = team_min<Team, int64_t>(t, sc, sm, len, len,
-                                               [&](int64_t p) -> int64_t { return text[p] == '\n' ? p : len; });
-    int64_t fl = nl;
-    if (fl > 0 && text[fl - 1] == '\r') --fl;
+    // the first line is "MULTICUT", so its end is one of the next two bytes
     const char head[] = "MULTICUT";
-    bool ok = fl == 8;
+    bool ok = len >= 8;
     for (int k = 0; ok && k < 8; ++k) ok = text[k] == head[k];
-    if (!ok) return -1;
+    const int64_t nl = len > 8 && text[8] == '\r' ? 9 : 8;
+    if (!ok || (nl < len && text[nl] != '\n')) return -1;
     const int64_t s0 = nl + 1 < len ? nl + 1 : len;
     const int64_t body = len - s0;
     uint64_t mark = sc.arena.mark();
     int64_t *tpos = sc.arena.take<int64_t>(body / 2 + 2);
     uint32_t *tval = sc.arena.take<uint32_t>(body / 2 + 2);
     if (!sc.arena.ok()) return 0;
-    // token starts: a non-space byte after a space (or at the body's start)
-    const int64_t ntok = team_compact(
-        t, sc, sm, body,
-        [&](int64_t q) { return !is_space_char(text[s0 + q]) && (q == 0 || is_space_char(text[s0 + q - 1])); },
-        [&](int64_t q, int64_t k) { tpos[k] = s0 + q; });
+    // token starts: a non-space byte after a space (or at the body's start).
+    // 16 bytes at a time, from the 16-byte boundary at or before the body on:
+    // bits of a group's token starts.  (Byte by byte, and with a pass that
+    // looked for the end of the first line, the parse of 3.8 MB took 0.14 ms.)
+    const int64_t g0 = s0 - (int64_t)((uintptr_t)(text + s0) & 15);
+    auto starts = [=](int64_t g) -> uint32_t {
+        const int64_t p0 = g0 + 16 * g;
+        uint32_t space = 0;  // bit k + 1: byte p0 + k is a space or outside the body; bit 0: the byte before
+        if (p0 >= s0 && p0 + 16 <= len) {
+            const uint4 w = *reinterpret_cast<const uint4 *>(text + p0);
+            const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+                space |= is_space_char((char)((x[k >> 2] >> (8 * (k & 3))) & 255)) ? 2u << k : 0u;
+        } else {
+            for (int k = 0; k < 16; ++k)
+                space |= p0 + k < s0 || p0 + k >= len || is_space_char(text[p0 + k]) ? 2u << k : 0u;
+        }
+        space |= p0 <= s0 || is_space_char(text[p0 - 1]) ? 1u : 0u;
+        return ~(space >> 1) & space & 0xffffu;
+    };
+    const int64_t ntok = team_scan<Team, int64_t>(
+        t, sc, sm, (len - g0 + 15) / 16, [=](int64_t g) -> int64_t { return __popc(starts(g)); },
+        [=](int64_t g, int64_t k, int64_t c) {
+            if (c)
+                for (uint32_t m = starts(g); m; m &= m - 1) tpos[k++] = g0 + 16 * g + __ffs(m) - 1;
+        });
     // convert every token; the first one that fails ends the input
     const int64_t first_bad = team_min<Team, int64_t>(t, sc, sm, ntok, ntok, [&](int64_t k) -> int64_t {
         const char *p = text + tpos[k];

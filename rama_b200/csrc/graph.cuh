@@ -296,7 +296,8 @@ __device__ __forceinline__ bool team_sort_records(const Team &t, Scratch &sc, ch
 }
 
 // Walks the ordered records of this CTA's share in tiles held in shared
-// memory.  A tile is a window of 4 * blockDim records less BUCKET_SMALL: the
+// memory.  A tile is a window of kk * blockDim records less BUCKET_SMALL, kk = 4
+// for large lists and 1 or 2 where that many tiles still find a CTA each: the
 // CTA that holds a small bucket's first record has all of it in its window,
 // and orders it there (every record goes to the number of smaller keys in its
 // bucket; the records pass through registers).  Records of longer buckets are
@@ -304,7 +305,7 @@ __device__ __forceinline__ bool team_sort_records(const Team &t, Scratch &sc, ch
 //
 // visit(T, base, prev, mine) is called by every thread of the CTA once per
 // tile, for its records win[base + 32 k] (k < 4; position order over (k, lane)
-// within a warp's 128): prev[k] is the record before, mine[k] whether the
+// within a warp's 32 kk; those from kk on are nobody's): prev[k] is the record before, mine[k] whether the
 // position belongs to this CTA.  Two windows in turn, so that a tile's records
 // are read while slower warps still visit the last one's.
 template <class Rec>
@@ -332,12 +333,16 @@ __device__ __forceinline__ void team_record_tiles(const Team &t, char *sm, const
                                                   Visit visit)
 {
     constexpr int K = 4;
-    const int W = K * blockDim.x, TILE = W - BUCKET_SMALL;
+    // records a thread of this walk
+    const int kk = n <= t.nblocks() * (int64_t)(blockDim.x - BUCKET_SMALL)       ? 1
+                   : n <= t.nblocks() * (int64_t)(2 * blockDim.x - BUCKET_SMALL) ? 2
+                                                                                 : K;
+    const int W = kk * blockDim.x, TILE = W - BUCKET_SMALL;
     const int64_t ntiles = (n + TILE - 1) / TILE;
     const int64_t per = (ntiles + t.nblocks() - 1) / t.nblocks();
     const int64_t t0 = (int64_t)t.block() * per;
     const int64_t t1 = t0 + per < ntiles ? t0 + per : ntiles;
-    const int base = warp_in_block() * 32 * K + lane_id();
+    const int base = warp_in_block() * 32 * kk + lane_id();
     int64_t a = t0 < t1 ? rec_owned_from(R, t0 * TILE, n) : n;
     int flip = 0;
     for (int64_t tile = t0; tile < t1; ++tile, flip ^= 1) {
@@ -357,13 +362,14 @@ __device__ __forceinline__ void team_record_tiles(const Team &t, char *sm, const
             e[k] = R.start[rec_bucket(r[k]) + 1];
         }
 #pragma unroll
-        for (int k = 0; k < K; ++k) win[base + 32 * k] = r[k];
+        for (int k = 0; k < K; ++k)
+            if (k < kk) win[base + 32 * k] = r[k];
         // the next tile's records on their way to L2 (a line per 128 bytes)
         if (tile + 1 < t1 && lane_id() % (128 / (int)sizeof(Rec)) == 0) {
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 const int64_t p = p0 + TILE + base + 32 * k;
-                if (p < n) asm volatile("prefetch.L2 [%0];" ::"l"(R.rec + p));
+                if (k < kk && p < n) asm volatile("prefetch.L2 [%0];" ::"l"(R.rec + p));
             }
         }
         __syncthreads();
@@ -373,7 +379,7 @@ __device__ __forceinline__ void team_record_tiles(const Team &t, char *sm, const
             const int i = base + 32 * k;
             const int64_t p = p0 + i;
             dst[k] = i;
-            if (p >= a && p < b && e[k] - s[k] <= BUCKET_SMALL) {
+            if (k < kk && p >= a && p < b && e[k] - s[k] <= BUCKET_SMALL) {
                 const auto key = rec_key(r[k]);
                 const int f = (int)(s[k] - p0), l = (int)(e[k] - p0);
                 int rank = 0;
@@ -388,7 +394,7 @@ __device__ __forceinline__ void team_record_tiles(const Team &t, char *sm, const
 #pragma unroll
         for (int k = 0; k < K; ++k) {
             const int64_t p = p0 + base + 32 * k;
-            if (p >= a && p < b) win[dst[k]] = r[k];
+            if (k < kk && p >= a && p < b) win[dst[k]] = r[k];
         }
         __syncthreads();
         RecTile<Rec> T;
@@ -403,7 +409,7 @@ __device__ __forceinline__ void team_record_tiles(const Team &t, char *sm, const
         for (int k = 0; k < K; ++k) {
             const int i = base + 32 * k;
             const int64_t p = p0 + i;
-            mine[k] = p >= a && p < b;
+            mine[k] = k < kk && p >= a && p < b;
             prev[k] = !mine[k] ? none : (p > a ? win[i - 1] : (p > 0 ? R.rec[p - 1] : none));
         }
         visit(T, base, prev, mine);

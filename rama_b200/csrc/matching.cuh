@@ -131,17 +131,13 @@ __device__ __noinline__ int32_t matching_contraction_map(const Team &t, Scratch 
                 const int w = warp_in_block(), nw = blockDim.x >> 5;
                 if (lane_id() == 31) wsum[w] = incl;
                 __syncthreads();
-                if (threadIdx.x == 0) {
-                    int tl = 0, tt = 0;
-                    for (int q = 0; q < nw; ++q) {
-                        const int x = wsum[q];
-                        wsum[32 + q] = tl;
-                        wsum[64 + q] = tt;
-                        tl += x & 0xffff;
-                        tt += x >> 16;
-                    }
-                    wsum[96] = tl ? atomicAdd(&cnt_next[0], tl) : 0;
-                    wsum[97] = tt ? atomicAdd(&cnt_next[1], tt) : 0;
+                if (w == 0) {  // (one thread walking the warps' sums held up the CTA for some 500 cycles a tile)
+                    const int x = lane_id() < nw ? wsum[lane_id()] : 0;
+                    const int upto = warp_incl_scan(x), all = __shfl_sync(FULL, upto, 31);
+                    wsum[32 + lane_id()] = (upto - x) & 0xffff;
+                    wsum[64 + lane_id()] = (upto - x) >> 16;
+                    const int mine = lane_id() == 0 ? all & 0xffff : all >> 16;
+                    if (lane_id() < 2) wsum[96 + lane_id()] = mine ? atomicAdd(&cnt_next[lane_id()], mine) : 0;
                 }
                 __syncthreads();
                 int lbase = wsum[96] + wsum[32 + w] + ((incl - packed) & 0xffff);

@@ -307,7 +307,7 @@ def run_ours(args, rank, world, local):
     return line
 
 
-KERNEL_OF_TEAM = {1: "k_solve_cta", 2: "k_solve_grid", 3: "k_solve_mixed"}
+KERNEL_OF_TEAM = {1: "k_solve_cta_alone", 2: "k_solve_grid", 3: "k_solve_cluster_alone"}
 
 
 def phase_roofline(stats, hbm):

@@ -116,6 +116,7 @@ struct rama_context {
     int cta_small_per_sm = 0;  // co-resident CTAs of k_solve_cta_small per SM
     int grid_per_sm_max = 0;  // occupancy maximum of k_solve_grid per SM
     int cluster_cap[17] = {};  // co-resident clusters of k_solve_mixed by cluster size (0: not known yet)
+    int cluster_alone_cap[17] = {};  // ... of k_solve_cluster_alone
     rama_tuning tune{};
     int parse_ctas = 0;   // co-resident CTAs of k_parse_grid
     char *p_text = nullptr;  // device copy of text for rama_parse_multicut_host
@@ -216,15 +217,18 @@ uint64_t ws_slice(int64_t n_edges, float tri_factor = 2.0f)
 // Launches the solve of the instances already in h->d_inst (queue order in
 // h->d_order).  team 2: one instance on the cooperative grid; otherwise the
 // first `ncluster` queue entries go to cluster teams and the rest to CTAs.
-// co-resident clusters of k_solve_mixed for a cluster size (0 if none fits)
-int cluster_capacity(rama_context *h, int size)
+// co-resident clusters of k_solve_mixed (alone: k_solve_cluster_alone) for a
+// cluster size (0 if none fits)
+int cluster_capacity(rama_context *h, int size, bool alone = false)
 {
     if (size < 1 || size > 16) return 0;
-    if (!h->cluster_cap[size]) {
-        if (size > 8 && cudaFuncSetAttribute((const void *)k_solve_mixed,
-                                             cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    int &cap = alone ? h->cluster_alone_cap[size] : h->cluster_cap[size];
+    const void *kernel = alone ? (const void *)k_solve_cluster_alone : (const void *)k_solve_mixed;
+    if (!cap) {
+        if (size > 8 &&
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
-            h->cluster_cap[size] = -1;
+            cap = -1;
             return 0;
         }
         cudaLaunchConfig_t cfg = {};
@@ -239,13 +243,13 @@ int cluster_capacity(rama_context *h, int size)
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int ncl = 0;
-        if (cudaOccupancyMaxActiveClusters(&ncl, (void *)k_solve_mixed, &cfg) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveClusters(&ncl, kernel, &cfg) != cudaSuccess) {
             cudaGetLastError();
             ncl = 0;
         }
-        h->cluster_cap[size] = ncl > 0 ? ncl : -1;
+        cap = ncl > 0 ? ncl : -1;
     }
-    return h->cluster_cap[size] > 0 ? h->cluster_cap[size] : 0;
+    return cap > 0 ? cap : 0;
 }
 
 // The cluster size of a launch of `ncluster` instances for clusters, the
@@ -271,7 +275,8 @@ int launch_solve(rama_context *h, int32_t count, int team, cudaStream_t st, int3
         void *args[] = {&L};
         const int per_sm = edges < h->tune.grid_small_max ? h->tune.grid_small_ctas_per_sm
                                                                 : h->tune.grid_ctas_per_sm;
-        CU(cudaLaunchCooperativeKernel((void *)k_solve_grid, dim3(per_sm * h->sms), dim3(THREADS), args, SMEM, st));
+        const void *k = per_sm == 1 ? (const void *)k_solve_grid_alone : (const void *)k_solve_grid;
+        CU(cudaLaunchCooperativeKernel(k, dim3(per_sm * h->sms), dim3(THREADS), args, SMEM, st));
     } else if (ncluster > 0) {
         const int csz = cluster_size(h, ncluster, batch, edges);
         const int64_t want = (int64_t)ncluster * csz + (count - ncluster);
@@ -291,11 +296,16 @@ int launch_solve(rama_context *h, int32_t count, int team, cudaStream_t st, int3
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        CU(cudaLaunchKernelEx(&cfg, k_solve_mixed, L));
+        if (count == 1 && cluster_capacity(h, csz, true) > 0)
+            CU(cudaLaunchKernelEx(&cfg, k_solve_cluster_alone, h->d_inst));
+        else
+            CU(cudaLaunchKernelEx(&cfg, k_solve_mixed, L));
     } else {
         CU(cudaMemsetAsync(h->d_queue, 0, sizeof(int32_t), st));
         CtaLaunch L{h->d_inst, h->d_order, count, h->d_queue};
-        if (h->tune.cta_threads == THREADS_SMALL) {
+        if (count == 1 && h->tune.cta_threads == THREADS) {
+            k_solve_cta_alone<<<1, THREADS, SMEM, st>>>(h->d_inst);
+        } else if (h->tune.cta_threads == THREADS_SMALL) {
             const int ctas = std::max(1, std::min<int>(count, h->sms * h->cta_small_per_sm));
             k_solve_cta_small<<<ctas, THREADS_SMALL, SMEM_SMALL, st>>>(L);
         } else {
@@ -483,6 +493,8 @@ int rama_create(int device, uint64_t workspace_bytes, rama_handle *out)
     h->sms = p.multiProcessorCount;
     // the sort stages a tile in shared memory: more than the default 48 KB
     for (const void *k : {(const void *)k_solve_grid, (const void *)k_solve_cta, (const void *)k_solve_mixed,
+                          (const void *)k_solve_grid_alone, (const void *)k_solve_cta_alone,
+                          (const void *)k_solve_cluster_alone,
                           (const void *)k_step_grid, (const void *)k_step_cta, (const void *)k_objective,
                           (const void *)k_parse_grid})
         CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));

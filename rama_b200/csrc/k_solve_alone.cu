@@ -1,0 +1,12 @@
+// k_solve_alone.cu -- one instance on one cluster, with the registers of a
+// whole SM per CTA (see kernels.cuh).
+#include "kernels.cuh"
+
+using namespace rama;
+
+__global__ void __launch_bounds__(THREADS, 1) k_solve_cluster_alone(Instance *io)
+{
+    extern __shared__ __align__(16) char sm[];
+    ClusterTeam t;
+    solve_instance(t, sm, make_scratch(io->ws, io->ws_bytes), io);
+}

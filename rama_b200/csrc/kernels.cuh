@@ -93,6 +93,13 @@ __global__ void __launch_bounds__(rama::THREADS, 2) k_solve_cta(rama::CtaLaunch 
 __global__ void __launch_bounds__(rama::THREADS_SMALL, 3) k_solve_cta_small(rama::CtaLaunch L);
 __global__ void __launch_bounds__(rama::THREADS, 2) k_solve_mixed(rama::MixedLaunch L);
 __global__ void __launch_bounds__(rama::THREADS, 2) k_solve_grid(rama::GridLaunch L);
+// One instance with one CTA per SM: 128 registers a thread instead of 64, so
+// that the phases keep their batches in registers instead of on the stack.
+// Used where a second CTA per SM gives nothing: one CTA or one cluster alone,
+// and the grids of one CTA per SM.
+__global__ void __launch_bounds__(rama::THREADS, 1) k_solve_cta_alone(rama::Instance *io);
+__global__ void __launch_bounds__(rama::THREADS, 1) k_solve_cluster_alone(rama::Instance *io);
+__global__ void __launch_bounds__(rama::THREADS, 1) k_solve_grid_alone(rama::GridLaunch L);
 __global__ void __launch_bounds__(rama::THREADS, 2) k_parse_grid(rama::ParseLaunch L);
 __global__ void __launch_bounds__(rama::THREADS, 2) k_step_cta(rama_step_args *a, char *ws, uint64_t bytes);
 __global__ void __launch_bounds__(rama::THREADS, 2) k_step_grid(rama_step_args *a, char *ws, uint64_t bytes);

@@ -819,39 +819,9 @@ __device__ __forceinline__ float rsum_serial(int n, Get v)
     return (float)r;
 }
 
-// The same sum by one thread for n <= 8 values at p[0, n): the loads are
-// independent and issued together, then a fixed tree over 8 values padded
-// with +0.0.  Adding an exact zero changes no sum, so this equals
-// rsum_serial(n, p[k]).
+// runs up to this length are summed in the pass over all edges, longer ones
+// from a list
 constexpr int RSUM_THREAD_MAX = 8;
-
-__device__ __forceinline__ float rsum_upto8(const float *p, int n)
-{
-    double x[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = k < n ? __dadd_rn(0.0, (double)p[k]) : 0.0;
-    const double a = __dadd_rn(__dadd_rn(x[0], x[1]), __dadd_rn(x[2], x[3]));
-    const double b = __dadd_rn(__dadd_rn(x[4], x[5]), __dadd_rn(x[6], x[7]));
-    return (float)__dadd_rn(a, b);
-}
-
-// The same sum by one thread for n <= 32 values at p[0, n): the complete
-// tree over 32 lanes (+0.0 in the empty ones) is the pairwise sum of four
-// complete trees over 8 (each as in rsum_upto8), so this equals
-// rsum_serial(n, p[k]); the loads of a group of 8 are issued together.
-__device__ __forceinline__ float rsum_upto32(const float *p, int n)
-{
-    double g[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        double x[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) x[k] = 8 * q + k < n ? __dadd_rn(0.0, (double)p[8 * q + k]) : 0.0;
-        g[q] = __dadd_rn(__dadd_rn(__dadd_rn(x[0], x[1]), __dadd_rn(x[2], x[3])),
-                         __dadd_rn(__dadd_rn(x[4], x[5]), __dadd_rn(x[6], x[7])));
-    }
-    return (float)__dadd_rn(__dadd_rn(g[0], g[1]), __dadd_rn(g[2], g[3]));
-}
 
 // Sums of more than RSUM_CHUNK values are defined by chunks: each chunk of
 // RSUM_CHUNK consecutive values is summed as above (kept in double), and the

@@ -218,8 +218,8 @@ typedef struct {
     int32_t grid_small_ctas_per_sm; /* ... and of one of fewer than grid_small_max edges */
     int64_t grid_small_max;
     int32_t cluster_ctas;        /* CTAs of a cluster team: 2, 4, 8 or 16; 8, the starting value, stands for 16
-                                    where the clusters have the GPU to themselves (8 for the smallest
-                                    graphs) down to 4 in a large batch */
+                                    where the clusters have the GPU to themselves, down to 4 in a large
+                                    batch */
     int64_t single_cluster_min;  /* a single solve of at least this many edges runs on a cluster ... */
     int64_t single_grid_min;     /* ... and from this many on on the whole GPU (else on one CTA); both count
                                     twice for solves without a dual */

@@ -35,17 +35,15 @@ constexpr int64_t DEFAULT_SINGLE_CLUSTER_MIN = 4000;  // a single solve from thi
 constexpr int64_t DEFAULT_SINGLE_GRID_MIN = 100000;   // ... and from this size on on the whole GPU
 // Solves without a dual have a fraction of the passes' work per edge, so they
 // change teams at twice these sizes.  Measured (ms, one CTA / cluster of 16 /
-// whole GPU): region graphs without a dual, 5,822 edges 0.88 / 1.03 / 1.49,
-// 8,785 edges 0.98 / 0.98 / 1.43, 208,942 edges - / 1.65 / 1.73; with, 2,874
-// edges 2.26 / 2.26 / 3.46, 5,822 edges 3.43 / 2.63 / 4.14, 89,308 edges
-// - / 4.62 / 5.02, 208,942 edges - / 7.10 / 5.31.
-constexpr int64_t WIDE_CLUSTER_MIN = 7000;  // single clusters below this size take 8 CTAs: 2.57 and 2.63 ms at 5,822
-                                            // edges with a dual, 2.15 and 2.05 at 8,064
-// One CTA per SM solves graphs of up to 1.5 M edges sooner (fewer partial
-// results to fold; 2.83 ms against 3.24 at 753,664 edges, 10.9 against 11.4 at
-// 1.14 M), two larger ones (4.49 against 4.70 at 3.06 M, 17.9 against 24.8 at
-// 24.8 M).
-constexpr int64_t DEFAULT_GRID_SMALL_MAX = 1500000;
+// whole GPU): region graphs without a dual, 5,822 edges 0.65 / 0.75 / 1.18,
+// 8,785 edges 0.75 / 0.76 / 1.15, 208,942 edges - / 1.37 / 1.39; with, 2,874
+// edges 1.57 / 1.73 / 2.87, 5,822 edges 2.40 / 1.99 / 3.30, 89,308 edges
+// - / 3.85 / 3.97, 149,106 edges - / 4.94 / 4.36.
+// One CTA per SM (with twice the registers) solves graphs of up to about 3 M
+// edges sooner, two larger ones.  Measured (ms, one / two): 753,664 edges 2.46 /
+// 3.25, 1.14 M 8.96 / 11.2, 2.63 M 17.6 / 18.8, 3.06 M 4.12 / 4.47, 3.30 M 66.2 /
+// 60.2, 11.3 M 11.1 / 9.7, 24.8 M 22.4 / 18.1.
+constexpr int64_t DEFAULT_GRID_SMALL_MAX = 3200000;
 constexpr int64_t DEFAULT_BATCH_CLUSTER_MIN = 10000;  // smaller batch instances always run on one CTA
 constexpr float DEFAULT_BATCH_CLUSTER_SHARE = 1.0f;   // ... larger ones on a cluster above this many
                                                       // times the batch's edges per CTA (256 region graphs
@@ -252,23 +250,22 @@ int cluster_capacity(rama_context *h, int size, bool alone = false)
     return cap > 0 ? cap : 0;
 }
 
-// The cluster size of a launch of `ncluster` instances for clusters, the
-// largest of `edges` edges.  One solve finishes soonest on the largest
-// cluster; where they do not all run at once the clusters' CTA time counts.
-// Measured (ms): region graph of 59,436 edges PD on 4, 8, 16 CTAs 7.88, 5.29,
-// 4.05; 12 graphs of 500 to 20,000 nodes on 4 and 16 7.00, 4.22; 40 of them
-// 6.12, 7.62; 256 of them on 4, 8, 16 15.8, 21.8, 34.2.
-int cluster_size(rama_context *h, int32_t ncluster, bool batch, int64_t edges)
+// The cluster size of a launch of `ncluster` instances for clusters.  One
+// solve finishes soonest on the largest cluster; where they do not all run at
+// once the clusters' CTA time counts.  Measured (ms): region graph of 59,436
+// edges PD on 4 and 16 CTAs 5.98, 3.09; 5,822 edges PD on 8 and 16 2.10, 1.99;
+// 12 graphs of 500 to 20,000 nodes on 4 and 16 7.00, 4.22; 40 of them 6.12,
+// 7.62; 256 of them on 4, 8, 16 15.8, 21.8, 34.2.
+int cluster_size(rama_context *h, int32_t ncluster)
 {
     if (h->tune.cluster_ctas != DEFAULT_CLUSTER_CTAS) return h->tune.cluster_ctas;
-    if (ncluster * SINGLE_CLUSTER_CTAS <= h->sms && (batch || edges >= WIDE_CLUSTER_MIN) &&
-        cluster_capacity(h, SINGLE_CLUSTER_CTAS) > 0)
+    if (ncluster * SINGLE_CLUSTER_CTAS <= h->sms && cluster_capacity(h, SINGLE_CLUSTER_CTAS) > 0)
         return SINGLE_CLUSTER_CTAS;
     return ncluster * DEFAULT_CLUSTER_CTAS <= h->sms ? DEFAULT_CLUSTER_CTAS : BATCH_CLUSTER_CTAS;
 }
 
 int launch_solve(rama_context *h, int32_t count, int team, cudaStream_t st, int32_t ncluster = 0,
-                 int64_t edges = 0, bool batch = false)
+                 int64_t edges = 0)
 {
     if (team == 2) {
         GridLaunch L{h->d_inst, h->ws, h->ws_bytes};
@@ -278,7 +275,7 @@ int launch_solve(rama_context *h, int32_t count, int team, cudaStream_t st, int3
         const void *k = per_sm == 1 ? (const void *)k_solve_grid_alone : (const void *)k_solve_grid;
         CU(cudaLaunchCooperativeKernel(k, dim3(per_sm * h->sms), dim3(THREADS), args, SMEM, st));
     } else if (ncluster > 0) {
-        const int csz = cluster_size(h, ncluster, batch, edges);
+        const int csz = cluster_size(h, ncluster);
         const int64_t want = (int64_t)ncluster * csz + (count - ncluster);
         const int64_t cap = (int64_t)std::max(1, cluster_capacity(h, csz)) * csz;
         const int64_t ctas = (std::min(want, cap) + csz - 1) / csz * csz;
@@ -745,7 +742,7 @@ int rama_batch_launch(rama_handle h, const int32_t *d_i, const int32_t *d_j, con
     if (count == 1 && opts[0].team == 2)
         rc = launch_solve(h, 1, 2, st, 0, h->b_in[0].n);
     else
-        rc = launch_solve(h, count, 1, st, ncluster, 0, true);
+        rc = launch_solve(h, count, 1, st, ncluster);
     if (rc) return rc;
     CU(cudaEventRecord(h->ev1, st));
     CU(cudaMemcpyAsync(h->b_host, h->d_inst, sizeof(Instance) * count, cudaMemcpyDeviceToHost, st));
@@ -811,7 +808,7 @@ int rama_batch_wait(rama_handle h, int64_t *num_labels, double *lbs, int32_t *st
         CU(cudaMemcpyAsync(h->d_inst, sub.data(), sizeof(Instance) * sub.size(), cudaMemcpyHostToDevice, h->b_stream));
         CU(cudaMemcpyAsync(h->d_order, order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice,
                            h->b_stream));
-        rc = launch_solve(h, (int32_t)sub.size(), 1, h->b_stream, ncl, 0, true);
+        rc = launch_solve(h, (int32_t)sub.size(), 1, h->b_stream, ncl);
         if (rc) return rc;
         CU(cudaMemcpyAsync(sub.data(), h->d_inst, sizeof(Instance) * sub.size(), cudaMemcpyDeviceToHost, h->b_stream));
         CU(cudaStreamSynchronize(h->b_stream));

@@ -488,10 +488,13 @@ __device__ __noinline__ Graph graph_from_edges(const Team &t, Scratch &sc, char 
                 dup |= prev[k].w == r.w && prev[k].x == r.x;
             }
     });
-    team_fold_maxi_minf(t, sc, sm, dup, mn);
-    // dims as in dCOO::init (src/dCOO.cu:47-51); the largest endpoint is a column
+    // dims as in dCOO::init (src/dCOO.cu:47-51); the largest endpoint is a
+    // column.  The last record is read before the fold's team sync: the caller
+    // hands its memory on with no sync of its own (the tile pass leaves the
+    // records of R as they are).
     g.cols = g.ecols = mx + 1;
     g.rows = uread(&R.rec[n - 1].w) + 1;
+    team_fold_maxi_minf(t, sc, sm, dup, mn);
     g.cmin = mn;
     g.uniq = dup == 0;
     sc.arena.top = top;
@@ -951,10 +954,10 @@ __device__ __noinline__ Graph graph_contract(const Team &t, Scratch &sc, char *,
         }
         for (; k < kept; k += S) put(k, tends[first + k], tcost[first + k]);
     }
+    h.rows = uread(&R.rec[n - 1].w) + 1;  // before the fold's team sync, after which the records' memory is handed on
     team_fold_maxi_minf(t, sc, sm, mc, mn);
     prof_mark(t, sc, PH_CONTRACT_RUNS);
     h.n = nk;
-    h.rows = uread(&R.rec[n - 1].w) + 1;
     h.cols = (mc > dmax ? mc : dmax) + 1;
     h.cmin = nk > 0 ? mn : unknown_cost();
     h.ecols = mc + 1;

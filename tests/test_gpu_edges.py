@@ -76,6 +76,19 @@ def test_tiles_of_nodes_and_edges(solver, oracle, nodes, team):
 
 
 @pytest.mark.parametrize("team", (1, 2, 3))
+@pytest.mark.parametrize("stride", (2, 3, 5, 8))
+@pytest.mark.parametrize("edges", (2, 700, 30000))
+def test_more_nodes_than_edges(solver, oracle, edges, stride, team):
+    """Edges that share no node, node ids with gaps between them: lists of
+    vertices that reach beyond what the sort of the edges took of the
+    workspace."""
+    k = np.random.default_rng(edges + stride).permutation(edges).astype(np.int32) * stride
+    c = np.random.default_rng(stride).normal(0.1, 1.0, edges).astype(np.float32)
+    for mode in ("P", "PD", "PD+", "D"):
+        same_as_oracle(solver, oracle, k, k + 1, c, mode, team)
+
+
+@pytest.mark.parametrize("team", (1, 2, 3))
 @pytest.mark.parametrize("factor", (0.01, 0.3, 1.0, 5.0))
 def test_truncated_cycles(solver, oracle, factor, team):
     """Few emissions an expansion, and some with more than the histogram's

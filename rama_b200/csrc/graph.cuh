@@ -14,7 +14,7 @@ struct Graph {
     int32_t rows, cols;  // dCOO::rows_ / cols_
     float cmin;          // smallest cost of an edge with row != col (NaN: not known)
     int32_t ecols;       // largest column of an edge + 1 (rows / cols keep dims from before the diagonal went)
-    int uniq;            // no two edges share both ends (0: not known)
+    int uniq;            // no two edges share both ends and none is a self-loop (0: not known)
     __device__ __forceinline__ int32_t max_dim() const { return rows > cols ? rows : cols; }
 };
 
@@ -86,13 +86,14 @@ __device__ void graph_set_dims(const Team &t, Scratch &sc, char *sm, Graph &g)
     g.cmin = mn;
 }
 
-// whether no two neighbours of the sorted edge list share both ends
+// whether no two neighbours of the sorted edge list share both ends, and no
+// edge is a self-loop (which stands twice in its vertex's list of neighbours)
 template <class Team>
 __device__ bool graph_is_simple(const Team &t, Scratch &sc, char *sm, const Graph &g)
 {
     const int32_t *row = g.row, *col = g.col;
     return team_sum<Team, int64_t>(t, sc, sm, g.n, [=](int64_t e) -> int64_t {
-               return e > 0 && row[e] == row[e - 1] && col[e] == col[e - 1];
+               return row[e] == col[e] || (e > 0 && row[e] == row[e - 1] && col[e] == col[e - 1]);
            }) == 0;
 }
 

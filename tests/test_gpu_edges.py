@@ -102,6 +102,22 @@ def test_truncated_cycles(solver, oracle, factor, team):
     same_as_oracle(solver, oracle, i, j, c, "D", team, tri_memory_factor=factor)
 
 
+@pytest.mark.parametrize("team", (1, 2))
+@pytest.mark.parametrize("seed", range(6))
+def test_cycles_beside_self_loops(solver, oracle, seed, team):
+    """The cycle search alone takes graphs with self-loops, whose vertices
+    stand twice in their own lists of neighbours."""
+    i, j, c = instances.random_graph(60, 6, seed=seed)
+    k = np.arange(60, dtype=np.int32)
+    loops = np.random.default_rng(seed).uniform(0.1, 1.0, 60).astype(np.float32)
+    G = oracle.Graph.from_edges(np.concatenate([i, k]), np.concatenate([j, k]), np.concatenate([c, loops]))
+    row, col, cost = G.arrays()
+    for length in (3, 4, 5):
+        want, raw = oracle.conflicted_cycles(G, length, 5.0)
+        got, graw = solver.step_cycles(row, col, cost, *G.dims, length, 5.0, team=team)
+        assert graw == raw and np.array_equal(got, want)
+
+
 @pytest.mark.parametrize("mode", ("P", "PD"))
 def test_clusters_of_every_size(solver, oracle, mode):
     """Batches of few, some and many instances for clusters, and one alone on

@@ -491,6 +491,13 @@ __device__ __forceinline__ void expansion_stage(const Team &t, Scratch &sc, char
         const int64_t tot = team_total<Team, int64_t>(t, sc, sm, mine);
         const int64_t start = count;
         const int64_t rem = budget - start;
+        if (tot > rem && rem == 0) {
+            // No room for any of them.  The histogram must not be read here:
+            // nothing would sync between that and the caller's next writes to
+            // this stage's workspace.
+            count = budget + 1;
+            break;
+        }
         // round-robin when the chunk does not fit: the largest K with
         // sum_q min(count_q, K) <= rem, and `extra` expansions keep one more.
         // K from a histogram of the counts; by bisection over sums where it
@@ -575,7 +582,7 @@ __device__ __forceinline__ void expansion_stage(const Team &t, Scratch &sc, char
             extra = rem - slo;
             __syncthreads();
         }
-        if (tot > 0 && rem > 0) {
+        if (tot > 0) {  // (and rem > 0)
             // positions: one scan of (kept below K) << 25 | (has more than K);
             // count_q is replaced by the number it keeps
             team_scan<Team, int64_t>(

@@ -102,6 +102,16 @@ def test_truncated_cycles(solver, oracle, factor, team):
     same_as_oracle(solver, oracle, i, j, c, "D", team, tri_memory_factor=factor)
 
 
+@pytest.mark.parametrize("team", (1, 2, 3))
+@pytest.mark.parametrize("pages", (1, 5, 300))
+def test_no_room_for_any_triangle(solver, oracle, pages, team):
+    """A budget of no triangle, and one that the first cycle length fills."""
+    i, j, c = book(pages, pages)
+    for mode in ("PD", "PD+", "D"):
+        for factor in (0.0, 0.1, 0.5 * pages, float(pages)):
+            same_as_oracle(solver, oracle, i, j, c, mode, team, tri_memory_factor=factor)
+
+
 @pytest.mark.parametrize("team", (1, 2))
 @pytest.mark.parametrize("seed", range(6))
 def test_cycles_beside_self_loops(solver, oracle, seed, team):

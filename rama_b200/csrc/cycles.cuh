@@ -351,6 +351,9 @@ __device__ __noinline__ bool attractive_lists(const Team &t, Scratch &sc, char *
     t.sync();
     m2 = team_bucket_starts(t, sc, sm, nrows, off, L, [](int64_t, int32_t, int32_t) {});
     if (L.has_big()) {
+        // every thread has seen it before the caller, which writes to this
+        // memory next, goes on
+        t.sync();
         sc.arena.release(m);
         return false;
     }

@@ -53,6 +53,21 @@ def test_neighbours_of_one_vertex(solver, oracle, degree, team):
 
 
 @pytest.mark.parametrize("team", (1, 2, 3))
+@pytest.mark.parametrize("gap", (1, 11))
+def test_hub_among_unused_ids(solver, oracle, gap, team):
+    """More attractive neighbours than the list sort takes, with and without
+    gaps in the node ids."""
+    degree = 4200
+    rng = np.random.default_rng(gap)
+    k = np.arange(1, degree + 1, dtype=np.int32)
+    i = np.concatenate([np.zeros(degree, np.int32), k[:-1]]) * gap
+    j = np.concatenate([k, k[1:]]) * gap
+    c = np.concatenate([rng.uniform(0.1, 1.0, degree), rng.normal(-0.2, 1.0, degree - 1)]).astype(np.float32)
+    for mode in ("PD", "D"):
+        same_as_oracle(solver, oracle, i, j, c, mode, team)
+
+
+@pytest.mark.parametrize("team", (1, 2, 3))
 @pytest.mark.parametrize("copies", (2, 3, 8, 33, 64, 65, 200))
 def test_parallel_edges(solver, oracle, copies, team):
     """Every edge `copies` times: neighbour lists with repeated entries and

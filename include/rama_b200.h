@@ -226,8 +226,8 @@ typedef struct {
     int64_t batch_cluster_min;   /* batch instances below this size always run on one CTA; larger ones on */
     float batch_cluster_share;   /* a cluster when they hold more than this many times the batch's edges
                                     per CTA */
-    int32_t cta_threads;         /* threads of a CTA that solves instances alone: 512 (two per SM) or
-                                    256 (three per SM, more instances in flight) */
+    int32_t cta_threads;         /* threads of a CTA in a batch without cluster instances: 512 (two per SM)
+                                    or 256 (three per SM, more instances in flight) */
 } rama_tuning;
 int rama_get_tuning(rama_handle h, rama_tuning *out);
 /* RAMA_ERR_INVALID_ARG for a value outside its range or a cluster size that
@@ -235,6 +235,9 @@ int rama_get_tuning(rama_handle h, rama_tuning *out);
 int rama_set_tuning(rama_handle h, const rama_tuning *t);
 
 int rama_get_stats(rama_handle h, rama_stats *out);
+/* The name of the kernel that the last solve or batch on this handle launched
+ * ("" before the first). */
+const char *rama_solve_kernel(rama_handle h);
 const char *rama_last_error(void);
 
 /* Objective of a labelling: sum of the costs of edges whose endpoints carry

@@ -111,7 +111,7 @@ class StepArgs(C.Structure):
 EXPORTS = ("rama_options_init", "rama_create", "rama_destroy", "rama_solve", "rama_solve_host", "rama_get_timeline",
            "rama_solve_batch", "rama_batch_launch", "rama_batch_poll", "rama_batch_wait", "rama_get_stats",
            "rama_last_error", "rama_objective", "rama_step", "rama_solve_small_static", "rama_parse_multicut",
-           "rama_parse_multicut_host", "rama_get_tuning", "rama_set_tuning")
+           "rama_parse_multicut_host", "rama_get_tuning", "rama_set_tuning", "rama_solve_kernel")
 
 _lib = None
 _lock = threading.Lock()
@@ -156,6 +156,8 @@ def load():
         L.rama_step.argtypes = [P, C.POINTER(StepArgs), P]
         L.rama_get_tuning.argtypes = [P, C.POINTER(RamaTuning)]
         L.rama_set_tuning.argtypes = [P, C.POINTER(RamaTuning)]
+        L.rama_solve_kernel.restype = C.c_char_p
+        L.rama_solve_kernel.argtypes = [P]
         _lib = L
         return L
 
@@ -207,6 +209,10 @@ class Handle:
         t = RamaTuning()
         check(load().rama_get_tuning(self.h, C.byref(t)))
         return t
+
+    def solve_kernel(self) -> str:
+        """The kernel that the last solve or batch launched."""
+        return load().rama_solve_kernel(self.h).decode()
 
     def set_tuning(self, t: RamaTuning):
         check(load().rama_set_tuning(self.h, C.byref(t)))

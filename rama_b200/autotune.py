@@ -18,10 +18,10 @@ built-in choices are guesses; this module measures them on the device:
   CTA to a cluster and from a cluster to the whole GPU -- each team is timed
   on graphs of increasing size and the switch goes to the first size at which
   the larger team wins;
-* batch_cluster_min / batch_cluster_share / cta_threads: which instances of
-  a batch get a cluster, and whether the instances solved alone take CTAs of
-  512 threads (two per SM) or 256 (three per SM), timed together on a batch
-  of 256 Delaunay graphs of uneven size.
+* cta_threads: whether a batch without cluster instances runs on CTAs of 512
+  threads (two per SM) or 256 (three per SM), timed on such a batch;
+* batch_cluster_min / batch_cluster_share: which instances of a batch get a
+  cluster, timed on a batch of 256 Delaunay graphs of uneven size.
 
 Every trial solve's labels and bound are checked to equal the first trial's:
 a tuning never changes a result, and the tuner fails loudly if one would.
@@ -244,27 +244,34 @@ def tune(device: int = 0, budget_s: float = 60.0, quick: bool = False) -> dict:
     tables["single"] = {"edges": sizes, "cta_ms": cta, "cluster_ms": clu, "grid_ms": grd}
     tr.set(**chosen)
 
+    # the CTA size of batches without cluster instances (the only launches it
+    # changes), on a batch of small graphs
+    batch = I.delaunay_batch(count=400 if not quick else 40, nmin=300, nmax=3000, seed=12)
+    tt = {}
+    for threads in (512, 256):
+        tr.set(**{**chosen, "cta_threads": threads, "batch_cluster_min": 1 << 40})
+        tt[threads] = tr.batch("small", batch, "PD")
+    chosen["cta_threads"] = pick_fastest(tt)
+    tables["cta_threads"] = tt
+    tr.set(**chosen)
+
     # batches: which instances get a cluster, on a batch large enough that
     # many clusters and CTAs run side by side (the cluster size that is best
     # for one solve alone need not be best there: both are tried, and the
-    # batch decides); and the CTA size of the instances that run alone (a
-    # batch without cluster instances runs on the per-instance CTA kernel of
-    # that size)
+    # batch decides)
     batch = I.delaunay_batch(count=256 if not quick else 24, nmin=500, nmax=20000, seed=11)
     csizes = [chosen["cluster_ctas"]] + [c for c in tc if c != chosen["cluster_ctas"] and c == base["cluster_ctas"]]
     tb = {}
     for csz in csizes:
-        for threads in (512, 256):
-            for bmin, share in ((10000, 1.0), (20000, 1.5), (20000, 3.0), (40000, 1.5), (1 << 40, 1.5)):
-                if time.perf_counter() - t0 > budget_s and tb:
-                    break
-                tr.set(**{**chosen, "cluster_ctas": csz, "batch_cluster_min": bmin, "batch_cluster_share": share,
-                          "cta_threads": threads})
-                tb[(bmin, share, threads, csz)] = tr.batch("batch", batch, "PD")
-    bmin, share, threads, csz = pick_fastest(tb)
-    chosen["batch_cluster_min"], chosen["batch_cluster_share"], chosen["cta_threads"] = bmin, share, threads
+        for bmin, share in ((10000, 1.0), (20000, 1.5), (20000, 3.0), (40000, 1.5), (1 << 40, 1.5)):
+            if time.perf_counter() - t0 > budget_s and tb:
+                break
+            tr.set(**{**chosen, "cluster_ctas": csz, "batch_cluster_min": bmin, "batch_cluster_share": share})
+            tb[(bmin, share, csz)] = tr.batch("batch", batch, "PD")
+    bmin, share, csz = pick_fastest(tb)
+    chosen["batch_cluster_min"], chosen["batch_cluster_share"] = bmin, share
     chosen["cluster_ctas"] = csz
-    tables["batch"] = {f"{k[0]}/{k[1]}/{k[2]}/{k[3]}": v for k, v in tb.items()}
+    tables["batch"] = {f"{k[0]}/{k[1]}/{k[2]}": v for k, v in tb.items()}
     tr.set(**chosen)
     return {"tuning": chosen, "default": base, "tables": tables, "seconds": round(time.perf_counter() - t0, 1)}
 

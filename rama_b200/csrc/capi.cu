@@ -116,6 +116,7 @@ struct rama_context {
     int cluster_cap[17] = {};  // co-resident clusters of k_solve_mixed by cluster size (0: not known yet)
     int cluster_alone_cap[17] = {};  // ... of k_solve_cluster_alone
     rama_tuning tune{};
+    const char *kernel = "";  // the solve kernel launched last
     int parse_ctas = 0;   // co-resident CTAs of k_parse_grid
     char *p_text = nullptr;  // device copy of text for rama_parse_multicut_host
     int64_t p_cap = 0;
@@ -273,6 +274,7 @@ int launch_solve(rama_context *h, int32_t count, int team, cudaStream_t st, int3
         const int per_sm = edges < h->tune.grid_small_max ? h->tune.grid_small_ctas_per_sm
                                                                 : h->tune.grid_ctas_per_sm;
         const void *k = per_sm == 1 ? (const void *)k_solve_grid_alone : (const void *)k_solve_grid;
+        h->kernel = per_sm == 1 ? "k_solve_grid_alone" : "k_solve_grid";
         CU(cudaLaunchCooperativeKernel(k, dim3(per_sm * h->sms), dim3(THREADS), args, SMEM, st));
     } else if (ncluster > 0) {
         const int csz = cluster_size(h, ncluster);
@@ -293,19 +295,28 @@ int launch_solve(rama_context *h, int32_t count, int team, cudaStream_t st, int3
         attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        if (count == 1 && cluster_capacity(h, csz, true) > 0)
+        if (count == 1 && cluster_capacity(h, csz, true) > 0) {
+            h->kernel = "k_solve_cluster_alone";
             CU(cudaLaunchKernelEx(&cfg, k_solve_cluster_alone, h->d_inst));
-        else
+        } else {
+            h->kernel = "k_solve_mixed";
             CU(cudaLaunchKernelEx(&cfg, k_solve_mixed, L));
+        }
     } else {
         CU(cudaMemsetAsync(h->d_queue, 0, sizeof(int32_t), st));
         CtaLaunch L{h->d_inst, h->d_order, count, h->d_queue};
-        if (count == 1 && h->tune.cta_threads == THREADS) {
+        // (one instance has an SM to itself, whatever CTAs suit a batch: region
+        // graphs of 879 and 2,979 edges PD 1.02 and 1.66 ms, on the kernel of
+        // 256 threads 1.33 and 2.47; tune.cta_threads is about batches)
+        if (count == 1) {
+            h->kernel = "k_solve_cta_alone";
             k_solve_cta_alone<<<1, THREADS, SMEM, st>>>(h->d_inst);
         } else if (h->tune.cta_threads == THREADS_SMALL) {
+            h->kernel = "k_solve_cta_small";
             const int ctas = std::max(1, std::min<int>(count, h->sms * h->cta_small_per_sm));
             k_solve_cta_small<<<ctas, THREADS_SMALL, SMEM_SMALL, st>>>(L);
         } else {
+            h->kernel = "k_solve_cta";
             const int ctas = std::max(1, std::min<int>(count, h->sms * h->cta_per_sm));
             k_solve_cta<<<ctas, THREADS, SMEM, st>>>(L);
         }
@@ -871,6 +882,8 @@ int rama_set_tuning(rama_handle h, const rama_tuning *t)
     h->tune = *t;
     return RAMA_OK;
 }
+
+const char *rama_solve_kernel(rama_handle h) { return h ? h->kernel : ""; }
 
 int rama_get_stats(rama_handle h, rama_stats *out)
 {

@@ -98,3 +98,25 @@ def test_small_cta_kernel_gives_the_same_batch_results():
     assert rc == 0
     for (lab, lb), (glab, glb) in zip(want, got):
         assert np.array_equal(lab, glab) and lb == glb
+
+
+@pytest.mark.gpu
+def test_one_instance_runs_on_the_kernel_for_one(oracle):
+    """The CTA size is about batches: a single solve keeps the kernel that has
+    an SM to itself."""
+    from rama_b200 import instances
+    from rama_b200.solver import Solver
+
+    g = instances.delaunay(400, np.random.default_rng(5))
+    b = instances.delaunay_batch(count=2, nmin=300, nmax=500, seed=18)
+    want = oracle.solve(*g, "PD")[:2]
+    s = Solver(0)
+    for threads, kernel in ((512, "k_solve_cta"), (256, "k_solve_cta_small")):
+        t = s.handle.tuning()
+        t.cta_threads = threads
+        s.handle.set_tuning(t)
+        lab, lb, _ = s.solve(*g, mode="PD")
+        assert s.handle.solve_kernel() == "k_solve_cta_alone"
+        assert np.array_equal(lab, want[0]) and lb == want[1]
+        _, _, rc = s.solve_batch(b, mode="PD")
+        assert rc == 0 and s.handle.solve_kernel() == kernel

@@ -213,16 +213,21 @@ int rama_parse_multicut_host(rama_handle h, const char *text, int64_t len, int32
  * are spent.  rama_create starts from built-in values;
  * rama_b200/autotune.py measures better ones per device and sets them.  No
  * counterpart in the reference (its launches have fixed shapes). */
+#define RAMA_CLUSTER_CTAS_AUTO 0
+#define RAMA_MIN_AUTO (-1)
+#define RAMA_AUTO_CLUSTER_MIN 4000
+#define RAMA_AUTO_GRID_MIN 100000
 typedef struct {
     int32_t grid_ctas_per_sm;    /* CTAs per SM of the whole-GPU solve (1 .. the occupancy maximum) ... */
     int32_t grid_small_ctas_per_sm; /* ... and of one of fewer than grid_small_max edges */
     int64_t grid_small_max;
-    int32_t cluster_ctas;        /* CTAs of a cluster team: 2, 4, 8 or 16; 8, the starting value, stands for 16
-                                    where the clusters have the GPU to themselves, down to 4 in a large
-                                    batch */
+    int32_t cluster_ctas;        /* CTAs of a cluster team: 2, 4, 8 or 16, or RAMA_CLUSTER_CTAS_AUTO (the
+                                    starting value): 16 where the clusters have the GPU to themselves, down
+                                    to 4 in a large batch */
     int64_t single_cluster_min;  /* a single solve of at least this many edges runs on a cluster ... */
-    int64_t single_grid_min;     /* ... and from this many on on the whole GPU (else on one CTA); both count
-                                    twice for solves without a dual */
+    int64_t single_grid_min;     /* ... and from this many on on the whole GPU (else on one CTA).  The starting
+                                    value RAMA_MIN_AUTO stands for RAMA_AUTO_CLUSTER_MIN and
+                                    RAMA_AUTO_GRID_MIN, twice that for solves without a dual */
     int64_t batch_cluster_min;   /* batch instances below this size always run on one CTA; larger ones on */
     float batch_cluster_share;   /* a cluster when they hold more than this many times the batch's edges
                                     per CTA */

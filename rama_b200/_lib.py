@@ -61,6 +61,15 @@ class RamaStats(C.Structure):
         ("phase_bytes", C.c_double * 32),
     ]
 
+
+# starting values of rama_tuning that leave a choice to the solver, and what
+# the single-solve thresholds are then (include/rama_b200.h)
+CLUSTER_CTAS_AUTO = 0
+MIN_AUTO = -1
+AUTO_CLUSTER_MIN = 4000
+AUTO_GRID_MIN = 100000
+
+
 class RamaTuning(C.Structure):
     _fields_ = [
         ("grid_ctas_per_sm", C.c_int32),
@@ -76,6 +85,10 @@ class RamaTuning(C.Structure):
 
     def as_dict(self):
         return {k: getattr(self, k) for k, _ in self._fields_}
+
+    def grid_min(self) -> int:
+        """Edges from which a single solve (with a dual) runs on the whole GPU."""
+        return AUTO_GRID_MIN if self.single_grid_min == MIN_AUTO else int(self.single_grid_min)
 
 
 PHASES = ("init", "cycles", "mp_build", "mp_iter", "dual_commit", "matching", "woc", "contract", "other",

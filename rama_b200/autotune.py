@@ -12,7 +12,7 @@ built-in choices are guesses; this module measures them on the device:
   CTAs take cheaper grid barriers, more CTAs hide more memory latency), timed
   on 3-D grids of growing size;
 * cluster_ctas: the cluster size, timed on mid-size Delaunay graphs, and
-  again (against the built-in size) inside the batch trial below, which has
+  again (against the automatic size) inside the batch trial below, which has
   the last word: a batch runs many clusters side by side;
 * single_cluster_min / single_grid_min: where a single solve moves from one
   CTA to a cluster and from a cluster to the whole GPU -- each team is timed
@@ -215,7 +215,9 @@ def tune(device: int = 0, budget_s: float = 60.0, quick: bool = False) -> dict:
     # cluster size on mid-size graphs
     mids = [I.delaunay(n, rng) for n in ((6000, 20000) if not quick else (3000,))]
     tc = {}
-    for csz in (4, 8, 16):
+    # (one cluster alone has 16 CTAs when the size is automatic, so 16 is no
+    # option of its own)
+    for csz in (_lib.CLUSTER_CTAS_AUTO, 4, 8):
         try:
             tr.set(**{**chosen, "cluster_ctas": csz})
         except _lib.RamaError:
@@ -238,9 +240,9 @@ def tune(device: int = 0, budget_s: float = 60.0, quick: bool = False) -> dict:
         clu.append(tr.solve("single%d" % k, g, "PD", team=3))
         grd.append(tr.solve("single%d" % k, g, "PD", team=2))
     if sizes:
-        chosen["single_cluster_min"] = crossover(sizes, cta, clu, int(base["single_cluster_min"]))
+        chosen["single_cluster_min"] = crossover(sizes, cta, clu, _lib.AUTO_CLUSTER_MIN)
         chosen["single_grid_min"] = max(chosen["single_cluster_min"],
-                                        crossover(sizes, clu, grd, int(base["single_grid_min"])))
+                                        crossover(sizes, clu, grd, _lib.AUTO_GRID_MIN))
     tables["single"] = {"edges": sizes, "cta_ms": cta, "cluster_ms": clu, "grid_ms": grd}
     tr.set(**chosen)
 

@@ -28,17 +28,21 @@ namespace {
 // Launch parameters a handle starts with (rama_tuning; the autotuner of
 // rama_b200/autotune.py replaces them with measured choices).  None of them
 // changes a result: every team computes the same solve.
-constexpr int DEFAULT_CLUSTER_CTAS = 8;  // rama_tuning's starting value: the size follows the use, as below
 constexpr int SINGLE_CLUSTER_CTAS = 16;  // CTAs of a cluster that has the GPU to itself
+constexpr int SOME_CLUSTER_CTAS = 8;     // ... of a few clusters at once (the portable maximum)
 constexpr int BATCH_CLUSTER_CTAS = 4;    // ... of many clusters in a batch
-constexpr int64_t DEFAULT_SINGLE_CLUSTER_MIN = 4000;  // a single solve from this size on runs on a cluster
-constexpr int64_t DEFAULT_SINGLE_GRID_MIN = 100000;   // ... and from this size on on the whole GPU
+constexpr int64_t SINGLE_CLUSTER_MIN = RAMA_AUTO_CLUSTER_MIN;  // a single solve from this size on runs on a cluster
+constexpr int64_t SINGLE_GRID_MIN = RAMA_AUTO_GRID_MIN;  // ... and from this size on on the whole GPU
 // Solves without a dual have a fraction of the passes' work per edge, so they
 // change teams at twice these sizes.  Measured (ms, one CTA / cluster of 16 /
 // whole GPU): region graphs without a dual, 5,822 edges 0.65 / 0.75 / 1.18,
 // 8,785 edges 0.75 / 0.76 / 1.15, 208,942 edges - / 1.37 / 1.39; with, 2,874
 // edges 1.57 / 1.73 / 2.87, 5,822 edges 2.40 / 1.99 / 3.30, 89,308 edges
-// - / 3.85 / 3.97, 149,106 edges - / 4.94 / 4.36.
+// - / 3.85 / 3.97, 149,106 edges - / 4.94 / 4.36.  PD+ crosses where PD does
+// (89,964 edges 7.55 / 8.31, 149,971 edges 9.06 / 8.36).  The line to the whole
+// GPU is theirs: the bound alone (D), which stays on the full graph, crosses at
+// some 33,000 edges (23,971 edges 4.63 / 5.22, 35,971 edges 5.90 / 5.55, 89,964
+// edges 8.93 / 6.14), and has no line of its own yet.
 // One CTA per SM (with twice the registers) solves graphs of up to about 3 M
 // edges sooner, two larger ones.  Measured (ms, one / two): 753,664 edges 2.46 /
 // 3.25, 1.14 M 8.96 / 11.2, 2.63 M 17.6 / 18.8, 3.06 M 4.12 / 4.47, 3.30 M 66.2 /
@@ -259,10 +263,10 @@ int cluster_capacity(rama_context *h, int size, bool alone = false)
 // 7.62; 256 of them on 4, 8, 16 15.8, 21.8, 34.2.
 int cluster_size(rama_context *h, int32_t ncluster)
 {
-    if (h->tune.cluster_ctas != DEFAULT_CLUSTER_CTAS) return h->tune.cluster_ctas;
+    if (h->tune.cluster_ctas != RAMA_CLUSTER_CTAS_AUTO) return h->tune.cluster_ctas;
     if (ncluster * SINGLE_CLUSTER_CTAS <= h->sms && cluster_capacity(h, SINGLE_CLUSTER_CTAS) > 0)
         return SINGLE_CLUSTER_CTAS;
-    return ncluster * DEFAULT_CLUSTER_CTAS <= h->sms ? DEFAULT_CLUSTER_CTAS : BATCH_CLUSTER_CTAS;
+    return ncluster * SOME_CLUSTER_CTAS <= h->sms ? SOME_CLUSTER_CTAS : BATCH_CLUSTER_CTAS;
 }
 
 int launch_solve(rama_context *h, int32_t count, int team, cudaStream_t st, int32_t ncluster = 0,
@@ -333,10 +337,13 @@ int solve_one(rama_context *h, const int32_t *d_i, const int32_t *d_j, const flo
     if (h->b_active) return fail(RAMA_ERR_INVALID_ARG, "a batch is in flight on this handle (call rama_batch_wait)");
     Options o = to_opts(opts);
     int team = opts->team;
-    if (team < 1 || team > 3)
-    {
-        const int64_t size = has_dual(o) ? n : n / 2;
-        team = size < h->tune.single_cluster_min ? 1 : (size < h->tune.single_grid_min ? 3 : 2);
+    if (team < 1 || team > 3) {
+        const int64_t times = has_dual(o) ? 1 : 2;
+        const int64_t cluster_min =
+            h->tune.single_cluster_min == RAMA_MIN_AUTO ? times * SINGLE_CLUSTER_MIN : h->tune.single_cluster_min;
+        const int64_t grid_min =
+            h->tune.single_grid_min == RAMA_MIN_AUTO ? times * SINGLE_GRID_MIN : h->tune.single_grid_min;
+        team = n < cluster_min ? 1 : (n < grid_min ? 3 : 2);
     }
     int rc = ensure_inst(h, 1);
     if (rc) return rc;
@@ -517,9 +524,9 @@ int rama_create(int device, uint64_t workspace_bytes, rama_handle *out)
     h->tune.grid_ctas_per_sm = per_sm;
     h->tune.grid_small_ctas_per_sm = 1;
     h->tune.grid_small_max = DEFAULT_GRID_SMALL_MAX;
-    h->tune.cluster_ctas = DEFAULT_CLUSTER_CTAS;
-    h->tune.single_cluster_min = DEFAULT_SINGLE_CLUSTER_MIN;
-    h->tune.single_grid_min = DEFAULT_SINGLE_GRID_MIN;
+    h->tune.cluster_ctas = RAMA_CLUSTER_CTAS_AUTO;
+    h->tune.single_cluster_min = RAMA_MIN_AUTO;
+    h->tune.single_grid_min = RAMA_MIN_AUTO;
     h->tune.batch_cluster_min = DEFAULT_BATCH_CLUSTER_MIN;
     h->tune.batch_cluster_share = DEFAULT_BATCH_CLUSTER_SHARE;
     h->tune.cta_threads = THREADS;
@@ -536,7 +543,7 @@ int rama_create(int device, uint64_t workspace_bytes, rama_handle *out)
                             SMEM_SMALL));
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_cta, k_solve_cta_small, THREADS_SMALL, SMEM_SMALL));
     h->cta_small_per_sm = std::max(1, per_sm_cta);
-    if (cluster_capacity(h, DEFAULT_CLUSTER_CTAS) < 1) {
+    if (cluster_capacity(h, SOME_CLUSTER_CTAS) < 1) {
         delete h;
         return fail(RAMA_ERR_CUDA, "no cluster of the solver kernel fits on the device");
     }
@@ -870,15 +877,17 @@ int rama_set_tuning(rama_handle h, const rama_tuning *t)
         return fail(RAMA_ERR_INVALID_ARG,
                     "grid CTAs per SM must lie in [1, " + std::to_string(h->grid_per_sm_max) + "]");
     const int c = t->cluster_ctas;
-    if (!(c == 2 || c == 4 || c == 8 || c == 16)) return fail(RAMA_ERR_INVALID_ARG, "cluster_ctas must be 2, 4, 8 or 16");
-    if (cluster_capacity(h, c) < 1)
+    if (!(c == RAMA_CLUSTER_CTAS_AUTO || c == 2 || c == 4 || c == 8 || c == 16))
+        return fail(RAMA_ERR_INVALID_ARG, "cluster_ctas must be 0 (automatic), 2, 4, 8 or 16");
+    if (c != RAMA_CLUSTER_CTAS_AUTO && cluster_capacity(h, c) < 1)
         return fail(RAMA_ERR_INVALID_ARG, "no cluster of " + std::to_string(c) + " CTAs fits on this device");
     if (t->cta_threads != THREADS && t->cta_threads != THREADS_SMALL)
         return fail(RAMA_ERR_INVALID_ARG, "cta_threads must be " + std::to_string(THREADS) + " or " +
                                               std::to_string(THREADS_SMALL));
-    if (t->single_cluster_min < 0 || t->single_grid_min < 0 || t->batch_cluster_min < 0 ||
+    if (t->single_cluster_min < RAMA_MIN_AUTO || t->single_grid_min < RAMA_MIN_AUTO || t->batch_cluster_min < 0 ||
         !(t->batch_cluster_share > 0.0f))
-        return fail(RAMA_ERR_INVALID_ARG, "thresholds must be non-negative and the share positive");
+        return fail(RAMA_ERR_INVALID_ARG, "thresholds must be non-negative (-1: automatic, those of a single solve) "
+                                          "and the share positive");
     h->tune = *t;
     return RAMA_OK;
 }

@@ -251,7 +251,7 @@ class Server:
                 ln.handle.set_tuning(tuning)
         self.lane_bytes = lane_bytes
         if solo_min_edges is None:
-            solo_min_edges = int(self.lanes[0].handle.tuning().single_grid_min)
+            solo_min_edges = self.lanes[0].handle.tuning().grid_min()
         self.solo_min_edges = solo_min_edges
 
     def close(self):

@@ -36,6 +36,60 @@ def test_cache_round_trip(tmp_path):
     assert autotune.load_cache(p) == {}
 
 
+def test_automatic_values_are_those_of_the_header():
+    import os
+    import re
+
+    from rama_b200 import _lib
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    with open(os.path.join(root, "include", "rama_b200.h")) as f:
+        defs = dict(re.findall(r"#define (RAMA_\w*AUTO\w*) \(?(-?\d+)\)?", f.read()))
+    assert {k: int(v) for k, v in defs.items()} == {
+        "RAMA_CLUSTER_CTAS_AUTO": _lib.CLUSTER_CTAS_AUTO, "RAMA_MIN_AUTO": _lib.MIN_AUTO,
+        "RAMA_AUTO_CLUSTER_MIN": _lib.AUTO_CLUSTER_MIN, "RAMA_AUTO_GRID_MIN": _lib.AUTO_GRID_MIN}
+    t = _lib.RamaTuning(single_grid_min=_lib.MIN_AUTO)
+    assert t.grid_min() == _lib.AUTO_GRID_MIN
+    t.single_grid_min = 7
+    assert t.grid_min() == 7
+
+
+@pytest.mark.gpu
+def test_thresholds_mean_what_they_say(oracle):
+    """A caller's thresholds hold in every mode; the automatic ones count twice
+    without a dual.  Any cluster size a caller asks for is accepted, 8 among
+    them, and changes no result."""
+    from rama_b200 import _lib, instances
+    from rama_b200.solver import Solver
+
+    g = instances.delaunay(1800, np.random.default_rng(6))  # 5,4xx edges: between the automatic line and its double
+    n = len(g[2])
+    assert _lib.AUTO_CLUSTER_MIN < n < 2 * _lib.AUTO_CLUSTER_MIN
+    s = Solver(0)
+    auto = s.handle.tuning()
+    assert (auto.cluster_ctas, auto.single_cluster_min, auto.single_grid_min) == (0, -1, -1)
+    for low, high, teams in ((-1, -1, {"P": 1, "PD": 3, "D": 3}), (n, -1, {"P": 3, "PD": 3}),
+                             (n + 1, n + 1, {"P": 1, "PD": 1}), (0, n, {"P": 2, "PD": 2}),
+                             (4000, 100000, {"P": 3, "PD": 3})):
+        t = s.handle.tuning()
+        t.single_cluster_min, t.single_grid_min = low, high
+        s.handle.set_tuning(t)
+        for mode, team in teams.items():
+            s.solve(*g, mode=mode)
+            assert s.stats().team == team
+    want = oracle.solve(*g, "PD")[:2]
+    for size in (0, 2, 4, 8, 16):
+        t = s.handle.tuning()
+        t.cluster_ctas = size
+        s.handle.set_tuning(t)
+        assert s.handle.tuning().cluster_ctas == size
+        lab, lb, _ = s.solve(*g, mode="PD", team=3)
+        assert np.array_equal(lab, want[0]) and lb == want[1]
+    t.single_grid_min = -2
+    with pytest.raises(_lib.RamaError):
+        s.handle.set_tuning(t)
+
+
 @pytest.mark.gpu
 def test_tuned_parameters_give_identical_results(tmp_path):
     """A quick tuning run (which itself checks every trial against the first

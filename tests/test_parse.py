@@ -112,3 +112,71 @@ def test_first_line_must_be_multicut(solver):
         _parse(solver, b"GRAPH\n0 1 1\n")
     i, j, c = _parse(solver, b"MULTICUT")
     assert len(c) == 0
+
+
+def _lines(n, seed):
+    rng = np.random.default_rng(seed)
+    i, j = rng.integers(0, 1 << 20, n), rng.integers(0, 1 << 20, n)
+    c = rng.normal(0.0, 2.0, n).astype(np.float32)
+    body = "".join("%d %d %s\n" % x for x in zip(i.tolist(), j.tolist(), [repr(float(x)) for x in c]))
+    return ("MULTICUT\n" + body).encode(), i, j, c
+
+
+def test_long_texts_in_turn():
+    """Texts on both sides of STAGE_MIN and of one, two and more pieces of the
+    pinned buffer, longer and shorter ones in turn, as bytes, bytearray and
+    memoryview, with the stream given and not, on one solver."""
+    import torch
+
+    from rama_b200 import solver as S
+
+    s = S.Solver(0)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    sizes = (S.STAGE_MIN * 3 // 2, S.STAGE_MIN * 3 // 2, S.STAGE_MIN * 5 // 4, S.STAGE_BYTES * 3 // 2,
+             S.STAGE_MIN * 9 // 8, S.STAGE_BYTES * 4, S.STAGE_MIN // 2, S.STAGE_BYTES)
+    for k, size in enumerate(sizes):
+        text, i, j, c = _lines(size // 30, k)
+        short = text[: size * 2 // 3]  # ends anywhere in a line: compared with the general form
+        for x in (text, bytearray(text), memoryview(text)):
+            gi, gj, gc = _parse(s, x)
+            assert np.array_equal(gi, i) and np.array_equal(gj, j) and np.array_equal(gc, c)
+        gi, gj, gc = (x.cpu().numpy() for x in s.parse_multicut(text, stream=stream))
+        assert np.array_equal(gi, i) and np.array_equal(gj, j) and np.array_equal(gc, c)
+        want = [x.cpu().numpy() for x in s.parse_multicut(short, stream=stream)]
+        assert all(np.array_equal(a, b) for a, b in zip(_parse(s, short), want))
+    assert s._stage is not None and s._stage.numel() == 2 * S.STAGE_BYTES
+
+
+def test_uploads_from_two_threads(solver):
+    """The pinned buffer of one solver, filled from two threads in turn."""
+    import threading
+
+    from rama_b200 import solver as S
+
+    texts = [bytes(np.random.default_rng(k).integers(0, 256, S.STAGE_MIN + S.STAGE_BYTES * k, dtype=np.uint8))
+             for k in range(4)]
+    solver._text_to_device(texts[0], None)
+    bad = []
+
+    def work(k):
+        for r in range(6):
+            x = texts[(k + r) % 4]
+            if solver._text_to_device(x, None).cpu().numpy().tobytes() != x:
+                bad.append((k, r))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
+
+
+def test_texts_of_many_lengths_leave_nothing_behind(solver):
+    """ctypes keeps every array class that is made: none is made per length."""
+    from rama_b200 import solver as S
+
+    base = b"MULTICUT\n" + b"1 2 0.5\n" * (S.STAGE_MIN // 8)
+    solver.parse_multicut(base)
+    classes = len(C.Array.__subclasses__())
+    for k in range(20):
+        solver.parse_multicut(base + b"1 2 0.5\n" * k)
+    assert len(C.Array.__subclasses__()) == classes

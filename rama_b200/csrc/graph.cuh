@@ -192,8 +192,9 @@ __device__ __forceinline__ void team_sort_long_records(const Team &t, char *sm, 
     t.sync();
 }
 
-// ends(e): (lo, hi) of edge e, loads only; nbh: bits of a node id
-template <class Team, class Ends>
+// ends(e): (lo, hi) of edge e, loads only; nbh: bits of a node id; PHASES: the
+// steps are timed as the contraction's (the initial sort is one phase)
+template <bool PHASES, class Team, class Ends>
 __device__ __forceinline__ bool team_sort_records(const Team &t, Scratch &sc, char *sm, int64_t n, int32_t nbk,
                                                   int nbh, const float *cost, Ends ends, Records &R)
 {
@@ -240,7 +241,7 @@ __device__ __forceinline__ bool team_sort_records(const Team &t, Scratch &sc, ch
         }
     }
     t.sync();
-    prof_mark(t, sc, PH_CSORT_SLOT);
+    if (PHASES) prof_mark(t, sc, PH_CSORT_SLOT);
     team_bucket_starts(t, sc, sm, nbk, start, L, [](int64_t, int32_t, int32_t) {});
     struct Item {
         int4 r;
@@ -257,9 +258,9 @@ __device__ __forceinline__ bool team_sort_records(const Team &t, Scratch &sc, ch
         },
         [=](int64_t, Item x) { rec[x.p] = x.r; });
     t.sync();
-    prof_mark(t, sc, PH_CSORT_SCATTER);
+    if (PHASES) prof_mark(t, sc, PH_CSORT_SCATTER);
     team_sort_long_records(t, sm, R, L);
-    prof_mark(t, sc, PH_CSORT_RANK);
+    if (PHASES) prof_mark(t, sc, PH_CSORT_RANK);
     if (L.has_big()) {
         // the buckets beyond BUCKET_MAX: their edges in input order, a stable
         // radix sort of (lo, hi), then each into its bucket's range
@@ -291,7 +292,7 @@ __device__ __forceinline__ bool team_sort_records(const Team &t, Scratch &sc, ch
         }
         t.sync();
         sc.arena.release(bm);
-        prof_mark(t, sc, PH_CSORT_BIG);
+        if (PHASES) prof_mark(t, sc, PH_CSORT_BIG);
     }
     return true;
 }
@@ -464,7 +465,7 @@ __device__ __noinline__ Graph graph_from_edges(const Team &t, Scratch &sc, char 
     const int nbh = bits_for((uint64_t)(mx > 0 ? mx : 1));
     uint64_t m = sc.arena.mark();
     Records R;
-    if (!team_sort_records(
+    if (!team_sort_records<false>(
             t, sc, sm, n, mx + 1, nbh, c,
             [=](int64_t e) {
                 const int32_t a = i[e], b = j[e];
@@ -735,7 +736,7 @@ __device__ __noinline__ Graph graph_contract(const Team &t, Scratch &sc, char *,
         fl[2] = -1;
     }
     Records R;
-    if (!team_sort_records(
+    if (!team_sort_records<true>(
             t, sc, sm, n, map_max + 1, nbh, A.cost,
             [=](int64_t e) {
                 const int32_t a = map[A.row[e]], b = map[A.col[e]];

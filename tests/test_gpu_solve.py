@@ -248,3 +248,19 @@ def test_async_batch_mixed_modes(solver, oracle):
         olab, olb, _ = oracle.solve(i, j, c, modes[k])
         assert lbs[k] == olb
         assert np.array_equal(out[lo[k]:lo[k] + nl[k]], olab)
+
+
+@pytest.mark.parametrize("team", (1, 2, 3))
+def test_phase_times_of_the_initial_sort(solver, team):
+    """The initial sort is timed as one phase; the contraction's phases belong
+    to contractions, and the bound alone has none."""
+    from rama_b200 import _lib
+
+    i, j, c = instances.grid2d(64, 64, seed=1001)
+    solver.solve(i, j, c, mode="D", team=team)
+    ms = dict(zip(_lib.PHASES, solver.stats().phase_ms))
+    assert ms["init"] > 0
+    assert all(v == 0 for k, v in ms.items() if k.startswith(("csort", "contract")))
+    solver.solve(i, j, c, mode="P", team=team)
+    ms = dict(zip(_lib.PHASES, solver.stats().phase_ms))
+    assert ms["init"] > 0 and ms["csort_slot"] > 0 and ms["contract_runs"] > 0

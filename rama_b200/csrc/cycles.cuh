@@ -698,7 +698,7 @@ __device__ __noinline__ void conflicted_cycles(const Team &t, Scratch &sc, char 
     int32_t *adj = nullptr;
     int64_t m2 = 0;
     if (A.n >= (int64_t(1) << 30) || !attractive_lists(t, sc, sm, A, N, pos_tol, off, adj, m2)) {
-        Csr C = build_symmetric_csr(t, sc, sm, A, N, [=](int64_t e) { return A.cost[e] > pos_tol; }, false);
+        Csr C = build_symmetric_csr(t, sc, sm, A, N, [=](int64_t e) { return A.cost[e] > pos_tol; });
         off = C.off;
         adj = C.adj;
         m2 = C.m2;

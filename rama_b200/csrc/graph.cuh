@@ -521,40 +521,13 @@ __device__ __noinline__ Graph graph_from_edges_sorted(const Team &t, Scratch &sc
     float *v1 = sc.arena.take<float>(n + 1), *v2 = sc.arena.take<float>(n + 1);
     Graph g = graph_alloc(t, sc, n);
     if (!sc.arena.ok()) return out;
-    // sort by (min, max) endpoint, stably: bucket by the smaller endpoint and
-    // order each bucket by (larger endpoint, edge index); hub rows of more
-    // than BUCKET_MAX edges: LSD radix sort
-    bool done = false;
-    {
-        uint64_t bm = sc.arena.mark();
-        int32_t *bst = sc.arena.take<int32_t>((int64_t)mx + 2);
-        int32_t *bidx = sc.arena.take<int32_t>(n + 1);
-        if (sc.arena.ok() && n < (int64_t(1) << 31)) {
-            done = team_bucket_sort(
-                t, sc, sm, n, mx + 1, [=](int64_t e) { return i[e] < j[e] ? i[e] : j[e]; },
-                [=](int64_t e) -> uint64_t {
-                    return ((uint64_t)(uint32_t)(i[e] < j[e] ? j[e] : i[e]) << 32) | (uint64_t)e;
-                },
-                k2, bidx, bst);
-            if (done) {
-                for (int64_t b = t.rank(); b <= mx; b += t.size())
-                    for (int32_t p = bst[b]; p < bst[b + 1]; ++p)
-                        k1[p] = pack_key((int32_t)b, (int32_t)(k2[p] >> 32), nb);
-                for (int64_t p = t.rank(); p < n; p += t.size()) v1[p] = c[bidx[p]];
-                t.sync();
-            }
-        }
-        sc.arena.release(bm);
+    for (int64_t e = t.rank(); e < n; e += t.size()) {
+        int32_t a = i[e], b = j[e];
+        k1[e] = pack_key(a < b ? a : b, a < b ? b : a, nb);
+        v1[e] = c[e];
     }
-    if (!done) {
-        for (int64_t e = t.rank(); e < n; e += t.size()) {
-            int32_t a = i[e], b = j[e];
-            k1[e] = pack_key(a < b ? a : b, a < b ? b : a, nb);
-            v1[e] = c[e];
-        }
-        t.sync();
-        team_sort_pairs(t, sc, sm, k1, v1, k2, v2, n, 2 * nb);
-    }
+    t.sync();
+    team_sort_pairs(t, sc, sm, k1, v1, k2, v2, n, 2 * nb);
     const uint64_t mask = (nb == 0) ? 0 : ((uint64_t(1) << nb) - 1);
     for (int64_t e = t.rank(); e < n; e += t.size()) {
         g.row[e] = (int32_t)(k1[e] >> nb);
@@ -1076,20 +1049,19 @@ struct Csr {
     int32_t *off;  // nrows + 1
     int32_t *adj;  // 2m
     float *w;      // 2m
-    int32_t *eid;  // 2m: index of the directed edge (in the kept order) -- optional
     int64_t m2;
 };
 
 template <class Team, class Keep>
-__device__ __noinline__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char *, const Graph &A, int32_t nrows, Keep keep,
-                                   bool with_eid, int64_t *kept_idx_out = nullptr)
+__device__ __noinline__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char *, const Graph &A, int32_t nrows,
+                                                Keep keep)
 {
     char *sm = team_smem();
     Csr C;
     C.nrows = nrows;
     C.m2 = 0;
     // 1. compact kept edges (their order stays (row,col)-sorted)
-    int64_t *kidx = kept_idx_out ? kept_idx_out : sc.arena.take<int64_t>(A.n + 1);
+    int64_t *kidx = sc.arena.take<int64_t>(A.n + 1);
     int32_t *deg = sc.arena.take<int32_t>((int64_t)nrows + 1);
     C.off = sc.arena.take<int32_t>((int64_t)nrows + 2);
     if (!sc.arena.ok()) return C;
@@ -1098,7 +1070,6 @@ __device__ __noinline__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char
     C.m2 = 2 * m;
     C.adj = sc.arena.take<int32_t>(2 * m + 1);
     C.w = sc.arena.take<float>(2 * m + 1);
-    C.eid = with_eid ? sc.arena.take<int32_t>(2 * m + 1) : nullptr;
     uint64_t mk = sc.arena.mark();
     uint64_t *k1 = sc.arena.take<uint64_t>(m + 1), *k2 = sc.arena.take<uint64_t>(m + 1);
     int32_t *v1 = sc.arena.take<int32_t>(m + 1), *v2 = sc.arena.take<int32_t>(m + 1);
@@ -1147,7 +1118,6 @@ __device__ __noinline__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char
             const int64_t dst = (int64_t)C.off[c] + (q - bst[c]);
             C.adj[dst] = A.row[e];
             C.w[dst] = A.cost[e];
-            if (with_eid) C.eid[dst] = (int32_t)p;
         }
     } else {
         team_sort_pairs(t, sc, sm, k1, v1, k2, v2, m, bits_for((uint64_t)(nrows > 0 ? nrows : 1)));
@@ -1158,7 +1128,6 @@ __device__ __noinline__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char
             int64_t dst = (int64_t)C.off[c] + (q - colstart[c]);
             C.adj[dst] = A.row[e];
             C.w[dst] = A.cost[e];
-            if (with_eid) C.eid[dst] = (int32_t)p;
         }
     }
     // forward entries: the kept edges of row r are contiguous in kidx order
@@ -1168,7 +1137,6 @@ __device__ __noinline__ Csr build_symmetric_csr(const Team &t, Scratch &sc, char
         int64_t dst = (int64_t)C.off[r] + infill[r] + (p - rowstart[r]);
         C.adj[dst] = A.col[e];
         C.w[dst] = A.cost[e];
-        if (with_eid) C.eid[dst] = (int32_t)p;
     }
     t.sync();
     sc.arena.release(mk);

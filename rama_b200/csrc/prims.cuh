@@ -1227,38 +1227,44 @@ __device__ __forceinline__ void smem_bitonic(uint64_t *key, int32_t *idx, int m,
     }
 }
 
-// The general form: the slot pass calls bk_slot(i) once per item (it may
-// store what it computes for the scatter pass), the scatter pass calls
-// bucket(i), sub(i) and pay(i); idx_out receives pay(i) of each item instead of
-// its index (team_bucket_sort below: pay(i) = i), and bucket_out, if given, the
-// bucket of each sorted position.
-//
-// Buckets of more than BUCKET_MAX items: with big_bits > 0 their items are
-// taken out in input order and sorted by a stable LSD radix sort of
-// big_key(i) (big_bits bits), which must order them as (bucket, sub) does
-// once equal keys keep their input order -- e.g. (bucket, hi) when sub is
-// (hi, item index).  With big_bits == 0 such a bucket makes the sort return
-// false.
-struct NoBigKey {
-    __device__ uint64_t operator()(int64_t) const { return 0; }
-};
-struct NoNote {
-    __device__ void operator()(int64_t, int64_t) const {}
-};
-
 // Items handled at once by a thread in the sort's streaming passes: their
 // loads are issued together, so a pass waits for one memory round trip per
 // batch instead of one per item.
 constexpr int SORT_BATCH = 4;
 
-// bk_slot(i) must only load: its value carries the bucket in the low 32 bits
-// (the high 32 bits are the caller's), and note(i, value) stores whatever the
-// caller keeps of it once the batch's loads are done.
-template <class Team, class BkSlot, class Bk, class Sub, class Pay, class BigKey = NoBigKey, class Note = NoNote>
-__device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_t n, int32_t nb, BkSlot bk_slot,
-                                    Bk bucket, Sub sub, Pay pay, uint64_t *keys_out, int32_t *idx_out,
-                                    int32_t *bstart, int32_t *bucket_out = nullptr, int detail_phase = -1,
-                                    BigKey big_key = BigKey(), int big_bits = 0, Note note = Note())
+// the slot of this lane's item in bucket b (-1: no item): the lanes of a warp
+// that share a bucket take theirs with one atomic; every lane must call
+__device__ __forceinline__ int32_t bucket_slot(int32_t *counts, int32_t b)
+{
+    const unsigned peers = __match_any_sync(FULL, b);
+    const int leader = __ffs(peers) - 1;
+    int32_t s = 0;
+    if (b >= 0 && lane_id() == leader) s = atomicAdd(&counts[b], __popc(peers));
+    return __shfl_sync(FULL, s, leader) + __popc(peers & lanemask_lt());
+}
+
+// The same for U items a lane at a time: the atomics of all of them are in
+// flight together (the contraction's slot passes of the 24.8 M edge volume
+// waited for four in turn before).
+template <int U>
+__device__ __forceinline__ void bucket_slots(int32_t *counts, const int32_t (&b)[U], int32_t (&s)[U])
+{
+    unsigned peers[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+        peers[k] = __match_any_sync(FULL, b[k]);
+        s[k] = 0;
+        if (b[k] >= 0 && lane_id() == __ffs(peers[k]) - 1) s[k] = atomicAdd(&counts[b[k]], __popc(peers[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+        s[k] = __shfl_sync(FULL, s[k], __ffs(peers[k]) - 1) + __popc(peers[k] & lanemask_lt());
+}
+
+// bucket(i) and sub(i) must only load.
+template <class Team, class Bk, class Sub>
+__device__ bool team_bucket_sort(const Team &t, Scratch &sc, char *sm, int64_t n, int32_t nb, Bk bucket, Sub sub,
+                                 uint64_t *keys_out, int32_t *idx_out, int32_t *bstart)
 {
     uint64_t am = sc.arena.mark();
     int32_t *slot = sc.arena.take<int32_t>(n + 1);
@@ -1279,35 +1285,19 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
         constexpr int U = SORT_BATCH;
         const int64_t S = t.size();
         for (int64_t base = (int64_t)t.rank() - lane_id(); base < n; base += S * U) {
-            int64_t w[U];
+            int32_t b[U], s[U];
 #pragma unroll
             for (int k = 0; k < U; ++k) {
                 const int64_t i = base + k * S + lane_id();
-                w[k] = i < n ? (int64_t)bk_slot(i) : int64_t(-1);
+                b[k] = i < n ? (int32_t)bucket(i) : -1;
             }
-            int32_t s0[U];
-            unsigned peers[U];
+            bucket_slots<U>(bstart, b, s);
 #pragma unroll
-            for (int k = 0; k < U; ++k) {
-                const int64_t i = base + k * S + lane_id();
-                const int32_t b = i < n ? (int32_t)(uint32_t)w[k] : -1;
-                peers[k] = __match_any_sync(FULL, b);
-                s0[k] = 0;
-                if (i < n && lane_id() == __ffs(peers[k]) - 1) s0[k] = atomicAdd(&bstart[b], __popc(peers[k]));
-            }
-#pragma unroll
-            for (int k = 0; k < U; ++k) {
-                const int64_t i = base + k * S + lane_id();
-                const int32_t s = __shfl_sync(FULL, s0[k], __ffs(peers[k]) - 1);
-                if (i < n) {
-                    slot[i] = s + __popc(peers[k] & lanemask_lt());
-                    note(i, w[k]);
-                }
-            }
+            for (int k = 0; k < U; ++k)
+                if (base + k * S + lane_id() < n) slot[base + k * S + lane_id()] = s[k];
         }
     }
     t.sync();
-    if (detail_phase >= 0) prof_mark(t, sc, detail_phase);
     // bucket starts; buckets of more than 64 items go to the warp and CTA
     // lists (any order); one of more than BUCKET_MAX ends the sort
     team_scan<Team, int64_t>(
@@ -1321,8 +1311,8 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
             else if (c > 64)
                 wlist[atomicAdd(&nlist[0], 1)] = (int32_t)b;
         });
-    const bool has_big = uread(&nlist[2]) != 0;
-    if (has_big && big_bits <= 0) {
+    if (uread(&nlist[2]) != 0) {
+        t.sync();  // every thread has seen it before the memory is handed on
         sc.arena.release(am);
         return false;
     }
@@ -1335,21 +1325,20 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
         const int64_t S = t.size();
         int64_t i0 = t.rank();
         for (; i0 + (U - 1) * S < n; i0 += U * S) {
-            int32_t b[U], p[U], pv[U];
+            int32_t b[U], p[U];
             uint64_t kv[U];
 #pragma unroll
             for (int k = 0; k < U; ++k) {
                 b[k] = (int32_t)bucket(i0 + k * S);
                 p[k] = slot[i0 + k * S];
                 kv[k] = sub(i0 + k * S);
-                pv[k] = pay(i0 + k * S);
             }
 #pragma unroll
             for (int k = 0; k < U; ++k) p[k] += bstart[b[k]];
 #pragma unroll
             for (int k = 0; k < U; ++k) {
                 tk[p[k]] = kv[k];
-                ti[p[k]] = pv[k];
+                ti[p[k]] = (int32_t)(i0 + k * S);
                 tb[p[k]] = b[k];
             }
         }
@@ -1357,19 +1346,18 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
             const int32_t b = (int32_t)bucket(i0);
             const int64_t p = (int64_t)bstart[b] + slot[i0];
             tk[p] = sub(i0);
-            ti[p] = pay(i0);
+            ti[p] = (int32_t)i0;
             tb[p] = b;
         }
     }
     t.sync();
-    if (detail_phase >= 0) prof_mark(t, sc, detail_phase + 1);
     // up to 64 items: each item's rank in its bucket is the number of smaller
     // keys there (neighbouring threads read the same bucket)
     {
-        // the rank of item p in its bucket; -1: sorted below (a bucket of
-        // 65..BUCKET_MAX items is copied as it is) or by the big path
-        auto rank_in_bucket = [=](int64_t p, int32_t s, int32_t e, uint64_t key) -> int32_t {
-            if (e - s > 64) return e - s <= BUCKET_MAX ? (int32_t)p : -1;
+        // the place of item p: its rank in its bucket (a bucket of more than
+        // 64 items is copied as it is and sorted below)
+        auto place = [=](int64_t p, int32_t s, int32_t e, uint64_t key) -> int32_t {
+            if (e - s > 64) return (int32_t)p;
             int32_t r = 0;
             for (int32_t q = s; q < e; ++q) {
                 const uint64_t o = tk[q];
@@ -1395,24 +1383,19 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
                 e[k] = bstart[b[k] + 1];
             }
 #pragma unroll
-            for (int k = 0; k < U; ++k) dst[k] = rank_in_bucket(p0 + k * S, s[k], e[k], kv[k]);
+            for (int k = 0; k < U; ++k) dst[k] = place(p0 + k * S, s[k], e[k], kv[k]);
 #pragma unroll
-            for (int k = 0; k < U; ++k)
-                if (dst[k] >= 0) {
-                    keys_out[dst[k]] = kv[k];
-                    idx_out[dst[k]] = iv[k];
-                    if (bucket_out) bucket_out[dst[k]] = b[k];
-                }
+            for (int k = 0; k < U; ++k) {
+                keys_out[dst[k]] = kv[k];
+                idx_out[dst[k]] = iv[k];
+            }
         }
         for (; p0 < n; p0 += S) {
             const int32_t b = tb[p0];
             const uint64_t key = tk[p0];
-            const int32_t dst = rank_in_bucket(p0, bstart[b], bstart[b + 1], key);
-            if (dst >= 0) {
-                keys_out[dst] = key;
-                idx_out[dst] = ti[p0];
-                if (bucket_out) bucket_out[dst] = b;
-            }
+            const int32_t dst = place(p0, bstart[b], bstart[b + 1], key);
+            keys_out[dst] = key;
+            idx_out[dst] = ti[p0];
         }
     }
     t.sync();
@@ -1467,47 +1450,6 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
         }
     }
     t.sync();
-    if (detail_phase >= 0) prof_mark(t, sc, detail_phase + 2);
-    // (compiled only for callers that give a big key)
-    if constexpr (!std::is_same<BigKey, NoBigKey>::value) if (has_big) {
-        // the buckets beyond BUCKET_MAX: their items in input order, a stable
-        // radix sort of big_key, then each into its bucket's range
-        auto bsize = [=](int64_t i) {
-            const int32_t b = (int32_t)bucket(i);
-            return bstart[b + 1] - bstart[b];
-        };
-        uint64_t bm = sc.arena.mark();
-        const int64_t nbig = team_sum<Team, int64_t>(t, sc, sm, n, [=](int64_t i) -> int64_t {
-            return bsize(i) > BUCKET_MAX ? 1 : 0;
-        });
-        uint64_t *bk1 = sc.arena.take<uint64_t>(nbig + 1), *bk2 = sc.arena.take<uint64_t>(nbig + 1);
-        int32_t *bv1 = sc.arena.take<int32_t>(nbig + 1), *bv2 = sc.arena.take<int32_t>(nbig + 1);
-        int32_t *kfirst = sc.arena.take<int32_t>((int64_t)nb + 1);
-        if (!sc.arena.ok()) return false;
-        team_compact(
-            t, sc, sm, n, [=](int64_t i) { return bsize(i) > BUCKET_MAX; },
-            [=](int64_t i, int64_t k) {
-                bk1[k] = big_key(i);
-                bv1[k] = (int32_t)i;
-            });
-        team_sort_pairs(t, sc, sm, bk1, bv1, bk2, bv2, nbig, big_bits);
-        for (int64_t k = t.rank(); k < nbig; k += t.size()) {
-            const int32_t b = (int32_t)bucket(bv1[k]);
-            if (k == 0 || (int32_t)bucket(bv1[k - 1]) != b) kfirst[b] = (int32_t)k;
-        }
-        t.sync();
-        for (int64_t k = t.rank(); k < nbig; k += t.size()) {
-            const int64_t i = bv1[k];
-            const int32_t b = (int32_t)bucket(i);
-            const int64_t p = (int64_t)bstart[b] + (k - kfirst[b]);
-            keys_out[p] = sub(i);
-            idx_out[p] = pay(i);
-            if (bucket_out) bucket_out[p] = b;
-        }
-        t.sync();
-        sc.arena.release(bm);
-        if (detail_phase >= 0) prof_mark(t, sc, PH_CSORT_BIG);
-    }
     sc.arena.release(am);
     return true;
 }
@@ -1521,7 +1463,7 @@ __device__ bool team_bucket_sort_ex(const Team &t, Scratch &sc, char *sm, int64_
 // bucket (bucket_rank).  Buckets of more than BUCKET_SMALL keys are listed by
 // team_bucket_starts and sorted by team_sort_long_buckets (a warp each up to
 // 256 keys, a CTA up to BUCKET_MAX); what lies beyond is the caller's general
-// path.  Against team_bucket_sort_ex this moves one key per item instead of
+// path.  Against team_bucket_sort this moves one key per item instead of
 // an index, a bucket and a key in and out, and takes five team syncs
 // instead of eight.
 // ---------------------------------------------------------------------------
@@ -1594,35 +1536,6 @@ __device__ __forceinline__ int32_t bucket_rank(const K *keys, int32_t s, int32_t
     return r;
 }
 
-// the slot of this lane's item in bucket b (-1: no item): the lanes of a warp
-// that share a bucket take theirs with one atomic; every lane must call
-__device__ __forceinline__ int32_t bucket_slot(int32_t *counts, int32_t b)
-{
-    const unsigned peers = __match_any_sync(FULL, b);
-    const int leader = __ffs(peers) - 1;
-    int32_t s = 0;
-    if (b >= 0 && lane_id() == leader) s = atomicAdd(&counts[b], __popc(peers));
-    return __shfl_sync(FULL, s, leader) + __popc(peers & lanemask_lt());
-}
-
-// The same for U items a lane at a time: the atomics of all of them are in
-// flight together (the contraction's slot passes of the 24.8 M edge volume
-// waited for four in turn before).
-template <int U>
-__device__ __forceinline__ void bucket_slots(int32_t *counts, const int32_t (&b)[U], int32_t (&s)[U])
-{
-    unsigned peers[U];
-#pragma unroll
-    for (int k = 0; k < U; ++k) {
-        peers[k] = __match_any_sync(FULL, b[k]);
-        s[k] = 0;
-        if (b[k] >= 0 && lane_id() == __ffs(peers[k]) - 1) s[k] = atomicAdd(&counts[b[k]], __popc(peers[k]));
-    }
-#pragma unroll
-    for (int k = 0; k < U; ++k)
-        s[k] = __shfl_sync(FULL, s[k], __ffs(peers[k]) - 1) + __popc(peers[k] & lanemask_lt());
-}
-
 template <class K, class Bar>
 __device__ __forceinline__ void smem_bitonic_keys(K *key, int m, int P, int lane, int nth, Bar bar)
 {
@@ -1680,14 +1593,6 @@ __device__ __forceinline__ void team_sort_long_buckets(const Team &t, char *sm, 
             __syncthreads();
         }
     }
-}
-
-template <class Team, class Bk, class Sub>
-__device__ bool team_bucket_sort(const Team &t, Scratch &sc, char *sm, int64_t n, int32_t nb, Bk bucket, Sub sub,
-                                 uint64_t *keys_out, int32_t *idx_out, int32_t *bstart)
-{
-    return team_bucket_sort_ex(
-        t, sc, sm, n, nb, bucket, bucket, sub, [](int64_t i) { return (int32_t)i; }, keys_out, idx_out, bstart);
 }
 
 // ---------------------------------------------------------------------------

@@ -535,7 +535,7 @@ __device__ __noinline__ int32_t woc_contraction_map(const Team &t, Scratch &sc, 
     for (int64_t p = t.rank(); p < P; p += t.size())
         if (chosen[p]) ekeep[pidx[p]] = 1;
     t.sync();
-    Csr C = build_symmetric_csr(t, sc, sm, A, F.nn, [=](int64_t e) { return ekeep[e] != 0; }, false);
+    Csr C = build_symmetric_csr(t, sc, sm, A, F.nn, [=](int64_t e) { return ekeep[e] != 0; });
     F.m2 = C.m2;
     F.off = C.off;
     F.c = C.adj;

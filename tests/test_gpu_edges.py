@@ -143,6 +143,97 @@ def test_cycles_beside_self_loops(solver, oracle, seed, team):
         assert graw == raw and np.array_equal(got, want)
 
 
+@pytest.fixture(scope="module")
+def by_kernel():
+    """A solver and a call for each kernel that one small instance alone, on
+    an untuned handle, does not run on."""
+    from rama_b200.solver import Solver
+
+    handles = {}
+
+    def tuned(**kw):
+        s = Solver(0)
+        t = s.handle.tuning()
+        for k, v in kw.items():
+            setattr(t, k, v)
+        s.handle.set_tuning(t)
+        return s
+
+    def run(kernel, i, j, c, mode, **kw):
+        if kernel not in handles:
+            handles[kernel] = tuned(**{"k_solve_grid": {"grid_small_max": 0},
+                                       "k_solve_cta_small": {"cta_threads": 256}}.get(kernel, {}))
+        s = handles[kernel]
+        if kernel == "k_solve_grid":
+            lab, lb, _ = s.solve(i, j, c, mode=mode, team=2, **kw)
+            got = [(lab, lb)]
+        else:  # the instance twice
+            nodes = int(max(i.max(), j.max())) + 1
+            got, _, rc = s.solve_batch(_batch([(i, j, c)] * 2, [nodes] * 2), mode=mode,
+                                       team=3 if kernel == "k_solve_mixed" else 1, **kw)
+            assert rc == 0
+        assert s.handle.solve_kernel() == kernel
+        return got
+
+    return run
+
+
+def _shapes():
+    def hub(degree):
+        rng = np.random.default_rng(degree)
+        k = np.arange(1, degree + 1, dtype=np.int32)
+        i = np.concatenate([np.zeros(degree, np.int32), k[:-1], k[:-2]])
+        return i, np.concatenate([k, k[1:], k[2:]]), rng.normal(0.4, 1.0, len(i)).astype(np.float32)
+
+    def copies(m):
+        i, j, _ = instances.random_graph(24, 4, seed=3)
+        c = np.random.default_rng(m).normal(0.2, 1.0, len(i) * m).astype(np.float32)
+        return np.tile(i, m), np.tile(j, m), c
+
+    def path(nodes):
+        k = np.arange(nodes - 1, dtype=np.int32)
+        return k, k + 1, np.random.default_rng(nodes).normal(0.3, 1.0, nodes - 1).astype(np.float32)
+
+    def pairs(edges):
+        k = np.arange(edges, dtype=np.int32) * 5
+        return k, k + 1, np.random.default_rng(edges).normal(0.1, 1.0, edges).astype(np.float32)
+
+    every = ("P", "PD+", "D")
+    out = [("messages%d" % n, book(n, n), every, {}) for n in (4, 5, 8, 9, 64, 65, 257, 4097)]
+    out += [("neighbours%d" % n, hub(n), every, {}) for n in (64, 65, 256, 257, 4096, 4097)]
+    out += [("copies%d" % n, copies(n), ("D",), {}) for n in (2, 33, 65)]  # (contractions of these go bad)
+    out += [("path%d" % n, path(n), every, {}) for n in (2, 511, 2048, 2049)]
+    out += [("pairs%d" % n, pairs(n), every, {}) for n in (2, 3000)]
+    out += [("budget%g" % f, book(300, 1), every, {"tri_memory_factor": f}) for f in (0.0, 0.1, 100.0, 300.0)]
+    return out
+
+
+SHAPES = _shapes()
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=[s[0] for s in SHAPES])
+@pytest.mark.parametrize("kernel", ("k_solve_grid", "k_solve_cta", "k_solve_cta_small", "k_solve_mixed"))
+def test_shapes_on_the_other_kernels(by_kernel, oracle, kernel, shape):
+    """The sizes above on the kernels of two CTAs per SM and of batches."""
+    _, (i, j, c), modes, kw = shape
+    for mode in modes:
+        olab, olb, _ = oracle.solve(i, j, c, mode, **kw)
+        for lab, lb in by_kernel(kernel, i, j, c, mode, **kw):
+            assert lb == olb and np.array_equal(lab, olab)
+
+
+@pytest.mark.parametrize("mode", ("P", "PD"))
+def test_several_tiles_a_cta(solver, by_kernel, oracle, mode):
+    """More edges than a tile for each of the 148 or 296 CTAs of a grid."""
+    i, j, c = instances.grid3d_longrange(64, 64, 32, seed=7)
+    olab, olb, _ = oracle.solve(i, j, c, mode)
+    lab, lb, _ = solver.solve(i, j, c, mode=mode, team=2)
+    assert solver.handle.solve_kernel() == "k_solve_grid_alone"
+    assert lb == olb and np.array_equal(lab, olab)
+    for lab, lb in by_kernel("k_solve_grid", i, j, c, mode):
+        assert lb == olb and np.array_equal(lab, olab)
+
+
 @pytest.mark.parametrize("mode", ("P", "PD"))
 def test_clusters_of_every_size(solver, oracle, mode):
     """Batches of few, some and many instances for clusters, and one alone on

@@ -236,6 +236,28 @@ def test_csum(solver, oracle, n, team):
 
 
 @pytest.mark.parametrize("team", TEAMS)
+@pytest.mark.parametrize("cancels", (False, True))
+def test_csum_of_many_values(solver, oracle, cancels, team):
+    """Values of one sign: the correctly rounded sum on every team.  Values
+    that cancel: a thread that adds m of them leaves an error of at most
+    m^2 u^2 sum|x| (u = 2^-53; m = 5,860 on one CTA's 512 threads), beside the
+    rounding of the result."""
+    import math
+
+    n = 3_000_000
+    x = np.abs(np.random.default_rng(1).normal(size=n)).astype(np.float32) * np.float32(100)
+    if cancels:
+        x = np.concatenate([x, -x[::-1], np.float32([1e-3, 3e-7])])[np.random.default_rng(2).permutation(2 * n + 2)]
+    want = math.fsum(x.tolist())
+    got = solver.step_csum(x, team=team)
+    if cancels:
+        m, u = math.ceil(len(x) / 512) + 64, 2.0 ** -53
+        assert abs(got - want) <= m * m * u * u * math.fsum(np.abs(x).tolist()) + u * abs(want)
+    else:
+        assert got == want == oracle.csum(x)
+
+
+@pytest.mark.parametrize("team", TEAMS)
 @pytest.mark.parametrize("n,bits", [(1, 8), (1000, 5), (100_000, 20), (300_001, 44), (1_000_000, 3),
                                     (3_000_017, 44)])
 def test_radix_sort_is_stable(solver, n, bits, team):

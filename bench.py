@@ -59,22 +59,23 @@ def peaks():
 
 
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of one solve
-# launch per input edge, from one ncu capture of a profiling-size case of the
-# same generator; the full instances are too large to capture under replay,
-# so the traffic is scaled by edge count (the algorithmic bytes per edge of
-# the two sizes are close: see roofline.algorithmic_bytes).
-#   C2 (k_solve_grid), 3-D grid 64x64x32 + long range, 753,664 edges, PD:
-#     335,417,600 B read + 1,157,507,584 B written;
-#   C4 (k_solve_mixed), 64 Delaunay graphs of the C4 generator, 1,048,829
-#     edges, PD: 407,300,096 B read + 1,957,661,440 B written.
+# launch per input edge, by configuration and kernel, from ncu captures of one
+# pass (nothing is replayed, so the full C2 instance is captured as it is):
+#   C2, 24,805,376 edges, PD, k_solve_grid:
+#     22,577,681,408 B read + 15,154,053,632 B written;
+#   its profiling-size case, 753,664 edges, PD, k_solve_grid_alone:
+#     45,874,432 B read + 446,084,608 B written;
+#   C4's profiling-size case (64 Delaunay graphs of its generator, 1,048,829
+#     edges, PD, k_solve_mixed; the full batch is scaled from it by its edges):
+#     409,097,472 B read + 1,993,044,736 B written.
 # Commands: ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,gpu__time_duration.sum
 #   --clock-control none -k regex:k_solve_grid -s 1 -c 1
-#   python bench.py --config c2s --steps 2 --warmup 1 --no-cpu-baseline --no-tune
-# (and -k regex:k_solve_ -s 1 -c 2 ... --config c4s --steps 3 --warmup 3 for C4)
-TRAFFIC_B_PER_EDGE = {("c2", "PD"): (335417600 + 1157507584) / 753664,
-                      ("c2s", "PD"): (335417600 + 1157507584) / 753664,
-                      ("c4", "PD"): (407300096 + 1957661440) / 1048829,
-                      ("c4s", "PD"): (407300096 + 1957661440) / 1048829}
+#   python bench.py --config c2 --steps 2 --warmup 1 --no-cpu-baseline --no-tune
+# (or --config c2s; and -k regex:k_solve_ -s 1 -c 2 ... --config c4s --steps 3 --warmup 3 for C4)
+TRAFFIC_B_PER_EDGE = {("c2", "PD", "k_solve_grid"): (22577681408 + 15154053632) / 24805376,
+                      ("c2s", "PD", "k_solve_grid_alone"): (45874432 + 446084608) / 753664,
+                      ("c4", "PD", "k_solve_mixed"): (409097472 + 1993044736) / 1048829,
+                      ("c4s", "PD", "k_solve_mixed"): (409097472 + 1993044736) / 1048829}
 
 
 def make_instance(cfg):

@@ -606,11 +606,22 @@ __device__ int64_t team_compact(const Team &t, Scratch &sc, char *sm, int64_t n,
 // CSUM: compensated FP64 sum of floats.  Every thread adds its elements with
 // TwoSum (the sum and its error, about 106 bits together), the pairs of a CTA
 // and then of the team are merged the same way, and the result is rounded
-// once.  The error of the pair is some 2^-35 of the result's last place at
-// 25 M elements (a few hundred roundings of the compensation, each 2^-53 of
-// it), so the result is the correctly rounded sum whatever the order and the
-// team, and equals the CPU oracle's, unless the exact sum comes that close to
-// the middle between two doubles without lying on it.
+// once.
+//
+// Its error.  The sum's part of a merge is exact together with the error that
+// joins the compensation; what is lost are the roundings of the compensation,
+// two a merge.  After k merges of values that add up to X in magnitude the
+// compensation is at most k u X (u = 2^-53), so m of them lose at most
+// m^2 u^2 X in all, m being a thread's additions and the some 20 merges over
+// its team.  Against the last place of the result S that is m^2 u (X / |S|):
+// for 25 M elements 2^-36 on the whole GPU (m = 350), 2^-30 on a cluster of 16
+// CTAs (3,050), 2^-22 on one CTA (48,800), and the oracle's fixed tree (m = 320)
+// 2^-36, all times X / |S|.  So for values of one sign (X = |S|: the bounds and
+// the thresholds) the result is the correctly rounded sum whatever the team,
+// and the oracle's, unless the exact sum comes that close to the middle between
+// two doubles without lying on it.  Where values cancel (the objective), the
+// factor X / |S| comes in: two teams may round differently once it takes up
+// those bits.
 //
 // What bounds it: the passes over memory for large n (7 FP64 additions per
 // element take less), the team sync and the L2 round trips for small n.  So

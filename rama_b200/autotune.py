@@ -17,7 +17,8 @@ built-in choices are guesses; this module measures them on the device:
 * single_cluster_min / single_grid_min: where a single solve moves from one
   CTA to a cluster and from a cluster to the whole GPU -- each team is timed
   on graphs of increasing size and the switch goes to the first size at which
-  the larger team wins;
+  the larger team wins (the automatic line stays where it gives every size
+  the same team);
 * cta_threads: whether a batch without cluster instances runs on CTAs of 512
   threads (two per SM) or 256 (three per SM), timed on such a batch;
 * batch_cluster_min / batch_cluster_share: which instances of a batch get a
@@ -126,6 +127,14 @@ def crossover(sizes: Sequence[int], small_team: Sequence[float], large_team: Seq
     # switch halfway (geometrically) between the last size the small team won
     # and the first size of the larger team's unbroken run of wins
     return int(round(float(np.sqrt(float(sizes[k - 1]) * float(sizes[k])))))
+
+
+def threshold(sizes: Sequence[int], small_team: Sequence[float], large_team: Sequence[float], auto: int) -> int:
+    """The crossover, or MIN_AUTO when the automatic line `auto` gives every
+    measured size the same team: the measurements then cannot tell the two
+    apart, and the automatic one also knows solves without a dual."""
+    c = crossover(sizes, small_team, large_team, auto)
+    return _lib.MIN_AUTO if all((n >= c) == (n >= auto) for n in sizes) else c
 
 
 # ---------------------------------------------------------------------------
@@ -240,9 +249,12 @@ def tune(device: int = 0, budget_s: float = 60.0, quick: bool = False) -> dict:
         clu.append(tr.solve("single%d" % k, g, "PD", team=3))
         grd.append(tr.solve("single%d" % k, g, "PD", team=2))
     if sizes:
-        chosen["single_cluster_min"] = crossover(sizes, cta, clu, _lib.AUTO_CLUSTER_MIN)
-        chosen["single_grid_min"] = max(chosen["single_cluster_min"],
-                                        crossover(sizes, clu, grd, _lib.AUTO_GRID_MIN))
+        low = threshold(sizes, cta, clu, _lib.AUTO_CLUSTER_MIN)
+        high = threshold(sizes, clu, grd, _lib.AUTO_GRID_MIN)
+        first = _lib.AUTO_CLUSTER_MIN if low == _lib.MIN_AUTO else low
+        if (_lib.AUTO_GRID_MIN if high == _lib.MIN_AUTO else high) < first:
+            high = first
+        chosen["single_cluster_min"], chosen["single_grid_min"] = low, high
     tables["single"] = {"edges": sizes, "cta_ms": cta, "cluster_ms": clu, "grid_ms": grd}
     tr.set(**chosen)
 

@@ -24,6 +24,17 @@ def test_crossover_between_last_loss_and_the_run_of_wins():
     assert autotune.crossover(sizes, [1, 1, 1, 1], [5, 5, 5, 5], default=7) == 64001
 
 
+def test_threshold_keeps_the_automatic_line_where_it_agrees():
+    from rama_b200 import _lib
+
+    sizes = [1000, 4000, 16000, 64000]
+    cta, clu = [1, 2, 9, 30], [3, 4, 6, 10]  # the switch lies between 4,000 and 16,000
+    assert autotune.threshold(sizes, cta, clu, 5000) == _lib.MIN_AUTO
+    assert autotune.threshold(sizes, cta, clu, 16000) == _lib.MIN_AUTO
+    assert autotune.threshold(sizes, cta, clu, 4000) == 8000
+    assert autotune.threshold(sizes, cta, clu, 16001) == 8000
+
+
 def test_cache_round_trip(tmp_path):
     p = str(tmp_path / "t.json")
     assert autotune.load_cache(p) == {}
